@@ -57,6 +57,8 @@ PROTOTYPES = {
     "gtm_get_draw_positions": [C.c_void_p, C.c_void_p],
     "gtm_set_recorded_draws": [C.c_void_p, C.c_void_p, C.c_uint64],
     "gtm_dataset_create": [C.c_void_p, C.POINTER(GraphsView), C.POINTER(C.c_void_p)],
+    "gtm_host_alloc": [C.c_uint64, C.POINTER(C.c_void_p)],
+    "gtm_host_free": [C.c_void_p],
     "gtm_validate_graphs": [C.POINTER(GraphsView)],
     "gtm_dataset_destroy": [C.c_void_p],
     "gtm_score": [C.c_void_p, C.c_void_p, C.c_int, C.c_int64, C.c_int64, C.c_void_p],

@@ -10,11 +10,11 @@
 #include <cstring>
 #include <new>
 #include <string>
-#include <thread>
 #include <vector>
 
 #include "gtm_handles.h"
 #include "gtm_kernels.cuh"
+#include "gtm_stage.h"
 
 // The general scoring kernel with or without four-at-a-time node words (graph sets with more than 32 nodes per graph).
 static const void *score_kernel_for(int max_nodes, int units = 1)
@@ -55,6 +55,20 @@ extern "C" int gtm_device_count(int *count_out)
 {
     if (!count_out) return fail(GTM_ERR_ARG, "count_out is null");
     GTM_CU(cudaGetDeviceCount(count_out));
+    return GTM_OK;
+}
+
+extern "C" int gtm_host_alloc(uint64_t bytes, void **out)
+{
+    if (!out) return fail(GTM_ERR_ARG, "out is null");
+    *out = nullptr;
+    GTM_CU(cudaHostAlloc(out, (size_t)std::max<uint64_t>(bytes, 1), cudaHostAllocPortable));
+    return GTM_OK;
+}
+
+extern "C" int gtm_host_free(void *p)
+{
+    if (p) GTM_CU(cudaFreeHost(p));
     return GTM_OK;
 }
 
@@ -99,6 +113,7 @@ extern "C" int gtm_create(const gtm_config *cfg, gtm_model **out)
     GTM_CU(cudaGetDeviceProperties(&prop, cfg->device));
     m->sm_count = prop.multiProcessorCount;
     { int st0 = pool_prepare(cfg->device); if (st0 != GTM_OK) { delete m; return st0; } }
+    stage_retain();                  // given back by gtm_destroy
 
     int st = GTM_OK;
     st = dev_alloc(&d.ta0, (size_t)d.C * d.SB * d.L0);
@@ -112,15 +127,14 @@ extern "C" int gtm_create(const gtm_config *cfg, gtm_model **out)
     if (st == GTM_OK) st = dev_alloc(&m->class_sum_tap, (size_t)d.K);
     if (st == GTM_OK) st = dev_alloc(&m->barrier, 1);
     if (st == GTM_OK) st = dev_alloc(&m->error, 1);
-    if (st == GTM_OK) st = dev_alloc(&m->score_error, 1);
-    if (st == GTM_OK && cudaMallocHost((void **)&m->flag_host, sizeof(int)) != cudaSuccess) st = fail(GTM_ERR_OOM, "page-locked host allocation failed");
+    if (st == GTM_OK && cudaMallocHost((void **)&m->score_error, sizeof(int)) != cudaSuccess) st = fail(GTM_ERR_OOM, "page-locked host allocation failed");
     if (st == GTM_OK) st = dev_alloc(&m->phase_cycles, 8);
     if (st != GTM_OK) { gtm_destroy(m); return st; }
     d.hv = hv;
     cudaMemset(hv, 0, (size_t)d.C * d.MB * sizeof(u32));
     cudaMemset(d.draw_pos, 0, (size_t)d.C * sizeof(u64));
     cudaMemset(d.weights, 0, (size_t)d.K * d.C * sizeof(int));
-    cudaMemset(m->score_error, 0, sizeof(int));
+    *m->score_error = 0;
 
     // learning grid: all CTAs must be co-resident (cooperative launch); no more warps than clauses
     st = fit_grid_for_global_state(d, m->sm_count, m->fit_block, &m->fit_grid);
@@ -139,12 +153,13 @@ extern "C" int gtm_destroy(gtm_model *m)
     cudaSetDevice(m->cfg.device);
     cudaFree(m->dm.ta0); cudaFree(m->dm.tam);
     cudaFree(m->dm.weights); cudaFree((void *)m->dm.hv); cudaFree(m->dm.draw_pos); cudaFree(m->recorded);
-    cudaFree(m->exchange); cudaFree(m->error); cudaFree(m->score_error); cudaFree(m->clause_node); cudaFree(m->update);
+    cudaFree(m->exchange); cudaFree(m->error); cudaFree(m->clause_node); cudaFree(m->update);
     cudaFree(m->class_sum_tap); cudaFree(m->barrier); cudaFree(m->phase_cycles);
     stream_model_destroy(&m->sm);
     tile_model_destroy(&m->tm);
-    if (m->flag_host) cudaFreeHost(m->flag_host);
+    if (m->score_error) cudaFreeHost(m->score_error);
     delete m;
+    stage_drop();
     return GTM_OK;
 }
 
@@ -220,14 +235,16 @@ extern "C" int gtm_get_ta_state(gtm_model *m, int layer, uint32_t *out)
     const DevModel &d = m->dm;
     const int W = layer_words(m, layer);
     const size_t total = (size_t)d.C * d.SB * W;
+    LaneGuard guard;
+    GTM_TRY(lane_acquire(m->cfg.device, &guard.lane));
     u32 *tmp;
     GTM_TRY(pool_alloc(&tmp, total, m->stream));
     planes_to_reference_kernel<<<(unsigned)std::min<size_t>((total + 255) / 256, 4096), 256, 0, m->stream>>>(layer_planes(m, layer), tmp, d.C, d.SB, W);
-    cudaError_t e = cudaMemcpyAsync(out, tmp, total * sizeof(u32), cudaMemcpyDeviceToHost, m->stream);
+    int st = stage_down(guard.lane, out, tmp, total * sizeof(u32), host_is_pinned(out), m->stream);
     cudaFreeAsync(tmp, m->stream);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(m->stream);
-    GTM_CU(e);
-    return GTM_OK;
+    if (st == GTM_OK) st = stage_down_finish(guard.lane);
+    if (st != GTM_OK) stage_abandon(guard.lane);
+    return st;
 }
 
 extern "C" int gtm_set_weights(gtm_model *m, const int32_t *w)
@@ -294,18 +311,6 @@ extern "C" int gtm_set_recorded_draws(gtm_model *m, const uint32_t *draws, uint6
 }
 
 // --------------------------------------------------------------------------------------------- datasets
-// `slack`: elements allocated beyond `count` (never copied, never interpreted)
-template <class T>
-static int upload(gtm_dataset *ds, const T **dev, const T *host, size_t count, cudaStream_t s, bool copy = true, size_t slack = 0)
-{
-    T *p;
-    GTM_TRY(pool_alloc(&p, count + slack, s));
-    ds->owned.push_back(p);
-    if (copy && count && host) GTM_CU(cudaMemcpyAsync(p, host, count * sizeof(T), cudaMemcpyHostToDevice, s));
-    *dev = p;
-    return GTM_OK;
-}
-
 template <class T>
 static int scratch(gtm_dataset *ds, T **dev, size_t count)
 {
@@ -314,38 +319,32 @@ static int scratch(gtm_dataset *ds, T **dev, size_t count)
     return GTM_OK;
 }
 
-__global__ void graph_edge_ranges_kernel(const u32 *node_index, const u32 *n_nodes, const u32 *edge_index, const u32 *degree,
-                                         int64_t n_graphs, u32 *e0, u32 *ne)
-{
-    for (int64_t gi = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; gi < n_graphs; gi += (int64_t)gridDim.x * blockDim.x) {
-        const u32 first = node_index[gi], last = first + n_nodes[gi] - 1;
-        const u32 start = edge_index[first];
-        e0[gi] = start;
-        ne[gi] = edge_index[last] + degree[last] - start;
-    }
-}
+// The graph arrays of a set live in one allocation, in this order, each on a 64-byte boundary; a small set goes up as one
+// copy of a host image of it.
+struct SetLayout {
+    size_t X, node_type, degree, edge_index, edge, node_index, n_nodes, edge0, edges, bytes;
+};
 
-// Fills graph_edge0 / graph_edges from the uploaded arrays (queued on the model's stream).
-static int derive_edge_ranges(gtm_dataset *ds, int64_t n_graphs)
+static SetLayout set_layout(const gtm_graphs_view *v, int L0)
 {
-    cudaStream_t s = ds->model->stream;
-    u32 *e0 = const_cast<u32 *>(ds->dg.graph_edge0), *ne = const_cast<u32 *>(ds->dg.graph_edges);
-    if (ds->total_edges == 0) {
-        GTM_CU(cudaMemsetAsync(e0, 0, (size_t)n_graphs * sizeof(u32), s));
-        GTM_CU(cudaMemsetAsync(ne, 0, (size_t)n_graphs * sizeof(u32), s));
-        return GTM_OK;
-    }
-    graph_edge_ranges_kernel<<<(unsigned)std::min<int64_t>((n_graphs + 255) / 256, 4096), 256, 0, s>>>(
-        ds->dg.node_index, ds->dg.n_nodes, ds->dg.edge_index, ds->dg.degree, n_graphs, e0, ne);
-    GTM_CU(cudaGetLastError());
-    return GTM_OK;
+    SetLayout l;
+    size_t at = 0;
+    auto take = [&](size_t words) { const size_t here = at; at = (at + words * sizeof(u32) + 63) & ~(size_t)63; return here; };
+    const size_t nodes = (size_t)v->total_nodes, graphs = (size_t)v->number_of_graphs;
+    l.X = take(nodes * L0 + 4);       // the tile kernel fetches literal rows with bulk copies widened to 16-byte boundaries
+    l.node_type = take(nodes); l.degree = take(nodes); l.edge_index = take(nodes);
+    l.edge = take(2 * (size_t)v->total_edges);
+    l.node_index = take(graphs); l.n_nodes = take(graphs); l.edge0 = take(graphs); l.edges = take(graphs);
+    l.bytes = at;
+    return l;
 }
 
 // Host arrays must have the layout that graphs.py produces: node_index and edge_index are exclusive prefix sums of the
 // node counts and out-degrees (graphs.py:101-102,127-128), every graph has 1..max_number_of_graph_nodes nodes.  The
 // kernels size their scratch rows from max_number_of_graph_nodes and index the arrays with these values, so anything
-// else is refused here.  Checks graphs [g_lo, g_hi) and their nodes.
-struct GraphChecks { u32 bad_count = 0, bad_index = 0, bad_edges = 0, n_min = ~0u, n_max = 0; };
+// else is refused here.  Checks graphs [g_lo, g_hi) and their nodes, and notes what the arrays have in common: constant
+// arrays are made on the device instead of being copied.
+struct GraphChecks { u32 bad_count = 0, bad_index = 0, bad_edges = 0, n_min = ~0u, n_max = 0, types = 0; };
 
 static void check_graph_span(const gtm_graphs_view *v, int64_t g_lo, int64_t g_hi, GraphChecks *out)
 {
@@ -368,35 +367,33 @@ static void check_graph_span(const gtm_graphs_view *v, int64_t g_lo, int64_t g_h
             const uint64_t want = vi + 1 < v->total_nodes ? (uint64_t)v->edge_index[vi + 1] : (uint64_t)v->total_edges;
             c.bad_edges |= (u32)(end != want);
         }
+        for (int64_t vi = v_lo; vi < v_hi; ++vi) c.types |= v->node_type[vi];
     }
     *out = c;
 }
 
-static int validate_graphs(const gtm_graphs_view *v, int64_t g_lo, int64_t g_hi, u32 *n_min_out = nullptr, u32 *n_max_out = nullptr)
+static int validate_graphs(const gtm_graphs_view *v, int64_t g_lo, int64_t g_hi, GraphChecks *all_out = nullptr)
 {
     if (g_lo == 0 && (v->node_index[0] != 0 || v->edge_index[0] != 0)) return fail(GTM_ERR_ARG, "node_index[0] and edge_index[0] must be 0");
-    // large sets are checked by a few threads side by side (the arrays are only read)
-    const int64_t span = g_hi - g_lo;
-    const int workers = (int)std::max<int64_t>(1, std::min<int64_t>(8, span / (1 << 18)));
-    std::vector<GraphChecks> parts((size_t)workers);
-    if (workers == 1) {
-        check_graph_span(v, g_lo, g_hi, &parts[0]);
-    } else {
-        std::vector<std::thread> threads;
-        for (int w = 0; w < workers; ++w)
-            threads.emplace_back(check_graph_span, v, g_lo + span * w / workers, g_lo + span * (w + 1) / workers, &parts[(size_t)w]);
-        for (std::thread &t : threads) t.join();
-    }
+    // large sets are checked by the copy threads side by side (the arrays are only read); a thread takes about 2^15 nodes
+    const int64_t span = g_hi - g_lo, nodes = span * (v->total_nodes / v->number_of_graphs + 1);
+    const int pieces = (int)std::max<int64_t>(1, std::min<int64_t>(std::min<int64_t>(16, span), nodes >> 15));
+    struct Job { const gtm_graphs_view *v; int64_t lo, span; int pieces; GraphChecks parts[16]; } job;
+    job.v = v; job.lo = g_lo; job.span = span; job.pieces = pieces;
+    host_parallel(pieces, [](void *c, int i) {
+        Job *j = (Job *)c;
+        check_graph_span(j->v, j->lo + j->span * i / j->pieces, j->lo + j->span * (i + 1) / j->pieces, &j->parts[i]);
+    }, &job);
     GraphChecks all;
-    for (const GraphChecks &c : parts) {
-        all.bad_count |= c.bad_count; all.bad_index |= c.bad_index; all.bad_edges |= c.bad_edges;
+    for (int i = 0; i < pieces; ++i) {
+        const GraphChecks &c = job.parts[i];
+        all.bad_count |= c.bad_count; all.bad_index |= c.bad_index; all.bad_edges |= c.bad_edges; all.types |= c.types;
         all.n_min = std::min(all.n_min, c.n_min); all.n_max = std::max(all.n_max, c.n_max);
     }
     if (all.bad_count) return fail(GTM_ERR_ARG, "a graph has no nodes or more than max_number_of_graph_nodes = %d", v->max_number_of_graph_nodes);
     if (all.bad_index) return fail(GTM_ERR_ARG, "node_index is not the running sum of number_of_graph_nodes (or exceeds total_nodes)");
     if (all.bad_edges) return fail(GTM_ERR_ARG, "edge_index is not the running sum of number_of_graph_node_edges (or exceeds total_edges)");
-    if (n_min_out) *n_min_out = all.n_min;
-    if (n_max_out) *n_max_out = all.n_max;
+    if (all_out) *all_out = all;
     return GTM_OK;
 }
 
@@ -417,51 +414,159 @@ static int check_view(const gtm_graphs_view *v)
 extern "C" int gtm_validate_graphs(const gtm_graphs_view *v)
 {
     GTM_TRY(check_view(v));
+    struct Keep { Keep() { stage_retain(); } ~Keep() { stage_drop(); } } keep;      // the copy threads stay while they check
     return validate_graphs(v, 0, v->number_of_graphs);
 }
 
-// copy_arrays == false: the per-node and per-graph arrays are only allocated; the caller copies them in pieces
-// (gtm_dataset_create_scored).
-static int dataset_build(gtm_model *m, const gtm_graphs_view *v, gtm_dataset *ds, bool copy_arrays = true)
+// What the copies of graphs [g0, g1) leave to the device: constant arrays, index arrays of equally large graphs, and the
+// edge rows of every graph (first and number; graphs own consecutive CSR rows).
+struct RangeFill {
+    int64_t g0, g1, v0, v1;
+    u32 e0;
+    int uniform_n;          // > 0: every graph has this many nodes; node_index and n_nodes are made here
+    int no_types;           // every node has type 0
+    int no_edges;           // no node has an edge: degree is 0, edge_index is e0
+    int next_graph;         // node_index of graph g1 is made too: a tile ends where the next graph's nodes begin
+    u32 *node_type, *degree, *edge_index, *node_index, *n_nodes, *graph_edge0, *graph_edges;
+};
+
+__global__ void __launch_bounds__(256) fill_range_kernel(RangeFill f)
+{
+    const int64_t t0 = blockIdx.x * (int64_t)blockDim.x + threadIdx.x, step = (int64_t)gridDim.x * blockDim.x;
+    if (f.no_types)
+        for (int64_t i = f.v0 + t0; i < f.v1; i += step) f.node_type[i] = 0;
+    if (f.no_edges)
+        for (int64_t i = f.v0 + t0; i < f.v1; i += step) { f.degree[i] = 0; f.edge_index[i] = f.e0; }
+    for (int64_t gi = f.g0 + t0; gi < f.g1; gi += step) {
+        u32 first, n;
+        if (f.uniform_n > 0) {
+            first = (u32)(f.v0 + (gi - f.g0) * f.uniform_n); n = (u32)f.uniform_n;
+            f.node_index[gi] = first;
+            f.n_nodes[gi] = n;
+        } else {
+            first = f.node_index[gi]; n = f.n_nodes[gi];
+        }
+        const u32 start = f.no_edges ? f.e0 : f.edge_index[first], last = first + n - 1;
+        f.graph_edge0[gi] = start;
+        f.graph_edges[gi] = f.no_edges ? 0u : f.edge_index[last] + f.degree[last] - start;
+    }
+    if (f.uniform_n > 0 && f.next_graph && t0 == 0) f.node_index[f.g1] = (u32)f.v1;
+}
+
+// Graphs [g0, g1) of the set: copies queued on stream `in`, and the rest of their arrays described for fill_range_kernel.
+static int upload_range(gtm_dataset *ds, const gtm_graphs_view *v, StageLane *lane, int64_t g0, int64_t g1, const GraphChecks &facts, cudaStream_t in,
+                        RangeFill *fill)
+{
+    const DevGraphs &dg = ds->dg;
+    const int64_t N = v->number_of_graphs;
+    const int L0 = ds->model->dm.L0;
+    RangeFill f;
+    memset(&f, 0, sizeof f);
+    f.g0 = g0; f.g1 = g1;
+    f.v0 = v->node_index[g0]; f.v1 = g1 < N ? (int64_t)v->node_index[g1] : v->total_nodes;
+    f.e0 = v->edge_index[f.v0];
+    const int64_t e1 = f.v1 < v->total_nodes ? (int64_t)v->edge_index[f.v1] : v->total_edges;
+    f.uniform_n = facts.n_min == facts.n_max ? (int)facts.n_min : 0;
+    f.no_types = facts.types == 0;
+    f.no_edges = e1 == (int64_t)f.e0;
+    f.next_graph = g1 < N;
+    f.node_type = const_cast<u32 *>(dg.node_type); f.degree = const_cast<u32 *>(dg.degree); f.edge_index = const_cast<u32 *>(dg.edge_index);
+    f.node_index = const_cast<u32 *>(dg.node_index); f.n_nodes = const_cast<u32 *>(dg.n_nodes);
+    f.graph_edge0 = const_cast<u32 *>(dg.graph_edge0); f.graph_edges = const_cast<u32 *>(dg.graph_edges);
+    *fill = f;
+    const bool pinned = host_is_pinned(v->X);
+    auto up = [&](const u32 *dst, const u32 *src, size_t first, size_t count, bool pin) {
+        return stage_up(lane, const_cast<u32 *>(dst) + first, src + first, count * sizeof(u32), pin, in);
+    };
+    const size_t v0 = (size_t)f.v0, nodes = (size_t)(f.v1 - f.v0), graphs = (size_t)(g1 - g0);
+    GTM_TRY(up(dg.X, v->X, v0 * L0, nodes * L0, pinned));
+    if (!f.no_types) GTM_TRY(up(dg.node_type, v->node_type, v0, nodes, host_is_pinned(v->node_type)));
+    if (!f.no_edges) {
+        GTM_TRY(up(dg.degree, v->number_of_graph_node_edges, v0, nodes, host_is_pinned(v->number_of_graph_node_edges)));
+        GTM_TRY(up(dg.edge_index, v->edge_index, v0, nodes, host_is_pinned(v->edge_index)));
+        GTM_TRY(up(dg.edge, v->edge, 2 * (size_t)f.e0, 2 * (size_t)(e1 - f.e0), host_is_pinned(v->edge)));
+    }
+    if (f.uniform_n == 0) {
+        GTM_TRY(up(dg.node_index, v->node_index, (size_t)g0, graphs + (g1 < N ? 1 : 0), host_is_pinned(v->node_index)));
+        GTM_TRY(up(dg.n_nodes, v->number_of_graph_nodes, (size_t)g0, graphs, host_is_pinned(v->number_of_graph_nodes)));
+    }
+    return GTM_OK;
+}
+
+static int fill_range(const RangeFill &f, cudaStream_t s)
+{
+    const int64_t items = std::max(f.no_types || f.no_edges ? f.v1 - f.v0 : 0, f.g1 - f.g0);
+    fill_range_kernel<<<(unsigned)std::min<int64_t>((items + 255) / 256, 1024), 256, 0, s>>>(f);
+    GTM_CU(cudaGetLastError());
+    return GTM_OK;
+}
+
+// A small set: validated, laid out in page-locked memory as it will lie on the device, one copy.
+static int upload_small(gtm_dataset *ds, const gtm_graphs_view *v, StageLane *lane, const SetLayout &l, char *dev, cudaStream_t s)
+{
+    char *img = lane->small;
+    const size_t nodes = (size_t)v->total_nodes, graphs = (size_t)v->number_of_graphs;
+    memcpy(img + l.X, v->X, nodes * ds->model->dm.L0 * sizeof(u32));
+    memcpy(img + l.node_type, v->node_type, nodes * sizeof(u32));
+    memcpy(img + l.degree, v->number_of_graph_node_edges, nodes * sizeof(u32));
+    memcpy(img + l.edge_index, v->edge_index, nodes * sizeof(u32));
+    if (v->total_edges) memcpy(img + l.edge, v->edge, 2 * (size_t)v->total_edges * sizeof(u32));
+    memcpy(img + l.node_index, v->node_index, graphs * sizeof(u32));
+    memcpy(img + l.n_nodes, v->number_of_graph_nodes, graphs * sizeof(u32));
+    u32 *e0 = (u32 *)(img + l.edge0), *ne = (u32 *)(img + l.edges);
+    for (size_t gi = 0; gi < graphs; ++gi) {
+        const u32 first = v->node_index[gi], last = first + v->number_of_graph_nodes[gi] - 1;
+        e0[gi] = v->edge_index[first];
+        ne[gi] = v->edge_index[last] + v->number_of_graph_node_edges[last] - e0[gi];
+    }
+    GTM_CU(cudaMemcpyAsync(dev, img, l.bytes, cudaMemcpyHostToDevice, s));
+    return GTM_OK;
+}
+
+enum class SetCopy { whole, in_ranges };        // in_ranges: the caller validates and copies the arrays range by range
+
+// Allocates the set's arrays and plans its scoring; the copies (SetCopy::whole) are queued on the model's stream and may
+// still be running when this returns.
+static int dataset_build(gtm_model *m, const gtm_graphs_view *v, gtm_dataset *ds, SetCopy copy, StageLane *lane)
 {
     const DevModel &d = m->dm;
     cudaStream_t s = m->stream;
-    // the tile kernel fetches literal rows with bulk copies widened to 16-byte boundaries: a little slack at the end
-    GTM_TRY(upload(ds, &ds->dg.X, v->X, (size_t)v->total_nodes * d.L0, s, copy_arrays, 4));
-    GTM_TRY(upload(ds, &ds->dg.node_type, v->node_type, (size_t)v->total_nodes, s, copy_arrays));
-    GTM_TRY(upload(ds, &ds->dg.degree, v->number_of_graph_node_edges, (size_t)v->total_nodes, s, copy_arrays));
-    GTM_TRY(upload(ds, &ds->dg.edge_index, v->edge_index, (size_t)v->total_nodes, s, copy_arrays));
-    GTM_TRY(upload(ds, &ds->dg.edge, v->edge, 2 * (size_t)v->total_edges, s, copy_arrays));
-    GTM_TRY(upload(ds, &ds->dg.node_index, v->node_index, (size_t)v->number_of_graphs, s, copy_arrays));
-    GTM_TRY(upload(ds, &ds->dg.n_nodes, v->number_of_graph_nodes, (size_t)v->number_of_graphs, s, copy_arrays));
-    {   // first edge row and number of edge rows of every graph (graphs own consecutive CSR rows): derived on the device
-        u32 *e0, *ne;
-        GTM_TRY(scratch(ds, &e0, (size_t)v->number_of_graphs));
-        GTM_TRY(scratch(ds, &ne, (size_t)v->number_of_graphs));
-        ds->dg.graph_edge0 = e0;
-        ds->dg.graph_edges = ne;
-        if (copy_arrays) GTM_TRY(derive_edge_ranges(ds, v->number_of_graphs));      // else: once the caller has copied the arrays
+    const SetLayout l = set_layout(v, d.L0);
+    char *dev;
+    GTM_TRY(scratch(ds, &dev, l.bytes));
+    DevGraphs &dg = ds->dg;
+    dg.X = (u32 *)(dev + l.X); dg.node_type = (u32 *)(dev + l.node_type); dg.degree = (u32 *)(dev + l.degree);
+    dg.edge_index = (u32 *)(dev + l.edge_index); dg.edge = (u32 *)(dev + l.edge);
+    dg.node_index = (u32 *)(dev + l.node_index); dg.n_nodes = (u32 *)(dev + l.n_nodes);
+    dg.graph_edge0 = (u32 *)(dev + l.edge0); dg.graph_edges = (u32 *)(dev + l.edges);
+    dg.n_types = 1;
+    dg.total_nodes = (u32)v->total_nodes; dg.total_edges = (u32)v->total_edges;
+    dg.max_nodes = ds->max_nodes; dg.error = m->score_error;
+    if (copy == SetCopy::whole) {
+        GraphChecks facts;
+        GTM_TRY(validate_graphs(v, 0, v->number_of_graphs, &facts));
+        ds->n_min = facts.n_min; ds->n_max = facts.n_max;
+        if (l.bytes <= kStageSmall) {
+            GTM_TRY(upload_small(ds, v, lane, l, dev, s));
+        } else {
+            RangeFill f;
+            GTM_TRY(upload_range(ds, v, lane, 0, v->number_of_graphs, facts, s, &f));
+            GTM_TRY(fill_range(f, s));
+        }
+    } else if (ds->max_nodes > 1) {                      // not validated yet: the tilings take these only as hints
+        u32 lo = ~0u, hi = 0;
+        for (int64_t gi = 0; gi < v->number_of_graphs; ++gi) {
+            lo = std::min(lo, v->number_of_graph_nodes[gi]);
+            hi = std::max(hi, v->number_of_graph_nodes[gi]);
+        }
+        if (lo >= 1 && hi <= (u32)ds->max_nodes) { ds->n_min = lo; ds->n_max = hi; }
     }
-    ds->dg.n_types = 1;
-    ds->dg.total_nodes = (u32)v->total_nodes; ds->dg.total_edges = (u32)v->total_edges;
-    ds->dg.max_nodes = ds->max_nodes; ds->dg.error = m->score_error;
-
-    // learning scratch
-    const size_t p_words = (size_t)std::max(1, d.D - 1) * ds->max_nodes * d.MW;
-    ds->fit_sc.NC = ds->NC; ds->fit_sc.cno_slots = d.D; ds->fit_sc.max_nodes = ds->max_nodes;
-    GTM_TRY(scratch(ds, &ds->fit_sc.cno, (size_t)d.D * d.C * ds->NC));
-    GTM_TRY(scratch(ds, &ds->fit_sc.n_inc, (size_t)d.C));
-    GTM_TRY(scratch(ds, &ds->P_pair[0], p_words));
-    GTM_TRY(scratch(ds, &ds->P_pair[1], p_words));
-    GTM_TRY(scratch(ds, &ds->Q_pair[0], p_words));
-    GTM_TRY(scratch(ds, &ds->Q_pair[1], p_words));
-    GTM_TRY(scratch(ds, &ds->rank_barrier, 64));
-    ds->fit_sc.P = ds->P_pair[0];
 
     // general scoring scratch: one slice per resident CTA
     // General scoring kernel, shared memory per CTA: vote partial; for depth > 1 the source-node message bits of a graph
     // (flush_messages) when they are small enough not to cost resident CTAs; for graph sets of 33..1024 nodes per graph the
     // transposed copy of the graph - and then the message bits too (up to 64 KB), in CTAs of 512 threads, one or two per SM.
+    const size_t p_words = (size_t)std::max(1, d.D - 1) * ds->max_nodes * d.MW;
     ds->score_part_words = 0;
     ds->score_t_stride = 0;
     ds->score_block = 256;
@@ -489,60 +594,83 @@ static int dataset_build(gtm_model *m, const gtm_graphs_view *v, gtm_dataset *ds
             ds->score_smem = 8 * per_warp;
         }
     }
-    if (ds->score_smem > 48 * 1024)
-        GTM_CU(cudaFuncSetAttribute(score_kernel_for(ds->max_nodes), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ds->score_smem));
-    int per_sm = 0;
-    GTM_CU(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, score_kernel_for(ds->max_nodes, ds->score_units), ds->score_block, ds->score_smem));
-    ds->score_grid = (int)std::max<int64_t>(1, std::min<int64_t>((int64_t)m->sm_count * std::max(1, per_sm), v->number_of_graphs));
     ds->cno_stride = (size_t)2 * d.C * ds->NC;
     ds->P_stride = p_words;
     ds->ninc_stride = (size_t)d.C;
     ds->score_sc.NC = ds->NC; ds->score_sc.cno_slots = 2; ds->score_sc.max_nodes = ds->max_nodes;
     ds->score_sc.cno = nullptr;   // allocated on first use of the general kernel (ensure_score_scratch)
 
-    GTM_TRY(stream_data_create(&ds->sd, m->sm, d, ds->dg, v, m->sm_count, s));
+    GTM_TRY(stream_data_create(&ds->sd, m->sm, d, v, ds->n_min, ds->n_max, m->sm_count, s));
     // tiles of whole graphs for the tile kernel: deeper models, or sets the node-stream kernel does not cover
     if (d.D > 1 || !ds->sd.supported || m->opt_score_kernel == 3) GTM_TRY(tile_data_create(&ds->td, m->tm, d, v, ds->n_min, ds->n_max, m->sm_count, s));
-    GTM_CU(cudaStreamSynchronize(s));
     return GTM_OK;
 }
 
-static int dataset_create(gtm_model *m, const gtm_graphs_view *v, gtm_dataset **out, bool copy_arrays)
+static int dataset_create(gtm_model *m, const gtm_graphs_view *v, gtm_dataset **out, SetCopy copy, StageLane *lane)
 {
-    GTM_TRY(bind(m));
-    if (!v || !out) return fail(GTM_ERR_ARG, "null argument");
     *out = nullptr;
-    GTM_TRY(check_view(v));
     gtm_dataset *ds = new (std::nothrow) gtm_dataset();
     if (!ds) return fail(GTM_ERR_OOM, "host allocation failed");
     ds->model = m;
     ds->n_graphs = v->number_of_graphs; ds->total_nodes = v->total_nodes; ds->total_edges = v->total_edges;
     ds->max_nodes = v->max_number_of_graph_nodes;
     ds->NC = words_for(ds->max_nodes);
-    // the pipelined caller validates chunk by chunk, just before each chunk is copied
-    int st = copy_arrays ? validate_graphs(v, 0, v->number_of_graphs, &ds->n_min, &ds->n_max) : GTM_OK;
-    if (st == GTM_OK) st = dataset_build(m, v, ds, copy_arrays);
-    if (st != GTM_OK) { gtm_dataset_destroy(ds); return st; }
+    const int st = dataset_build(m, v, ds, copy, lane);
+    if (st != GTM_OK) {
+        cudaStreamSynchronize(m->stream);               // nothing may still be reading the host arrays when the call returns
+        gtm_dataset_destroy(ds);
+        return st;
+    }
     *out = ds;
     return GTM_OK;
 }
 
 extern "C" int gtm_dataset_create(gtm_model *m, const gtm_graphs_view *v, gtm_dataset **out)
 {
-    return dataset_create(m, v, out, true);
+    GTM_TRY(bind(m));
+    if (!v || !out) return fail(GTM_ERR_ARG, "null argument");
+    *out = nullptr;
+    GTM_TRY(check_view(v));
+    LaneGuard guard;
+    GTM_TRY(lane_acquire(m->cfg.device, &guard.lane));
+    GTM_TRY(dataset_create(m, v, out, SetCopy::whole, guard.lane));
+    const cudaError_t e = cudaStreamSynchronize(m->stream);
+    if (e != cudaSuccess) { gtm_dataset_destroy(*out); *out = nullptr; }
+    GTM_CU(e);
+    return GTM_OK;
 }
 
 extern "C" int gtm_dataset_destroy(gtm_dataset *ds)
 {
     if (!ds) return GTM_OK;
     cudaSetDevice(ds->model->cfg.device);
-    cudaStreamSynchronize(ds->model->stream);
-    for (void *p : ds->owned) cudaFreeAsync(p, ds->model->stream);
-    cudaFree(ds->Y);
+    for (void *p : ds->owned) cudaFreeAsync(p, ds->model->stream);        // in stream order, behind the kernels that use them
+    if (ds->Y) cudaFree(ds->Y);
     stream_data_destroy(&ds->sd);
     tile_data_destroy(&ds->td);
+    if (ds->comm.block) cudaStreamSynchronize(ds->model->stream);
     fit_comm_release(ds);
     delete ds;
+    return GTM_OK;
+}
+
+// Scratch of the learning kernels (every layer kept), made when the set is first learned from or evaluated by a tap.
+int ensure_fit_scratch(gtm_dataset *ds)
+{
+    if (ds->fit_sc.cno) return GTM_OK;
+    const DevModel &d = ds->model->dm;
+    const size_t p_words = (size_t)std::max(1, d.D - 1) * ds->max_nodes * d.MW;
+    ds->fit_sc.NC = ds->NC; ds->fit_sc.cno_slots = d.D; ds->fit_sc.max_nodes = ds->max_nodes;
+    u32 *cno;
+    GTM_TRY(scratch(ds, &cno, (size_t)d.D * d.C * ds->NC));
+    GTM_TRY(scratch(ds, &ds->fit_sc.n_inc, (size_t)d.C));
+    GTM_TRY(scratch(ds, &ds->P_pair[0], p_words));
+    GTM_TRY(scratch(ds, &ds->P_pair[1], p_words));
+    GTM_TRY(scratch(ds, &ds->Q_pair[0], p_words));
+    GTM_TRY(scratch(ds, &ds->Q_pair[1], p_words));
+    GTM_TRY(scratch(ds, &ds->rank_barrier, 64));
+    ds->fit_sc.P = ds->P_pair[0];
+    ds->fit_sc.cno = cno;
     return GTM_OK;
 }
 
@@ -558,22 +686,32 @@ static int check_range(gtm_model *m, gtm_dataset *ds, int n_types, int64_t first
     return GTM_OK;
 }
 
-// What the word that scoring kernels raise means to the caller (cleared once it was seen).
-static int score_flag_status(gtm_model *m, int flag)
+// What the word that scoring kernels raise means to the caller (page-locked host memory that the device writes; the
+// stream has been waited for).  Cleared once it was seen.
+static int score_flag_status(gtm_model *m)
 {
+    const int flag = *(volatile int *)m->score_error;
     if (flag == 0) return GTM_OK;
-    cudaMemsetAsync(m->score_error, 0, sizeof(int), m->stream);
+    *(volatile int *)m->score_error = 0;
     if (flag == 2) return fail(GTM_ERR_TIMEOUT, "a scoring kernel gave up waiting for a bulk copy into shared memory; the class sums are not valid");
     return fail(GTM_ERR_ARG, "a scoring kernel skipped a malformed graph (node count or node range out of bounds)");
 }
 
+// Launch shape and scratch of the general scoring kernel, made on its first use.
 static int ensure_score_scratch(gtm_dataset *ds)
 {
     if (ds->score_sc.cno) return GTM_OK;
+    const void *fn = score_kernel_for(ds->max_nodes, ds->score_units);
+    if (ds->score_smem > 48 * 1024) GTM_CU(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ds->score_smem));
+    int per_sm = 0;
+    GTM_CU(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, ds->score_block, ds->score_smem));
+    ds->score_grid = (int)std::max<int64_t>(1, std::min<int64_t>((int64_t)ds->model->sm_count * std::max(1, per_sm), ds->n_graphs));
     const size_t slices = (size_t)ds->score_grid * ds->score_units;     // one slice per graph in flight
-    GTM_TRY(scratch(ds, &ds->score_sc.cno, ds->cno_stride * slices));
+    u32 *cno;
+    GTM_TRY(scratch(ds, &cno, ds->cno_stride * slices));
     GTM_TRY(scratch(ds, &ds->score_sc.P, ds->P_stride * slices));
     GTM_TRY(scratch(ds, &ds->score_sc.n_inc, ds->ninc_stride * slices));
+    ds->score_sc.cno = cno;
     return GTM_OK;
 }
 
@@ -615,6 +753,16 @@ static int refresh_tile_lists(gtm_model *m)
     return GTM_OK;
 }
 
+static bool scores_by_stream(gtm_model *m, gtm_dataset *ds, int n_types)
+{
+    return (m->opt_score_kernel == 0 || m->opt_score_kernel == 2) && stream_supported(ds->sd, n_types);
+}
+
+static bool scores_by_tile(gtm_model *m, gtm_dataset *ds, int n_types)
+{
+    return (m->opt_score_kernel == 0 || m->opt_score_kernel == 3) && tile_supported(ds->td, n_types);
+}
+
 extern "C" int gtm_score_device(gtm_model *m, gtm_dataset *ds, int n_types, int64_t first, int64_t count,
                                 int32_t *sums_dev)
 {
@@ -626,15 +774,124 @@ extern "C" int gtm_score_device(gtm_model *m, gtm_dataset *ds, int n_types, int6
         return fail(GTM_ERR_ARG, "the node-stream scoring kernel does not cover this model / graph set");
     if (m->opt_score_kernel == 3 && !tile_supported(ds->td, n_types))
         return fail(GTM_ERR_ARG, "the tile scoring kernel does not cover this model / graph set");
-    if ((m->opt_score_kernel == 0 || m->opt_score_kernel == 2) && stream_supported(ds->sd, n_types)) {
+    if (scores_by_stream(m, ds, n_types)) {
         GTM_TRY(refresh_lists(m));
-        return stream_score(m->sm, ds->sd, m->dm, ds->dg, n_types, first, count, sums_dev, m->stream);
+        return stream_score(&m->sm, ds->sd, m->dm, ds->dg, n_types, first, count, sums_dev, 0, m->stream);
     }
-    if ((m->opt_score_kernel == 0 || m->opt_score_kernel == 3) && tile_supported(ds->td, n_types)) {
+    if (scores_by_tile(m, ds, n_types)) {
         GTM_TRY(refresh_tile_lists(m));
-        return tile_score(m->tm, ds->td, m->dm, ds->dg, n_types, first, count, sums_dev, m->score_error, m->stream);
+        return tile_score(&m->tm, ds->td, m->dm, ds->dg, n_types, first, count, sums_dev, m->score_error, 0, m->stream);
     }
     return launch_score_general(m, ds, n_types, first, count, sums_dev, nullptr);
+}
+
+// Scoring of graphs [first, first+count) into host memory by a tiled kernel, pipelined: chunks of whole tiles are scored
+// on two streams in turn, so that one chunk's last tiles and the next one's first share the chip, and class sums go back
+// on a copy stream meanwhile.  With `v` (and the whole set as the range) the set's arrays go up too, chunk by chunk on
+// another copy stream - a chunk is the literal rows, per-node arrays and edge rows of a contiguous range of graphs -, each
+// validated just before it is copied and scored when it has landed.
+static int score_in_chunks(gtm_model *m, gtm_dataset *ds, const gtm_graphs_view *v, bool by_stream, int n_types, int64_t first, int64_t count,
+                           int32_t *out, StageLane *lane)
+{
+    const DevModel &d = m->dm;
+    const int64_t n = ds->n_graphs;
+    const int uniform_gpt = by_stream ? ds->sd.graphs_per_tile : ds->td.graphs_per_tile;
+    const std::vector<int> &table = by_stream ? ds->sd.tile_graph_host : ds->td.tile_graph_host;
+    const int all_tiles = by_stream ? ds->sd.n_tiles : ds->td.n_tiles;
+    auto tile_first = [&](int t) -> int64_t {           // first graph of tile t
+        if (t >= all_tiles) return n;
+        return uniform_gpt > 0 ? std::min<int64_t>((int64_t)t * uniform_gpt, n) : (int64_t)table[(size_t)t];
+    };
+    auto tile_of = [&](int64_t g) -> int {
+        return uniform_gpt > 0 ? (int)(g / uniform_gpt) : (int)(std::upper_bound(table.begin(), table.end(), (int)g) - table.begin()) - 1;
+    };
+    const int t_lo = tile_of(first), t_hi = tile_of(first + count - 1) + 1, tiles = t_hi - t_lo;
+    // Chunks of a quarter of the range, and of 1 to 8 MB where arrays go up: little of the copies is left uncovered and the
+    // per-chunk work of the host stays small.  The tile kernel takes a tile per CTA: whole half-waves of them, two chunks
+    // side by side fill the chip.
+    int chunk_tiles = (tiles + 3) / 4;
+    if (v) {
+        const size_t tile_bytes = std::max<size_t>(1, set_layout(v, d.L0).bytes / (size_t)all_tiles);
+        chunk_tiles = (int)std::max<size_t>(((size_t)1 << 20) / tile_bytes, std::min<size_t>((size_t)chunk_tiles, ((size_t)8 << 20) / tile_bytes)) + 1;
+    }
+    if (!by_stream) chunk_tiles = (chunk_tiles + m->sm_count - 1) / m->sm_count * m->sm_count;
+    const bool pinned_out = host_is_pinned(out);
+    int *dev = nullptr;
+    auto body = [&]() -> int {
+        if (by_stream) {
+            GTM_TRY(refresh_lists(m));
+            GTM_TRY(stream_reserve(&m->sm, ds->sd, d, std::min(chunk_tiles, tiles)));
+        } else {
+            GTM_TRY(refresh_tile_lists(m));
+        }
+        GTM_TRY(pool_alloc(&dev, (size_t)count * d.K, m->stream));
+        GTM_CU(cudaEventRecord(lane->event[0], m->stream));       // allocations, tile tables and literal lists are in stream order
+        GTM_CU(cudaStreamWaitEvent(lane->in, lane->event[0], 0));
+        GTM_CU(cudaStreamWaitEvent(lane->aux, lane->event[0], 0));
+        int turn = 0;
+        for (int t0 = t_lo; t0 < t_hi; t0 += chunk_tiles, turn ^= 1) {
+            const int64_t g0 = std::max(first, tile_first(t0)), g1 = std::min(first + count, tile_first(t0 + chunk_tiles));
+            if (g1 <= g0) continue;
+            const size_t cnt = (size_t)(g1 - g0), at = (size_t)(g0 - first) * d.K;
+            cudaStream_t cs = turn ? lane->aux : m->stream;
+            if (v) {
+                GraphChecks facts;
+                RangeFill f;
+                GTM_TRY(validate_graphs(v, g0, g1, &facts));      // overlaps the copies of the chunks before
+                GTM_TRY(upload_range(ds, v, lane, g0, g1, facts, lane->in, &f));
+                GTM_CU(cudaEventRecord(lane->event[1], lane->in));
+                GTM_CU(cudaStreamWaitEvent(cs, lane->event[1], 0));
+                GTM_TRY(fill_range(f, cs));
+            }
+            if (by_stream) GTM_TRY(stream_score(&m->sm, ds->sd, d, ds->dg, n_types, g0, (int64_t)cnt, dev + at, turn, cs));
+            else GTM_TRY(tile_score(&m->tm, ds->td, d, ds->dg, n_types, g0, (int64_t)cnt, dev + at, m->score_error, turn, cs));
+            GTM_CU(cudaEventRecord(lane->event[2], cs));
+            GTM_CU(cudaStreamWaitEvent(lane->back, lane->event[2], 0));
+            GTM_TRY(stage_down(lane, out + at, dev + at, cnt * d.K * sizeof(int), pinned_out, lane->back));
+        }
+        GTM_CU(cudaEventRecord(lane->event[1], lane->aux));       // everything that used the set is in the order of the model's stream
+        GTM_CU(cudaStreamWaitEvent(m->stream, lane->event[1], 0));
+        GTM_TRY(stage_down_finish(lane));
+        if (v) GTM_CU(cudaStreamSynchronize(lane->in));
+        GTM_CU(cudaStreamSynchronize(m->stream));
+        return score_flag_status(m);
+    };
+    const int st = body();
+    if (st != GTM_OK) {                                           // nothing may still be reading the host arrays when the call returns
+        stage_abandon(lane);
+        cudaStreamSynchronize(m->stream);
+    }
+    if (dev) cudaFreeAsync(dev, m->stream);
+    return st;
+}
+
+// Class sums of graphs [first, first+count) into host memory; waits for them.
+static int score_to_host(gtm_model *m, gtm_dataset *ds, int n_types, int64_t first, int64_t count, int32_t *out, StageLane *lane)
+{
+    const size_t bytes = (size_t)count * m->dm.K * sizeof(int);
+    // a few results: the kernel writes them to page-locked host memory itself, which takes less than starting a copy
+    if (bytes <= 16 * 1024) {
+        int *direct = (int *)(lane->small + kStageSmall);
+        GTM_TRY(gtm_score_device(m, ds, n_types, first, count, direct));
+        GTM_CU(cudaStreamSynchronize(m->stream));
+        GTM_TRY(score_flag_status(m));
+        memcpy(out, direct, bytes);
+        return GTM_OK;
+    }
+    // results whose way back (50 GB/s) is worth hiding behind the kernel
+    if (bytes >= 512 * 1024) {
+        const bool by_stream = scores_by_stream(m, ds, n_types);
+        if (by_stream || scores_by_tile(m, ds, n_types)) return score_in_chunks(m, ds, nullptr, by_stream, n_types, first, count, out, lane);
+    }
+    int *dev;
+    GTM_TRY(pool_alloc(&dev, (size_t)count * m->dm.K, m->stream));
+    int st = gtm_score_device(m, ds, n_types, first, count, dev);
+    if (st == GTM_OK) st = stage_down(lane, out, dev, bytes, host_is_pinned(out), m->stream);
+    cudaFreeAsync(dev, m->stream);
+    if (st == GTM_OK) st = stage_down_finish(lane);
+    if (st != GTM_OK) { stage_abandon(lane); cudaStreamSynchronize(m->stream); return st; }
+    GTM_CU(cudaStreamSynchronize(m->stream));
+    return score_flag_status(m);
 }
 
 extern "C" int gtm_score(gtm_model *m, gtm_dataset *ds, int n_types, int64_t first, int64_t count, int32_t *out)
@@ -643,24 +900,13 @@ extern "C" int gtm_score(gtm_model *m, gtm_dataset *ds, int n_types, int64_t fir
     GTM_TRY(check_range(m, ds, n_types, first, count));
     if (count == 0) return GTM_OK;
     if (!out) return fail(GTM_ERR_ARG, "class_sums_out is null");
-    int *dev;
-    GTM_TRY(pool_alloc(&dev, (size_t)count * m->dm.K, m->stream));
-    int st = gtm_score_device(m, ds, n_types, first, count, dev);
-    cudaError_t e = cudaSuccess;
-    if (st == GTM_OK) e = cudaMemcpyAsync(out, dev, (size_t)count * m->dm.K * sizeof(int), cudaMemcpyDeviceToHost, m->stream);
-    cudaFreeAsync(dev, m->stream);
-    if (st == GTM_OK && e == cudaSuccess) e = cudaMemcpyAsync(m->flag_host, m->score_error, sizeof(int), cudaMemcpyDeviceToHost, m->stream);
-    if (st == GTM_OK && e == cudaSuccess) e = cudaStreamSynchronize(m->stream);
-    if (st != GTM_OK) return st;
-    GTM_CU(e);
-    return score_flag_status(m, *m->flag_host);
+    LaneGuard guard;
+    GTM_TRY(lane_acquire(m->cfg.device, &guard.lane));
+    return score_to_host(m, ds, n_types, first, count, out, guard.lane);
 }
 
-// Upload and scoring of a whole host graph set in one call.  Sets that the node-stream kernel or the tile kernel covers
-// are pipelined: the graph arrays go up in chunks of whole tiles (two full waves of thread blocks) on a copy stream - a
-// chunk is the literal rows, per-node arrays and edge rows of a contiguous range of graphs - each chunk is scored as soon
-// as it has landed, and its class sums go back on a second copy stream while the next chunk is scored.  Host arrays are
-// validated chunk by chunk, just before they are copied.  Other sets take gtm_dataset_create followed by gtm_score.
+// Upload and scoring of a whole host graph set in one call.  A small set is one copy, one kernel and one wait; larger sets
+// that a tiled kernel covers are pipelined; other sets take gtm_dataset_create followed by gtm_score.
 // The dataset stays valid for later calls either way.
 extern "C" int gtm_dataset_create_scored(gtm_model *m, const gtm_graphs_view *v, int n_types, int32_t *out,
                                          gtm_dataset **dataset_out)
@@ -671,100 +917,27 @@ extern "C" int gtm_dataset_create_scored(gtm_model *m, const gtm_graphs_view *v,
     if (!m->has_state) return fail(GTM_ERR_STATE, "model has no state: call gtm_init_state or gtm_set_ta_state first");
     if (n_types < 1) return fail(GTM_ERR_ARG, "number_of_node_types must be positive");
     GTM_TRY(check_view(v));
+    LaneGuard guard;
+    GTM_TRY(lane_acquire(m->cfg.device, &guard.lane));
     // what a tiled kernel may cover; stream_supported / tile_supported decide once the tiles are made
     const bool pipelined = m->opt_score_kernel != 1 && n_types <= 8 && v->max_number_of_graph_nodes <= 1024 &&
-                           (m->sm.lit_off != nullptr || m->tm.applicable);
+                           (m->sm.applicable || m->tm.applicable) && set_layout(v, m->dm.L0).bytes > kStageSmall;
     gtm_dataset *ds = nullptr;
-    GTM_TRY(dataset_create(m, v, &ds, !pipelined));
-    const int64_t n = ds->n_graphs;
-    int st = GTM_OK;
-    const bool by_stream = pipelined && (m->opt_score_kernel == 0 || m->opt_score_kernel == 2) && stream_supported(ds->sd, n_types);
-    const bool by_tile = pipelined && !by_stream && (m->opt_score_kernel == 0 || m->opt_score_kernel == 3) && tile_supported(ds->td, n_types);
-    if (!by_stream && !by_tile) {
+    GTM_TRY(dataset_create(m, v, &ds, pipelined ? SetCopy::in_ranges : SetCopy::whole, guard.lane));
+    const bool by_stream = pipelined && scores_by_stream(m, ds, n_types);
+    const bool by_tile = pipelined && !by_stream && scores_by_tile(m, ds, n_types);
+    int st;
+    if (by_stream || by_tile) {
+        st = score_in_chunks(m, ds, v, by_stream, n_types, 0, ds->n_graphs, out, guard.lane);
+    } else {
         if (pipelined) {   // the arrays were not copied, but no tiled kernel turned out to cover the set
             gtm_dataset_destroy(ds);
             ds = nullptr;
-            GTM_TRY(dataset_create(m, v, &ds, true));
+            GTM_TRY(dataset_create(m, v, &ds, SetCopy::whole, guard.lane));
         }
-        st = gtm_score(m, ds, n_types, 0, n, out);
-        if (st != GTM_OK) { gtm_dataset_destroy(ds); return st; }
-        *dataset_out = ds;
-        return GTM_OK;
+        st = score_to_host(m, ds, n_types, 0, ds->n_graphs, out, guard.lane);
+        if (st != GTM_OK) cudaStreamSynchronize(m->stream);
     }
-
-    const DevModel &d = m->dm;
-    // tiles of the kernel that will run: first graph of tile t
-    const int n_tiles = by_stream ? ds->sd.n_tiles : ds->td.n_tiles;
-    const int uniform_gpt = by_stream ? ds->sd.graphs_per_tile : ds->td.graphs_per_tile;
-    const std::vector<int> &table = by_stream ? ds->sd.tile_graph_host : ds->td.tile_graph_host;
-    auto tile_first = [&](int t) -> int64_t {
-        if (t >= n_tiles) return n;
-        return uniform_gpt > 0 ? std::min<int64_t>((int64_t)t * uniform_gpt, n) : (int64_t)table[(size_t)t];
-    };
-    const int chunk_tiles = std::max(1, 2 * (by_stream ? ds->sd.grid : ds->td.grid));
-    cudaStream_t in = nullptr, back = nullptr;
-    std::vector<cudaEvent_t> events;
-    int *dev = nullptr;
-    auto body = [&]() -> int {
-        GTM_CU(cudaStreamCreateWithFlags(&in, cudaStreamNonBlocking));
-        GTM_CU(cudaStreamCreateWithFlags(&back, cudaStreamNonBlocking));
-        if (by_stream) GTM_TRY(refresh_lists(m));
-        else GTM_TRY(refresh_tile_lists(m));
-        GTM_TRY(pool_alloc(&dev, (size_t)n * d.K, m->stream));
-        auto event = [&](cudaStream_t s, cudaEvent_t *e) -> int {
-            GTM_CU(cudaEventCreateWithFlags(e, cudaEventDisableTiming));
-            events.push_back(*e);
-            GTM_CU(cudaEventRecord(*e, s));
-            return GTM_OK;
-        };
-        auto up = [&](const u32 *dst, const u32 *src, size_t first, size_t count) -> int {
-            if (count) GTM_CU(cudaMemcpyAsync(const_cast<u32 *>(dst) + first, src + first, count * sizeof(u32), cudaMemcpyHostToDevice, in));
-            return GTM_OK;
-        };
-        cudaEvent_t ready;
-        GTM_TRY(event(m->stream, &ready));                 // allocations, tile tables and literal lists are in stream order
-        GTM_CU(cudaStreamWaitEvent(in, ready, 0));
-        for (int t0 = 0; t0 < n_tiles; t0 += chunk_tiles) {
-            const int64_t g0 = tile_first(t0), g1 = tile_first(t0 + chunk_tiles);
-            if (g1 <= g0) continue;
-            GTM_TRY(validate_graphs(v, g0, g1));            // overlaps the copies of the chunks before
-            const size_t cnt = (size_t)(g1 - g0);
-            const size_t v0 = v->node_index[g0], v1 = g1 < n ? (size_t)v->node_index[g1] : (size_t)v->total_nodes;
-            const size_t e0 = v->edge_index[v0], e1 = v1 < (size_t)v->total_nodes ? (size_t)v->edge_index[v1] : (size_t)v->total_edges;
-            GTM_TRY(up(ds->dg.X, v->X, v0 * d.L0, (v1 - v0) * d.L0));
-            GTM_TRY(up(ds->dg.node_type, v->node_type, v0, v1 - v0));
-            GTM_TRY(up(ds->dg.degree, v->number_of_graph_node_edges, v0, v1 - v0));
-            GTM_TRY(up(ds->dg.edge_index, v->edge_index, v0, v1 - v0));
-            if (e1 > e0) GTM_TRY(up(ds->dg.edge, v->edge, 2 * e0, 2 * (e1 - e0)));
-            // one element more: a tile ends where the next graph's nodes begin
-            GTM_TRY(up(ds->dg.node_index, v->node_index, (size_t)g0, cnt + (g1 < n ? 1 : 0)));
-            GTM_TRY(up(ds->dg.n_nodes, v->number_of_graph_nodes, (size_t)g0, cnt));
-            cudaEvent_t landed, scored;
-            GTM_TRY(event(in, &landed));
-            GTM_CU(cudaStreamWaitEvent(m->stream, landed, 0));
-            if (by_stream) GTM_TRY(stream_score(m->sm, ds->sd, d, ds->dg, n_types, g0, (int64_t)cnt, dev + (size_t)g0 * d.K, m->stream));
-            else GTM_TRY(tile_score(m->tm, ds->td, d, ds->dg, n_types, g0, (int64_t)cnt, dev + (size_t)g0 * d.K, m->score_error, m->stream));
-            GTM_TRY(event(m->stream, &scored));
-            GTM_CU(cudaStreamWaitEvent(back, scored, 0));
-            GTM_CU(cudaMemcpyAsync(out + (size_t)g0 * d.K, dev + (size_t)g0 * d.K, cnt * d.K * sizeof(int), cudaMemcpyDeviceToHost, back));
-        }
-        GTM_TRY(derive_edge_ranges(ds, v->number_of_graphs));       // every array has been queued before this point of the stream
-        GTM_CU(cudaMemcpyAsync(m->flag_host, m->score_error, sizeof(int), cudaMemcpyDeviceToHost, m->stream));
-        GTM_CU(cudaStreamSynchronize(in));
-        GTM_CU(cudaStreamSynchronize(back));
-        GTM_CU(cudaStreamSynchronize(m->stream));
-        return score_flag_status(m, *m->flag_host);
-    };
-    st = body();
-    if (st != GTM_OK) {                                    // nothing may still be reading the host arrays when the call returns
-        if (in) cudaStreamSynchronize(in);
-        if (back) cudaStreamSynchronize(back);
-        cudaStreamSynchronize(m->stream);
-    }
-    if (dev) cudaFreeAsync(dev, m->stream);
-    for (cudaEvent_t e : events) cudaEventDestroy(e);
-    if (in) cudaStreamDestroy(in);
-    if (back) cudaStreamDestroy(back);
     if (st != GTM_OK) { gtm_dataset_destroy(ds); return st; }
     *dataset_out = ds;
     return GTM_OK;
@@ -779,18 +952,24 @@ static int transform_common(gtm_model *m, gtm_dataset *ds, int n_types, int64_t 
     if (count == 0) return GTM_OK;
     int *sums_dev = nullptr, *co_dev = nullptr, *no_dev = nullptr;
     const size_t n_sums = (size_t)count * m->dm.K, n_co = (size_t)count * m->dm.C, n_no = n_co * (size_t)node_stride;
+    LaneGuard guard;
+    GTM_TRY(lane_acquire(m->cfg.device, &guard.lane));
     int st = pool_alloc(&sums_dev, n_sums, m->stream);
     if (st == GTM_OK && clause_out) st = pool_alloc(&co_dev, n_co, m->stream);
     if (st == GTM_OK && node_out) st = pool_alloc(&no_dev, n_no, m->stream);
     if (st == GTM_OK) st = launch_score_general(m, ds, n_types, first, count, sums_dev, co_dev, no_dev, node_stride);
-    cudaError_t e = cudaSuccess;
-    if (st == GTM_OK && sums_out) e = cudaMemcpyAsync(sums_out, sums_dev, n_sums * sizeof(int), cudaMemcpyDeviceToHost, m->stream);
-    if (st == GTM_OK && e == cudaSuccess && clause_out) e = cudaMemcpyAsync(clause_out, co_dev, n_co * sizeof(int), cudaMemcpyDeviceToHost, m->stream);
-    if (st == GTM_OK && e == cudaSuccess && node_out) e = cudaMemcpyAsync(node_out, no_dev, n_no * sizeof(int), cudaMemcpyDeviceToHost, m->stream);
+    auto down = [&](int32_t *host, const int *dev, size_t n) {
+        if (st == GTM_OK && host) st = stage_down(guard.lane, host, dev, n * sizeof(int), host_is_pinned(host), m->stream);
+    };
+    down(sums_out, sums_dev, n_sums);
+    down(clause_out, co_dev, n_co);
+    down(node_out, no_dev, n_no);
     if (sums_dev) cudaFreeAsync(sums_dev, m->stream);
     if (co_dev) cudaFreeAsync(co_dev, m->stream);
     if (no_dev) cudaFreeAsync(no_dev, m->stream);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(m->stream);
+    if (st == GTM_OK) st = stage_down_finish(guard.lane);
+    if (st != GTM_OK) stage_abandon(guard.lane);
+    const cudaError_t e = cudaStreamSynchronize(m->stream);
     if (st != GTM_OK) return st;
     GTM_CU(e);
     return GTM_OK;
@@ -837,6 +1016,7 @@ extern "C" int gtm_debug_evaluate(gtm_model *m, gtm_dataset *ds, int n_types, in
     GTM_TRY(bind(m));
     GTM_TRY(check_range(m, ds, n_types, graph, 1));
     const DevModel &d = m->dm;
+    GTM_TRY(ensure_fit_scratch(ds));
     std::vector<u32> nn(1), ni(1);
     GTM_CU(cudaMemcpy(nn.data(), ds->dg.n_nodes + graph, sizeof(u32), cudaMemcpyDeviceToHost));
     const int n = (int)nn[0], words = (n + 31) / 32;
@@ -1053,10 +1233,9 @@ extern "C" int gtm_check_skipped_graphs(gtm_model *m, int *skipped_out)
     GTM_TRY(bind(m));
     if (!skipped_out) return fail(GTM_ERR_ARG, "skipped_out is null");
     GTM_CU(cudaStreamSynchronize(m->stream));
-    int flag = 0;
-    GTM_CU(cudaMemcpy(&flag, m->score_error, sizeof(int), cudaMemcpyDeviceToHost));
-    if (flag) GTM_CU(cudaMemset(m->score_error, 0, sizeof(int)));
+    const int flag = *(volatile int *)m->score_error;
+    if (flag == 2) return score_flag_status(m);
+    *(volatile int *)m->score_error = 0;
     *skipped_out = flag == 1;
-    if (flag == 2) return score_flag_status(m, flag);
     return GTM_OK;
 }

@@ -19,8 +19,8 @@ struct gtm_model {
     u32 *recorded = nullptr;
     // learning-kernel buffers
     int fit_grid = 0, fit_block = 512;
-    int *flag_host = nullptr;                 // page-locked landing place of score_error
-    int *score_error = nullptr;               // raised by scoring kernels that skipped a malformed graph (device-pointer inputs)
+    int *score_error = nullptr;               // raised by scoring kernels that skipped a malformed graph (device-pointer inputs); page-locked
+                                              // host memory, so that the host reads it without a copy
     int *error = nullptr, *clause_node = nullptr, *update = nullptr, *class_sum_tap = nullptr;
     unsigned long long *exchange = nullptr;   // vote exchange area of a single-GPU fit (exchange_bytes(1, K))
     int opt_fit_block_clauses = 0;            // > 0: clauses per thread block of the state-resident kernel (0: automatic)
@@ -91,5 +91,6 @@ struct gtm_dataset {
 int fit_grid_for_global_state(const DevModel &d, int sm_count, int block, int *grid_out);
 int launch_fit(gtm_model *m, gtm_dataset *ds, int n_types, const int *Y_dev, int64_t first, int64_t count, int epochs,
                int eval_only);
+int ensure_fit_scratch(gtm_dataset *ds);
 void fit_comm_release(gtm_dataset *ds);
 size_t exchange_bytes(int world, int K);

@@ -1,0 +1,65 @@
+// Host side of the copies between a caller's pageable arrays and the device: a few copy threads, page-locked staging
+// buffers, copy streams and events, all kept between calls (gtm_stage.cu).
+//
+// A cudaMemcpyAsync from or to pageable memory is one host thread copying through a small buffer of the driver: 6 to
+// 12 GB/s, with the copy engine idle most of the time, and a fresh result array costs that thread a page fault every
+// 4 KB on top.  Here a few threads copy pieces to or from page-locked buffers while the copy engine moves the pieces
+// before: 120,000 images of 32 bytes up and their 4.8 MB of class sums down took 0.9 ms through pageable copies.
+#pragma once
+#include <cuda_runtime.h>
+#include <stddef.h>
+
+constexpr size_t kStagePiece = (size_t)4 << 20;      // bytes of one staging buffer
+constexpr int kStageSlots = 4;                       // staging buffers per direction
+constexpr size_t kStageSmall = (size_t)256 << 10;    // sets and results up to this size go through the small buffer
+
+// Runs fn(ctx, i) for i in [0, count) on the copy threads and the calling thread; returns when all are done.  When the
+// threads are busy with another caller's work, the calling thread does everything itself.
+void host_parallel(int count, void (*fn)(void *ctx, int i), void *ctx);
+
+// memcpy by several threads when it is large enough to pay; `past_caches` (64-byte aligned dst): with streaming stores.
+void host_copy(void *dst, const void *src, size_t bytes, bool past_caches);
+
+struct StageSlot {
+    char *host = nullptr;
+    cudaEvent_t done = nullptr;
+    bool busy = false;
+    void *dst = nullptr;         // a piece on its way down: where it goes once it has landed
+    size_t bytes = 0;
+};
+
+// What one call borrows: copy streams, events, staging buffers.  Lives on one device.
+struct StageLane {
+    int device = -1;
+    cudaStream_t in = nullptr, back = nullptr, aux = nullptr;    // copies up, copies down, a second stream for kernels
+    cudaEvent_t event[4] = {};   // free for the borrower's use
+    char *small = nullptr;       // [2][kStageSmall] page-locked: packed inputs, results
+    char *big = nullptr;         // one allocation behind the slots' buffers, made on first use
+    StageSlot up[kStageSlots], down[kStageSlots];
+    int up_next = 0, down_next = 0;
+};
+
+// A lane of the device, from the free list or new.  At most kLanesKept lanes per device stay on the list; all of them,
+// and the copy threads, are given back when the last model is destroyed (stage_retain / stage_drop).
+int lane_acquire(int device, StageLane **out);
+void lane_release(StageLane *lane);
+void stage_retain();
+void stage_drop();
+
+struct LaneGuard {
+    StageLane *lane = nullptr;
+    ~LaneGuard() { if (lane) lane_release(lane); }
+};
+
+bool host_is_pinned(const void *p);
+
+// Queues a copy of `bytes` to the device on stream s.  The source may be reused when the call returns, unless it is
+// page-locked memory of the caller: then it must stay until the stream has passed the copy.
+int stage_up(StageLane *lane, void *dst, const void *src, size_t bytes, bool pinned, cudaStream_t s);
+
+// Queues a copy of `bytes` to the host on stream s; dst holds them once stage_down_finish has returned.
+int stage_down(StageLane *lane, void *dst, const void *src, size_t bytes, bool pinned, cudaStream_t s);
+int stage_down_finish(StageLane *lane);
+
+// After an error: waits until nothing of the lane is in flight and forgets it.
+void stage_abandon(StageLane *lane);

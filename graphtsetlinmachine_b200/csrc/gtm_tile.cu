@@ -134,7 +134,7 @@ struct TileArgs {
     int64_t first, count;               // graphs written: [first, first+count)
     int64_t n_graphs;
     int *class_sums;                    // [count][K]
-    unsigned *tile_counter;             // dynamic tile scheduler (zeroed before launch)
+    unsigned *tile_counter;             // tiles handed out beyond the first of every CTA; left at zero
     int TNC, PS, words_a, words_b, stage_rows, gmax;
     int rot_step;                       // message transposition: block column j is read rotated by (rot_step * j) & 31
     const TileLayer *layers;            // [D]
@@ -273,11 +273,8 @@ __global__ void __launch_bounds__(kTileThreads, 2) tile_score_kernel(DevModel m,
     __syncthreads();
     unsigned parity = 0;
 
-    while (true) {
-        if (tid == 0) misc[0] = a.tile_lo + (int)atomicAdd(a.tile_counter, 1u);
-        __syncthreads();
-        const int tile = misc[0];
-        if (tile >= a.tile_hi) break;
+    const int more = a.tile_hi - a.tile_lo - (int)gridDim.x;         // tiles beyond the first of every CTA
+    for (int tile = a.tile_lo + (int)blockIdx.x; tile < a.tile_hi;) {
         const int g0 = a.tile_graph ? a.tile_graph[tile] : (int)min((int64_t)tile * a.graphs_per_tile, a.n_graphs);
         const int g1 = a.tile_graph ? a.tile_graph[tile + 1] : (int)min((int64_t)(tile + 1) * a.graphs_per_tile, a.n_graphs);
         const int ng = g1 - g0;
@@ -325,7 +322,7 @@ __global__ void __launch_bounds__(kTileThreads, 2) tile_score_kernel(DevModel m,
                 lead = (int)(w0 - a0);
                 if (tid == 0) bulk_copy_to_shared(smem_u32(bufB), g.X + a0, (unsigned)((a1 - a0) * sizeof(u32)), bar);
                 if (!mbar_wait(bar, parity)) {
-                    if (a.error) atomicExch(a.error, 2);
+                    if (a.error) *(volatile int *)a.error = 2;
                     mbar_wait(bar, parity);           // the copy may still be in flight: give it one more bounded wait
                 }
                 parity ^= 1u;
@@ -554,7 +551,15 @@ __global__ void __launch_bounds__(kTileThreads, 2) tile_score_kernel(DevModel m,
             const int64_t gi = (int64_t)g0 + gl;
             if (gi >= a.first && gi < a.first + a.count) a.class_sums[(size_t)(gi - a.first) * m.K + k] = sums[gl * KP + k];
         }
-        __syncthreads();                              // the shared tables are rewritten by the next tile
+        // ---- next tile: the CTA whose request is the last of the launch leaves the counter at zero ----
+        if (more <= 0) break;
+        if (tid == 0) {
+            const int got = (int)atomicAdd(a.tile_counter, 1u);
+            if (got == more + (int)gridDim.x - 1) *a.tile_counter = 0u;
+            misc[0] = a.tile_lo + (int)gridDim.x + got;
+        }
+        __syncthreads();                              // misc; the shared tables are rewritten by the next tile
+        tile = misc[0];
     }
 }
 
@@ -591,13 +596,15 @@ int tile_model_create(TileModel *tm, const DevModel &d)
         GTM_TRY(dev_alloc(&tm->order[l], (size_t)d.C));
         GTM_TRY(dev_alloc(&tm->blk_off[l], (size_t)((d.C + 31) / 32) + 1));
     }
+    GTM_TRY(dev_alloc(&tm->counters, 2));
+    GTM_CU(cudaMemset(tm->counters, 0, 2 * sizeof(unsigned)));
     tm->applicable = true;
     return GTM_OK;
 }
 
 void tile_model_destroy(TileModel *tm)
 {
-    cudaFree(tm->Wt); cudaFree(tm->hvm); cudaFree(tm->layers);
+    cudaFree(tm->Wt); cudaFree(tm->hvm); cudaFree(tm->layers); cudaFree(tm->counters); cudaFree(tm->surv_r[0]); cudaFree(tm->surv_r[1]);
     for (int l = 0; l < kMaxDepth; ++l) { cudaFree(tm->cnt[l]); cudaFree(tm->order[l]); cudaFree(tm->blk_off[l]); cudaFree(tm->list[l]); }
     *tm = TileModel();
 }
@@ -743,7 +750,6 @@ int tile_data_create(TileData *td, const TileModel &tm, const DevModel &d, const
         GTM_CU(cudaMemcpyAsync(td->tile_graph, tg.data(), tg.size() * sizeof(int), cudaMemcpyHostToDevice, s));
         GTM_TRY(pool_alloc(&td->gpos, (size_t)N, s));
         GTM_CU(cudaMemcpyAsync(td->gpos, gpos.data(), (size_t)N * sizeof(unsigned short), cudaMemcpyHostToDevice, s));
-        GTM_CU(cudaStreamSynchronize(s));             // gpos goes out of scope
     }
     plan = tile_plan(d, TNC, td->gmax);
     td->PS = plan.PS;
@@ -756,7 +762,6 @@ int tile_data_create(TileData *td, const TileModel &tm, const DevModel &d, const
     GTM_CU(cudaOccupancyMaxActiveBlocksPerMultiprocessorWithFlags(&per_sm, fn, kTileThreads, td->smem, 0));
     if (per_sm < 1) { tile_data_destroy(td); return GTM_OK; }
     td->grid = std::max(1, std::min(sm_count * per_sm, td->n_tiles));
-    GTM_TRY(pool_alloc(&td->tile_counter, 1, s));
     td->n_graphs = N;
     td->supported = 1;
     return GTM_OK;
@@ -766,20 +771,16 @@ void tile_data_destroy(TileData *td)
 {
     if (td->tile_graph) cudaFreeAsync(td->tile_graph, td->stream);
     if (td->gpos) cudaFreeAsync(td->gpos, td->stream);
-    if (td->tile_counter) cudaFreeAsync(td->tile_counter, td->stream);
-    if (td->surv_r) cudaFreeAsync(td->surv_r, td->stream);
-    td->tile_graph = nullptr; td->gpos = nullptr; td->tile_counter = nullptr; td->surv_r = nullptr;
+    td->tile_graph = nullptr; td->gpos = nullptr;
     td->supported = 0;
 }
 
 bool tile_supported(const TileData &td, int n_types) { return td.supported != 0 && n_types <= kTileMaxTypes; }
 
-int tile_score(const TileModel &tm, TileData &td, const DevModel &d, const DevGraphs &dg, int n_types, int64_t first,
-               int64_t count, int *sums_dev, int *error_dev, cudaStream_t s)
+int tile_score(TileModel *model, const TileData &td, const DevModel &d, const DevGraphs &dg, int n_types, int64_t first,
+               int64_t count, int *sums_dev, int *error_dev, int lane, cudaStream_t s)
 {
-    const int U = (td.TNC / 4 + 1) / 2;
-    if (!td.surv_r)            // node bits of every clause between layers, per resident CTA, layer parity and quad pair; allocated on first use
-        GTM_TRY(pool_alloc(&td.surv_r, 2 * (size_t)td.grid * 2 * U * d.C, s));
+    TileModel &tm = *model;
     DevGraphs g = dg;
     g.n_types = n_types;
     TileArgs a;
@@ -798,16 +799,23 @@ int tile_score(const TileModel &tm, TileData &td, const DevModel &d, const DevGr
     }
     a.tile_lo = lo; a.tile_hi = hi;
     a.first = first; a.count = count; a.n_graphs = td.n_graphs;
-    a.class_sums = sums_dev; a.tile_counter = td.tile_counter;
+    a.class_sums = sums_dev; a.tile_counter = tm.counters + lane;
     a.TNC = td.TNC; a.PS = td.PS; a.words_a = td.words_a; a.words_b = td.words_b; a.stage_rows = td.stage_rows; a.gmax = td.gmax;
     int inv = 1;                                       // inverse of the (odd) message row stride modulo 32
     while ((td.PS * inv) % 32 != 1) inv += 2;
     a.rot_step = ((32 / td.TNC) * inv) & 31;
     a.layers = tm.layers; a.Wt = tm.Wt; a.KROW = tm.KROW; a.hvm = tm.hvm;
-    a.surv_r = td.surv_r;
+    const int grid = std::max(1, std::min(td.grid, hi - lo)), U = (td.TNC / 4 + 1) / 2;
+    // node bits of every clause between layers, per CTA, layer parity and quad pair: kept by the model, grows on demand
+    const size_t need = 2 * (size_t)grid * 2 * U * d.C;
+    if (need > tm.surv_cap[lane]) {
+        cudaFree(tm.surv_r[lane]);                     // waits for the kernels that use it
+        tm.surv_r[lane] = nullptr; tm.surv_cap[lane] = 0;
+        GTM_TRY(dev_alloc(&tm.surv_r[lane], need));
+        tm.surv_cap[lane] = need;
+    }
+    a.surv_r = tm.surv_r[lane];
     a.error = error_dev;
-    GTM_CU(cudaMemsetAsync(td.tile_counter, 0, sizeof(unsigned), s));
-    const int grid = std::max(1, std::min(td.grid, hi - lo));
     DevModel dm = d;
     void *args[] = {&dm, &g, &a};
     GTM_CU(cudaLaunchKernel(tile_kernel_for(d.K), dim3(grid), dim3(kTileThreads), args, td.smem, s));

@@ -29,6 +29,9 @@ struct TileModel {
     int *Wt = nullptr;            // [C][KROW] weights, clause-major
     u32 *hvm = nullptr;           // [C][MB] hypervector bits reduced modulo the message size
     TileLayer *layers = nullptr;  // [D] device copy of the pointers above
+    unsigned *counters = nullptr; // [2] tile counters of two launches side by side
+    uint4 *surv_r[2] = {};        // per launch: [grid][2][quad pairs][C][2] node bits of every clause on the pair's two quads after a layer
+    size_t surv_cap[2] = {};
 };
 
 struct TileData {
@@ -44,8 +47,6 @@ struct TileData {
     int *tile_graph = nullptr;          // [n_tiles+1] first graph of every tile (NULL for uniform sets)
     unsigned short *gpos = nullptr;     // [N] first node slot of every graph inside its tile (NULL for uniform sets)
     std::vector<int> tile_graph_host;
-    unsigned *tile_counter = nullptr;
-    uint4 *surv_r = nullptr;            // [grid][2][quad pairs][C][2] node bits of every clause on the pair's two quads after a layer
     cudaStream_t stream = nullptr;
     int grid = 0;
     size_t smem = 0;
@@ -59,7 +60,8 @@ int tile_data_create(TileData *td, const TileModel &tm, const DevModel &d, const
                      int sm_count, cudaStream_t s);
 void tile_data_destroy(TileData *td);
 bool tile_supported(const TileData &td, int n_types);
-int tile_score(const TileModel &tm, TileData &td, const DevModel &d, const DevGraphs &dg, int n_types, int64_t first,
-               int64_t count, int *sums_dev, int *error_dev, cudaStream_t s);
+// `lane` (0 or 1): launches that may run side by side, on disjoint tiles, take different ones.
+int tile_score(TileModel *model, const TileData &td, const DevModel &d, const DevGraphs &dg, int n_types, int64_t first,
+               int64_t count, int *sums_dev, int *error_dev, int lane, cudaStream_t s);
 
 }  // namespace gtm

@@ -1,0 +1,73 @@
+"""Result arrays in recycled page-locked memory.
+
+A result of a few megabytes in a fresh numpy array costs a page fault per page and a copy out of a staging buffer; in
+page-locked memory the copy engine writes it directly, in the time of the transfer.  Page-locking is slow (about a
+millisecond for 4 MB), so the memory of an array that nobody refers to any more is kept for the next result.
+"""
+
+import collections
+import ctypes as C
+import threading
+import weakref
+
+import numpy as np
+
+from . import _lib
+
+SMALLEST, LARGEST = 64 << 10, 16 << 20      # bytes of an array that is worth it / that is not too much to lock
+MOST = 128 << 20                            # bytes locked at a time, arrays in use included
+
+_free = collections.defaultdict(collections.deque)      # size class -> addresses
+_lock = threading.Lock()
+_locked = 0
+
+
+def _size_class(nbytes):
+    """Next size of the form 2^k or 1.5 * 2^k: at most a third is unused."""
+    size = 1 << (nbytes - 1).bit_length()
+    return size * 3 // 4 if nbytes <= size * 3 // 4 else size
+
+
+def _give_back(address, size):
+    _free[size].append(address)             # atomic: may run in the garbage collector of any thread
+
+
+def _take(size):
+    """Address of a free block, or a newly locked one while the limit allows; 0 when it does not."""
+    global _locked
+    try:
+        return _free[size].popleft()
+    except IndexError:
+        pass
+    lib = _lib.load()
+    with _lock:
+        if _locked + size > MOST:           # free blocks of other sizes make room
+            for other, blocks in list(_free.items()):
+                while blocks and _locked + size > MOST:
+                    try:
+                        address = blocks.popleft()
+                    except IndexError:
+                        break
+                    lib.gtm_host_free(address)
+                    _locked -= other
+        if _locked + size > MOST:
+            return 0
+        out = C.c_void_p()
+        if lib.gtm_host_alloc(size, C.byref(out)) != 0:
+            return 0
+        _locked += size
+        return out.value
+
+
+def empty(shape, dtype):
+    """Like ``numpy.empty``."""
+    nbytes = int(np.prod(shape, dtype=np.int64)) * np.dtype(dtype).itemsize
+    if not SMALLEST <= nbytes <= LARGEST:
+        return np.empty(shape, dtype=dtype)
+    size = _size_class(nbytes)
+    address = _take(size)
+    if not address:
+        return np.empty(shape, dtype=dtype)
+    block = (C.c_ubyte * size).from_address(address)    # every array made from it keeps it alive
+    weakref.finalize(block, _give_back, address, size).atexit = False
+    return np.frombuffer(block, dtype=dtype, count=nbytes // np.dtype(dtype).itemsize).reshape(shape)

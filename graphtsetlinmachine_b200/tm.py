@@ -21,7 +21,7 @@ import sys
 
 import numpy as np
 
-from . import _lib
+from . import _lib, hostmem
 
 __all__ = ["CommonTsetlinMachine", "MultiClassGraphTsetlinMachine", "MultiOutputGraphTsetlinMachine",
            "GraphTsetlinMachine"]
@@ -33,6 +33,13 @@ def _ptr(a):
 
 def _u32(a):
     return np.ascontiguousarray(a, dtype=np.uint32)
+
+
+def _same_set(a, b):
+    """Whether two graph-set signatures (digests; an empty array stands for none) are equal."""
+    if isinstance(a, bytes) and isinstance(b, bytes):
+        return a == b
+    return np.array_equal(a, b)
 
 
 class _Dataset:
@@ -273,7 +280,7 @@ class CommonTsetlinMachine:
         return self.number_of_ta_chunks if layer == 0 else self.number_of_message_chunks
 
     def _download_ta(self, layer):
-        out = np.empty(self.number_of_clauses * self._layer_chunks(layer) * self.number_of_state_bits, dtype=np.uint32)
+        out = hostmem.empty(self.number_of_clauses * self._layer_chunks(layer) * self.number_of_state_bits, dtype=np.uint32)
         _lib.check(self._lib.gtm_get_ta_state(self._model, layer, _ptr(out)))
         return out
 
@@ -290,7 +297,7 @@ class CommonTsetlinMachine:
             _lib.check(self._lib.gtm_init_state(self._model, 1))
         elif not incremental:
             _lib.check(self._lib.gtm_init_state(self._model, 0))   # message layers keep their state (tm.py:524-526)
-        if not np.array_equal(self.graphs_signature_train, graphs.signature):
+        if not _same_set(self.graphs_signature_train, graphs.signature):
             self.graphs_signature_train = graphs.signature
             if self._train_set is not None:
                 self._train_set.close()
@@ -323,7 +330,7 @@ class CommonTsetlinMachine:
         if not self.initialized:
             print("Error: Model not trained.")
             sys.exit(-1)
-        if not np.array_equal(self.graphs_signature_test, graphs.signature):
+        if not _same_set(self.graphs_signature_test, graphs.signature):
             self.graphs_signature_test = graphs.signature
             if self._test_set is not None:
                 self._test_set.close()
@@ -335,10 +342,11 @@ class CommonTsetlinMachine:
         if not self.initialized:
             print("Error: Model not trained.")
             sys.exit(-1)
-        class_sum = np.zeros((graphs.number_of_graphs, self.number_of_outputs), dtype=np.int32) if out is None else out
+        # the engine writes every element of its results
+        class_sum = hostmem.empty((graphs.number_of_graphs, self.number_of_outputs), dtype=np.int32) if out is None else out
         assert class_sum.dtype == np.int32 and class_sum.flags.c_contiguous
         assert class_sum.shape == (graphs.number_of_graphs, self.number_of_outputs)
-        if not np.array_equal(self.graphs_signature_test, graphs.signature):
+        if not _same_set(self.graphs_signature_test, graphs.signature):
             # a new graph set: upload and scoring in one pipelined call; the set stays resident for later calls
             if self._test_set is not None:
                 self._test_set.close()
@@ -354,8 +362,8 @@ class CommonTsetlinMachine:
     def transform(self, graphs):
         """tm.py:814-851: (clause outputs int32[N][clauses], class sums)."""
         self._score_init(graphs)
-        class_sum = np.zeros((graphs.number_of_graphs, self.number_of_outputs), dtype=np.int32)
-        transformed_X = np.zeros((graphs.number_of_graphs, self.number_of_clauses), dtype=np.int32)
+        class_sum = hostmem.empty((graphs.number_of_graphs, self.number_of_outputs), dtype=np.int32)
+        transformed_X = hostmem.empty((graphs.number_of_graphs, self.number_of_clauses), dtype=np.int32)
         _lib.check(self._lib.gtm_transform(self._model, self._test_set.handle, int(graphs.number_of_node_types()), 0,
                                            int(graphs.number_of_graphs), _ptr(transformed_X), _ptr(class_sum)))
         return transformed_X, class_sum
@@ -364,8 +372,8 @@ class CommonTsetlinMachine:
         """tm.py:853-900: (per-node clause outputs int32[N][clauses][max nodes], class sums)."""
         self._score_init(graphs)
         n_max = int(np.max(graphs.number_of_graph_nodes))
-        class_sum = np.zeros((graphs.number_of_graphs, self.number_of_outputs), dtype=np.int32)
-        transformed_X = np.zeros((graphs.number_of_graphs, self.number_of_clauses, n_max), dtype=np.int32)
+        class_sum = hostmem.empty((graphs.number_of_graphs, self.number_of_outputs), dtype=np.int32)
+        transformed_X = hostmem.empty((graphs.number_of_graphs, self.number_of_clauses, n_max), dtype=np.int32)
         _lib.check(self._lib.gtm_transform_nodewise(self._model, self._test_set.handle, int(graphs.number_of_node_types()),
                                                     0, int(graphs.number_of_graphs), n_max, _ptr(transformed_X), _ptr(class_sum)))
         return transformed_X, class_sum

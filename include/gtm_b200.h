@@ -147,13 +147,18 @@ int gtm_score(gtm_model *model, gtm_dataset *dataset, int number_of_node_types, 
 
 /* Upload + scoring of a whole graph set in one call (the reference does both inside `_score`: tm.py:759-784 uploads,
  * tm.py:786-812 scores): class_sums_out int32[number_of_graphs][CLASSES]; *dataset_out is the resident graph set, as
- * from gtm_dataset_create, for later calls.  Sets of single-node graphs are pipelined - chunks are scored while the next
+ * from gtm_dataset_create, for later calls.  Larger sets that a tiled kernel covers are pipelined - chunks are scored while the next
  * chunk is still being copied and the previous chunk's sums are on their way back; page-locked host arrays make the
  * copies asynchronous.  Host pointers are borrowed for the call only. */
 int gtm_dataset_create_scored(gtm_model *model, const gtm_graphs_view *graphs, int number_of_node_types,
                               int32_t *class_sums_out, gtm_dataset **dataset_out);
 int gtm_score_device(gtm_model *model, gtm_dataset *dataset, int number_of_node_types, int64_t first,
                      int64_t count, int32_t *class_sums_device);
+
+/* Page-locked host memory (the role of pycuda's pagelocked_empty; no counterpart call in the reference): arrays in it are
+ * copied from and to the device directly, other arrays through the library's own page-locked buffers. */
+int gtm_host_alloc(uint64_t bytes, void **out);
+int gtm_host_free(void *p);
 
 /* Scoring for callers that must not allocate device memory.  NO COUNTERPART IN THE REFERENCE (it allocates per graph
  * set with cuda.mem_alloc, tm.py:759-784).
