@@ -131,6 +131,7 @@ extern "C" int gtm_create(const gtm_config *cfg, gtm_model **out)
     if (st == GTM_OK) st = dev_alloc(&m->phase_cycles, 8);
     if (st != GTM_OK) { gtm_destroy(m); return st; }
     d.hv = hv;
+    m->hv_host.assign((size_t)d.C * d.MB, 0);
     cudaMemset(hv, 0, (size_t)d.C * d.MB * sizeof(u32));
     cudaMemset(d.draw_pos, 0, (size_t)d.C * sizeof(u64));
     cudaMemset(d.weights, 0, (size_t)d.K * d.C * sizeof(int));
@@ -154,7 +155,7 @@ extern "C" int gtm_destroy(gtm_model *m)
     cudaFree(m->dm.ta0); cudaFree(m->dm.tam);
     cudaFree(m->dm.weights); cudaFree((void *)m->dm.hv); cudaFree(m->dm.draw_pos); cudaFree(m->recorded);
     cudaFree(m->exchange); cudaFree(m->error); cudaFree(m->clause_node); cudaFree(m->update);
-    cudaFree(m->class_sum_tap); cudaFree(m->barrier); cudaFree(m->phase_cycles);
+    cudaFree(m->class_sum_tap); cudaFree(m->barrier); cudaFree(m->phase_cycles); cudaFree(m->chain_sync); cudaFree(m->hv_off); cudaFree(m->hv_clause);
     stream_model_destroy(&m->sm);
     tile_model_destroy(&m->tm);
     if (m->score_error) cudaFreeHost(m->score_error);
@@ -272,6 +273,8 @@ extern "C" int gtm_set_hypervectors(gtm_model *m, const uint32_t *hv)
     if (!hv) return fail(GTM_ERR_ARG, "hypervectors is null");
     GTM_CU(cudaMemcpyAsync((void *)m->dm.hv, hv, (size_t)m->dm.C * m->dm.MB * sizeof(u32), cudaMemcpyHostToDevice, m->stream));
     GTM_CU(cudaStreamSynchronize(m->stream));
+    m->hv_host.assign(hv, hv + (size_t)m->dm.C * m->dm.MB);
+    m->hv_lists_valid = false;
     m->lists_dirty = true; ++m->state_version;
     return GTM_OK;
 }

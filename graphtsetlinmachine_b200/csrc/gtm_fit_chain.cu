@@ -1,0 +1,165 @@
+// Launch logic of the learning kernel for one GPU (gtm_fit_chain.cuh).
+#include <cuda_runtime.h>
+
+#include <algorithm>
+#include <cstring>
+#include <vector>
+
+#include "gtm_handles.h"
+#include "gtm_fit_chain.cuh"
+
+const void *fit_chain_kernel_rw1(bool one_layer, bool hybrid);
+const void *fit_chain_kernel_rw4(bool one_layer, bool hybrid);
+const void *fit_chain_kernel_rw16(bool one_layer, bool hybrid);
+const void *fit_chain_kernel_rw32(bool one_layer, bool hybrid);
+
+static const void *chain_kernel_for(int rw, bool one_layer, bool hybrid)
+{
+    return rw == 1 ? fit_chain_kernel_rw1(one_layer, hybrid) : rw == 4 ? fit_chain_kernel_rw4(one_layer, hybrid)
+         : rw == 16 ? fit_chain_kernel_rw16(one_layer, hybrid) : fit_chain_kernel_rw32(one_layer, hybrid);
+}
+
+__global__ void largest_edge_type_kernel(const u32 *edge, size_t edges, u32 *out)
+{
+    u32 most = 0;
+    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < edges; i += (size_t)gridDim.x * blockDim.x) most = max(most, edge[2 * i + 1]);
+    most = __reduce_max_sync(kFull, most);
+    if ((threadIdx.x & 31) == 0 && most > 0) atomicMax(out, most);
+}
+
+// Message buffers of a set, the largest edge type, and the clauses of every message bit: made on the first fit.
+static int chain_prepare(gtm_model *m, gtm_dataset *ds, int rw)
+{
+    const DevModel &d = m->dm;
+    if (!m->chain_sync) GTM_TRY(dev_alloc(&m->chain_sync, (size_t)2 * d.K + 1));
+    if (d.D == 1) return GTM_OK;
+    if (!m->hv_lists_valid) {
+        std::vector<int> off((size_t)d.MS + 1, 0), list((size_t)d.C * d.MB);
+        for (u32 h : m->hv_host) ++off[h % (u32)d.MS + 1];
+        for (int b = 0; b < d.MS; ++b) off[(size_t)b + 1] += off[(size_t)b];
+        std::vector<int> at(off.begin(), off.end() - 1);
+        for (size_t i = 0; i < m->hv_host.size(); ++i) list[(size_t)at[m->hv_host[i] % (u32)d.MS]++] = (int)(i / (size_t)d.MB);
+        if (!m->hv_off) {
+            GTM_TRY(dev_alloc(&m->hv_off, off.size()));
+            GTM_TRY(dev_alloc(&m->hv_clause, list.size()));
+        }
+        GTM_CU(cudaMemcpyAsync(m->hv_off, off.data(), off.size() * sizeof(int), cudaMemcpyHostToDevice, m->stream));
+        GTM_CU(cudaMemcpyAsync(m->hv_clause, list.data(), list.size() * sizeof(int), cudaMemcpyHostToDevice, m->stream));
+        GTM_CU(cudaStreamSynchronize(m->stream));
+        m->hv_lists_valid = true;
+    }
+    if (ds->largest_edge_type < 0) {
+        u32 *out, most = 0;
+        GTM_TRY(pool_alloc(&out, 1, m->stream));
+        GTM_CU(cudaMemsetAsync(out, 0, sizeof(u32), m->stream));
+        if (ds->total_edges > 0) largest_edge_type_kernel<<<(unsigned)std::min<int64_t>((ds->total_edges + 255) / 256, 1184), 256, 0, m->stream>>>(ds->dg.edge, (size_t)ds->total_edges, out);
+        GTM_CU(cudaMemcpyAsync(&most, out, sizeof(u32), cudaMemcpyDeviceToHost, m->stream));
+        cudaFreeAsync(out, m->stream);
+        GTM_CU(cudaStreamSynchronize(m->stream));
+        ds->largest_edge_type = (int)std::min<u32>(most, 1u << 30);
+    }
+    if (!ds->chain_msg) {
+        const size_t bits = (size_t)(d.D - 1) * d.C * rw, rows = (size_t)(d.D - 1) * 32 * d.MW * rw, nodes = (size_t)(d.D - 1) * ds->max_nodes * d.MW;
+        const size_t total = ((bits + 63) & ~(size_t)63) + ((rows + 63) & ~(size_t)63) + nodes;
+        u32 *p;
+        GTM_TRY(pool_alloc(&p, total, m->stream));
+        ds->owned.push_back(p);
+        GTM_CU(cudaMemsetAsync(p, 0, total * sizeof(u32), m->stream));        // padding bytes of the rows are never written
+        ds->chain_bits = p;
+        ds->chain_rows_t = p + ((bits + 63) & ~(size_t)63);
+        ds->chain_rows_n = ds->chain_rows_t + ((rows + 63) & ~(size_t)63);
+        ds->chain_msg = true;
+    }
+    return GTM_OK;
+}
+
+struct ChainPlan { bool ok = false, hybrid = false; int rw = 0, grid = 0, threads = 0; size_t smem = 0; ChainArgs a; };
+
+static ChainPlan plan_chain(const gtm_model *m, const gtm_dataset *ds)
+{
+    const DevModel &d = m->dm;
+    ChainPlan plan;
+    memset(&plan.a, 0, sizeof plan.a);
+    ChainArgs &a = plan.a;
+    plan.rw = ds->max_nodes <= 32 ? 1 : ds->max_nodes <= 128 ? 4 : ds->max_nodes <= 512 ? 16 : 32;
+    const int rw = plan.rw, rw4 = std::max(rw, 4), KP = (d.K + 3) & ~3, D1 = d.D - 1;
+    const int words_all = d.L0 + D1 * d.M;
+    a.max_nodes = ds->max_nodes;
+    bool one_p = true;
+    for (int l = 1; l < d.D; ++l) one_p = one_p && d.p_mask[l] == d.p_mask[0];
+    a.narrow = one_p && d.L0 <= 32 && (d.D == 1 || d.M <= 32);
+    if (a.narrow) {
+        // the stream of one Type-I class is made in the shadow of the vote exchange; room for up to four classes
+        a.spec_rounds = d.p_mask[0] >= 1.0f ? 0 : (d.K + 3 + 32 * words_all + 127) / 128;
+        a.pre_words = (std::max(4 * a.spec_rounds, (d.K + 3) / 32 + 1 + std::min(d.K, 4) * words_all) + 4 + 7) & ~3;
+    }
+    // One CTA learns a model of few clauses alone: every grid-wide step (about 2,000 cycles; one per graph, and two per
+    // message layer) costs more than a second or third clause per warp.
+    int cpc = m->opt_fit_block_clauses;
+    if (cpc <= 0) cpc = d.C <= (d.D > 1 ? 64 : 32) ? d.C : (d.C + m->sm_count - 1) / m->sm_count;
+    for (int attempt = 0; attempt < 2; ++attempt) {
+        const int grid = (d.C + cpc - 1) / cpc;
+        const bool solo = grid == 1;
+        if (grid > m->sm_count) return plan;
+        const int want_warps = a.narrow ? std::max(8, cpc) : 32;
+        for (int variant = 0; variant < 4; ++variant) {        // planes resident, then include planes only; with and without staged graphs
+            const bool hybrid = variant >= 2, stage = (variant & 1) == 0;
+            const int warps = std::min(want_warps, (hybrid ? kChainThreads : kChainResidentThreads) / 32);
+            a.stage_nodes = stage ? std::min(ds->max_nodes, 512) : 0;
+            a.stage_words = stage ? (std::min(ds->max_nodes * d.L0, 4096) + 3) & ~3 : 0;
+            a.stage_edges = stage && D1 > 0 ? 512 : 0;
+            a.clause_words = (4 + KP + rw4 + words_all * (hybrid ? 1 : d.SB) + 3) & ~3;
+            const size_t msg = D1 == 0 ? 0 : solo ? (size_t)d.D * ds->max_nodes * d.MW : (size_t)96 * rw;
+            const size_t words = (size_t)7 * KP + 16 + (size_t)kChainStages * ((a.stage_words + 3 * a.stage_nodes + 2 * a.stage_edges + 3) & ~3) +
+                                 ((msg + 3) & ~(size_t)3) + (size_t)32 * std::max(d.L0, D1 > 0 ? d.MW : 0) * rw + (size_t)kTransposedTypes * rw4 +
+                                 (size_t)cpc * (kChainRec + a.pre_words + a.clause_words);
+            const size_t smem = words * sizeof(u32);
+            const void *fn = chain_kernel_for(rw, d.D == 1, hybrid);
+            cudaFuncAttributes fa;
+            if (cudaFuncGetAttributes(&fa, fn) != cudaSuccess) { cudaGetLastError(); return plan; }
+            if (smem + fa.sharedSizeBytes > 227 * 1024 || 32 * warps > fa.maxThreadsPerBlock) continue;
+            plan.ok = true; plan.hybrid = hybrid; plan.grid = grid; plan.threads = 32 * warps; plan.smem = smem;
+            a.clauses_per_cta = cpc; a.solo = solo;
+            return plan;
+        }
+        if (!solo || m->opt_fit_block_clauses > 0) break;
+        cpc = (d.C + m->sm_count - 1) / m->sm_count;           // too much for one CTA: all SMs
+    }
+    return plan;
+}
+
+// Learns with fit_chain_kernel; *done = 0 when it does not cover the model or the set.
+int launch_fit_chain(gtm_model *m, gtm_dataset *ds, int n_types, const int *Y_dev, int64_t first, int64_t count, int epochs, int *done)
+{
+    const DevModel &d = m->dm;
+    *done = 0;
+    if (d.K > 32 || d.SB > 8 || ds->max_nodes > 1024 || n_types > kTransposedTypes) return GTM_OK;
+    ChainPlan plan = plan_chain(m, ds);
+    if (!plan.ok) return GTM_OK;
+    GTM_TRY(chain_prepare(m, ds, plan.rw));
+    if (d.D > 1 && !plan.a.solo && ds->largest_edge_type > kChainMaxType) return GTM_OK;
+    ChainArgs &a = plan.a;
+    a.Y = Y_dev; a.first = first; a.count = count; a.epochs = epochs;
+    // accumulators, arrival counter and the error word start every launch at zero
+    a.votes = m->chain_sync; a.barrier = (unsigned *)(m->chain_sync + 2 * d.K); a.error = (int *)a.barrier + 1;
+    GTM_CU(cudaMemsetAsync(m->chain_sync, 0, ((size_t)2 * d.K + 1) * sizeof(unsigned long long), m->stream));
+    a.clause_node = m->clause_node; a.update = m->update; a.class_sum_tap = m->class_sum_tap;
+    a.phase_cycles = m->phase_cycles; a.timers = m->opt_fit_timers;
+    a.wait_ns = (unsigned long long)m->opt_fit_wait_ms * 1000000ull;
+    a.missing = m->opt_fit_missing_cta;
+    a.node_bits = ds->chain_bits; a.rows_t = ds->chain_rows_t; a.rows_n = ds->chain_rows_n;
+    a.bit_off = m->hv_off; a.bit_clause = m->hv_clause; a.tmax = std::max(0, ds->largest_edge_type);
+    DevGraphs g = ds->dg;
+    g.n_types = n_types;
+    DevModel dm = d;
+    const void *fn = chain_kernel_for(plan.rw, d.D == 1, plan.hybrid);
+    GTM_CU(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)plan.smem));
+    void *args[] = {&dm, &g, &a};
+    GTM_CU(cudaLaunchCooperativeKernel(fn, dim3(plan.grid), dim3(plan.threads), args, plan.smem, m->stream));
+    *done = 1;
+    int err = 0;
+    GTM_CU(cudaMemcpyAsync(&err, a.error, sizeof(int), cudaMemcpyDeviceToHost, m->stream));
+    GTM_CU(cudaStreamSynchronize(m->stream));
+    if (err) return fail(GTM_ERR_TIMEOUT, "a bounded wait of the learning kernel (grid barrier or vote exchange) gave up");
+    return GTM_OK;
+}

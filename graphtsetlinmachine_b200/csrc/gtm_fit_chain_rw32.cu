@@ -1,0 +1,9 @@
+// fit_chain_kernel for transposed rows of 32 node words.
+#include "gtm_fit_chain.cuh"
+
+const void *fit_chain_kernel_rw32(bool one_layer, bool hybrid)
+{
+    using namespace gtm;
+    if (one_layer) return hybrid ? (const void *)fit_chain_kernel<32, true, true> : (const void *)fit_chain_kernel<32, true, false>;
+    return hybrid ? (const void *)fit_chain_kernel<32, false, true> : (const void *)fit_chain_kernel<32, false, false>;
+}

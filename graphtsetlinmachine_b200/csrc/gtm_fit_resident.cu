@@ -634,6 +634,11 @@ int launch_fit(gtm_model *m, gtm_dataset *ds, int n_types, const int *Y_dev, int
     const bool sharded = cm.world > 1 && !eval_only;
     if (sharded && !cm.connected) return fail(GTM_ERR_STATE, "clause sharding was prepared but the ranks are not connected (gtm_shard_connect)");
     if (sharded && cm.broken) return fail(GTM_ERR_STATE, "an earlier sharded fit timed out; prepare and connect the ranks again");
+    if (!sharded && !eval_only && m->opt_fit_kernel == 0) {
+        int done;
+        GTM_TRY(launch_fit_chain(m, ds, n_types, Y_dev, first, count, epochs, &done));
+        if (done) return GTM_OK;
+    }
     GTM_TRY(ensure_fit_scratch(ds));
     DevGraphs g = ds->dg;
     g.n_types = n_types;

@@ -30,6 +30,11 @@ struct gtm_model {
     int opt_fit_timers = 0;                   // 1: the learning kernels time their phases (gtm_debug_fit_phase_cycles)
     int opt_score_kernel = 0;                 // 0 auto, 1 general kernel, 2 node-stream kernel, 3 tile kernel
     unsigned *barrier = nullptr;
+    // learning on one GPU (gtm_fit_chain.cu): vote accumulators, arrival counter and error word; clauses of every message bit
+    unsigned long long *chain_sync = nullptr;
+    std::vector<u32> hv_host;                 // hypervectors as set
+    bool hv_lists_valid = false;
+    int *hv_off = nullptr, *hv_clause = nullptr;
     unsigned long long *phase_cycles = nullptr;
     // node-stream scoring: derived include lists (rebuilt when the automata changed)
     StreamModel sm;
@@ -67,6 +72,10 @@ struct gtm_dataset {
     u32 *P_pair[2] = {nullptr, nullptr};
     u32 *Q_pair[2] = {nullptr, nullptr};   // [D-1][max_nodes][MW] destination message rows by graph parity (learning, merged marks)
     unsigned *rank_barrier = nullptr;      // arrival counter of the barriers among one rank's CTAs
+    // learning on one GPU: message buffers (gtm_fit_chain.cu)
+    bool chain_msg = false;
+    u32 *chain_bits = nullptr, *chain_rows_t = nullptr, *chain_rows_n = nullptr;
+    int largest_edge_type = -1;            // -1: not known yet
     // scoring scratch of the general path: one slice per CTA
     EvalScratch score_sc;
     size_t cno_stride = 0, P_stride = 0, ninc_stride = 0;
@@ -91,6 +100,7 @@ struct gtm_dataset {
 int fit_grid_for_global_state(const DevModel &d, int sm_count, int block, int *grid_out);
 int launch_fit(gtm_model *m, gtm_dataset *ds, int n_types, const int *Y_dev, int64_t first, int64_t count, int epochs,
                int eval_only);
+int launch_fit_chain(gtm_model *m, gtm_dataset *ds, int n_types, const int *Y_dev, int64_t first, int64_t count, int epochs, int *done);
 int ensure_fit_scratch(gtm_dataset *ds);
 void fit_comm_release(gtm_dataset *ds);
 size_t exchange_bytes(int world, int K);

@@ -1,0 +1,100 @@
+"""GPU suite, learning kernel for one GPU (gtm_fit_chain): automata, weights, draws and scores equal the CPU checker's bit for
+bit at the edges of its dispatch - node-word sizes of the transposed rows, row-wise graphs, classes per decision pass, layers
+of more than 32 words, layers of different probabilities, one CTA or many, planes in global memory, and what it leaves to
+the other learning kernels (large edge types, more classes, wider automata)."""
+
+import numpy as np
+import pytest
+
+from cases import state_of
+from oracle.oracle import OracleTM
+from util import EngineTM, encode_labels, random_graphs
+
+pytestmark = pytest.mark.gpu
+
+
+def agree(kw, graphs, classes, seed, epochs=2, options=None):
+    rng = np.random.default_rng(seed)
+    encY = encode_labels(rng.integers(0, classes, size=graphs.number_of_graphs), classes, kw["threshold"])
+    cpu, gpu = OracleTM(**kw), EngineTM(**kw, options=options)
+    for tm in (cpu, gpu):
+        tm.set_graphs(graphs)
+        tm.prepare()
+    for _ in range(epochs):
+        for tm in (cpu, gpu):
+            tm.fit(encY)
+        a, b = state_of(cpu, kw["depth"]), state_of(gpu, kw["depth"])
+        assert np.array_equal(a["ta_state"], b["ta_state"])
+        for x, y in zip(a["message_ta_state"], b["message_ta_state"]):
+            assert np.array_equal(x, y)
+        assert np.array_equal(a["clause_weights"], b["clause_weights"])
+        assert np.array_equal(a["draws"], b["draws"])
+    assert np.array_equal(cpu.score(), gpu.score())
+    gpu.close()
+
+
+def model(rng, *, clauses, classes, hv, depth, ms, s=2.5, **more):
+    hvs = np.stack([rng.choice(ms, size=2, replace=False) for _ in range(clauses)]).astype(np.uint32)
+    return dict(clauses=clauses, classes=classes, literals=2 * hv, threshold=20, s=s, depth=depth, message_size=ms, message_bits=2,
+                hypervectors=hvs, **more)
+
+
+@pytest.mark.parametrize("nodes,depth,clauses,classes,hv,ms,n", [
+    (1, 1, 5, 2, 3, 8, 40),                 # one CTA, row-wise, a few literals
+    (3, 2, 40, 15, 16, 33, 25),             # one CTA with messages; a full decision pass
+    (4, 3, 33, 16, 40, 32, 25),             # just past row-wise; the second decision pass has one class
+    (32, 2, 300, 31, 33, 100, 8), (33, 2, 300, 32, 32, 64, 8),                                  # one node word / more
+    (128, 3, 90, 3, 64, 37, 6), (129, 2, 90, 3, 65, 40, 6),
+    (512, 2, 150, 2, 20, 70, 3), (513, 2, 150, 2, 20, 70, 3), (1024, 2, 150, 2, 20, 64, 2), (1025, 2, 70, 2, 20, 64, 2),
+    (20, 3, 200, 4, 600, 700, 6),           # layers of more than 32 words: updates as work items
+])
+def test_sizes(engine_lib, nodes, depth, clauses, classes, hv, ms, n):
+    rng = np.random.default_rng(nodes + clauses)
+    np.random.seed(nodes)
+    graphs = random_graphs(n, rng, hv_size=hv, max_nodes=nodes, node_types=2, edge_types=3, max_degree=2)
+    graphs2 = random_graphs(2, rng, init_with=graphs, fixed_nodes=nodes, node_types=2, edge_types=3, max_degree=2)
+    for g in (graphs, graphs2):             # mixed sizes, then the largest alone
+        kw = model(rng, clauses=clauses, classes=classes, hv=hv, depth=depth, ms=ms, max_nodes=nodes, seed=nodes)
+        agree(kw, g, classes, 3)
+
+
+@pytest.mark.parametrize("more", [dict(s=(2.0, 3.0, 4.0)), dict(s=1.0), dict(boost=0), dict(max_included=3), dict(state_bits=1), dict(state_bits=9),
+                                  dict(q=0.3)])
+@pytest.mark.parametrize("hv,ms", [(20, 50), (560, 50)])
+def test_options(engine_lib, more, hv, ms):
+    rng = np.random.default_rng(7)
+    np.random.seed(7)
+    graphs = random_graphs(15, rng, hv_size=hv, max_nodes=9, node_types=1, edge_types=2)
+    kw = model(rng, clauses=70, classes=5, hv=hv, depth=3, ms=ms, max_nodes=9, seed=5, **more)
+    agree(kw, graphs, 5, 4)
+
+
+@pytest.mark.parametrize("largest", [24, 25, 300])
+def test_edge_types(engine_lib, largest):
+    """The window of pulled messages covers edge types up to 24; beyond, another kernel learns."""
+    rng = np.random.default_rng(largest)
+    np.random.seed(9)
+    graphs = random_graphs(12, rng, hv_size=24, max_nodes=20, edge_types=2, max_degree=3)
+    graphs.edge[:, 1] = rng.integers(0, largest + 1, size=len(graphs.edge))
+    graphs.edge[0, 1] = largest
+    kw = model(rng, clauses=150, classes=3, hv=24, depth=3, ms=45, max_nodes=20, seed=6)
+    agree(kw, graphs, 3, 5)
+
+
+@pytest.mark.parametrize("clauses,depth,hv,ms,nodes", [(7000, 2, 512, 512, 6), (16000, 1, 700, 8, 40)])
+def test_planes_in_global_memory(engine_lib, clauses, depth, hv, ms, nodes):
+    """Models whose automata exceed shared memory keep only the include planes there."""
+    rng = np.random.default_rng(clauses)
+    np.random.seed(2)
+    graphs = random_graphs(4, rng, hv_size=hv, max_nodes=nodes, edge_types=2)
+    kw = model(rng, clauses=clauses, classes=4, hv=hv, depth=depth, ms=ms, max_nodes=nodes, seed=8)
+    agree(kw, graphs, 4, 6)
+
+
+@pytest.mark.parametrize("per_cta", [1, 7, 60])
+def test_clause_ranges(engine_lib, per_cta):
+    rng = np.random.default_rng(1)
+    np.random.seed(3)
+    graphs = random_graphs(20, rng, hv_size=30, max_nodes=12, edge_types=2)
+    kw = model(rng, clauses=60, classes=3, hv=30, depth=2, ms=64, max_nodes=12, seed=4)
+    agree(kw, graphs, 3, 8, options={"fit_block_clauses": per_cta})
