@@ -783,7 +783,7 @@ extern "C" int gtm_score_device(gtm_model *m, gtm_dataset *ds, int n_types, int6
     }
     if (scores_by_tile(m, ds, n_types)) {
         GTM_TRY(refresh_tile_lists(m));
-        return tile_score(&m->tm, ds->td, m->dm, ds->dg, n_types, first, count, sums_dev, m->score_error, 0, m->stream);
+        return tile_score(&m->tm, ds->td, m->dm, ds->dg, n_types, first, count, sums_dev, nullptr, m->score_error, 0, m->stream);
     }
     return launch_score_general(m, ds, n_types, first, count, sums_dev, nullptr);
 }
@@ -847,7 +847,7 @@ static int score_in_chunks(gtm_model *m, gtm_dataset *ds, const gtm_graphs_view 
                 GTM_TRY(fill_range(f, cs));
             }
             if (by_stream) GTM_TRY(stream_score(&m->sm, ds->sd, d, ds->dg, n_types, g0, (int64_t)cnt, dev + at, turn, cs));
-            else GTM_TRY(tile_score(&m->tm, ds->td, d, ds->dg, n_types, g0, (int64_t)cnt, dev + at, m->score_error, turn, cs));
+            else GTM_TRY(tile_score(&m->tm, ds->td, d, ds->dg, n_types, g0, (int64_t)cnt, dev + at, nullptr, m->score_error, turn, cs));
             GTM_CU(cudaEventRecord(lane->event[2], cs));
             GTM_CU(cudaStreamWaitEvent(lane->back, lane->event[2], 0));
             GTM_TRY(stage_down(lane, out + at, dev + at, cnt * d.K * sizeof(int), pinned_out, lane->back));
@@ -946,7 +946,28 @@ extern "C" int gtm_dataset_create_scored(gtm_model *m, const gtm_graphs_view *v,
     return GTM_OK;
 }
 
-// clause outputs per graph and / or per node through the general scoring kernel; results land in host arrays
+// Tiles of a set that was made without them: sets of models without message layers that the node-stream kernel scores.
+static int ensure_tiles(gtm_model *m, gtm_dataset *ds)
+{
+    if (ds->td.supported || ds->tiles_tried || !m->tm.applicable) return GTM_OK;
+    std::vector<u32> nodes;
+    gtm_graphs_view v;
+    memset(&v, 0, sizeof v);
+    v.number_of_graphs = ds->n_graphs;
+    v.max_number_of_graph_nodes = ds->max_nodes;
+    if (ds->n_min != ds->n_max || ds->n_max == 0) {                       // ragged: the packing goes by the graphs' sizes
+        nodes.resize((size_t)ds->n_graphs);
+        GTM_CU(cudaMemcpyAsync(nodes.data(), ds->dg.n_nodes, nodes.size() * sizeof(u32), cudaMemcpyDeviceToHost, m->stream));
+        GTM_CU(cudaStreamSynchronize(m->stream));
+        v.number_of_graph_nodes = nodes.data();
+    }
+    GTM_TRY(tile_data_create(&ds->td, m->tm, m->dm, &v, ds->n_min, ds->n_max, m->sm_count, m->stream));
+    GTM_CU(cudaStreamSynchronize(m->stream));                             // the packing's host arrays go out of scope
+    ds->tiles_tried = true;
+    return GTM_OK;
+}
+
+// clause outputs per graph and / or per node; results land in host arrays
 static int transform_common(gtm_model *m, gtm_dataset *ds, int n_types, int64_t first, int64_t count, int32_t *clause_out,
                             int32_t *node_out, int node_stride, int32_t *sums_out)
 {
@@ -960,7 +981,16 @@ static int transform_common(gtm_model *m, gtm_dataset *ds, int n_types, int64_t 
     int st = pool_alloc(&sums_dev, n_sums, m->stream);
     if (st == GTM_OK && clause_out) st = pool_alloc(&co_dev, n_co, m->stream);
     if (st == GTM_OK && node_out) st = pool_alloc(&no_dev, n_no, m->stream);
-    if (st == GTM_OK) st = launch_score_general(m, ds, n_types, first, count, sums_dev, co_dev, no_dev, node_stride);
+    if (st == GTM_OK) {
+        // clause outputs of whole graphs come out of the tile kernel too; outputs per node only out of the general one
+        if (!node_out && clause_out && m->opt_score_kernel != 1) st = ensure_tiles(m, ds);
+        if (st == GTM_OK && !node_out && clause_out && m->opt_score_kernel != 1 && tile_supported(ds->td, n_types)) {
+            st = refresh_tile_lists(m);
+            if (st == GTM_OK) st = tile_score(&m->tm, ds->td, m->dm, ds->dg, n_types, first, count, sums_dev, co_dev, m->score_error, 0, m->stream);
+        } else if (st == GTM_OK) {
+            st = launch_score_general(m, ds, n_types, first, count, sums_dev, co_dev, no_dev, node_stride);
+        }
+    }
     auto down = [&](int32_t *host, const int *dev, size_t n) {
         if (st == GTM_OK && host) st = stage_down(guard.lane, host, dev, n * sizeof(int), host_is_pinned(host), m->stream);
     };
@@ -975,7 +1005,7 @@ static int transform_common(gtm_model *m, gtm_dataset *ds, int n_types, int64_t 
     const cudaError_t e = cudaStreamSynchronize(m->stream);
     if (st != GTM_OK) return st;
     GTM_CU(e);
-    return GTM_OK;
+    return score_flag_status(m);
 }
 
 extern "C" int gtm_transform(gtm_model *m, gtm_dataset *ds, int n_types, int64_t first, int64_t count,

@@ -91,6 +91,7 @@ struct gtm_dataset {
     StreamData sd;
     // tile scoring
     TileData td;
+    bool tiles_tried = false;      // tiles were made, or found not to fit, for a set that did not come with them
     // clause-sharded learning
     FitComm comm;
 };

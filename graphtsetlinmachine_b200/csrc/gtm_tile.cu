@@ -1,4 +1,4 @@
-// Tile scoring: batched inference for any depth on graph sets whose graphs have at most 128 nodes.
+// Tile scoring: batched inference for any depth on graph sets whose graphs have at most 1,024 nodes.
 //
 // The reference evaluates one graph at a time with five kernels per message layer (tm.py:563-662 driving
 // kernels.py:407-615).  Here a persistent CTA takes a TILE of consecutive whole graphs (32*TNC node slots, graphs
@@ -21,6 +21,16 @@
 //   5. after the last layer, per graph and warp, the weights of the clauses that fired are summed over the warp with
 //      redux.sync and added to the graph's class sums in shared memory (kernels.py:279-317, unclamped).
 //
+// Graphs of 129 to 1,024 nodes are a tile each ("span"): 32 clauses x 256 nodes is the unit of work as for small graphs, the
+// literal rows lie in planes of eight node words so that rows stay 32 bytes apart (rows of 128 bytes put the same quad of all
+// rows into the same banks), and since no single unit sees a whole graph, the fired clauses are collected as bits first and
+// vote after the layer.  What bounds it is shared-memory bandwidth: 128 bytes of literal row per included literal and graph.
+// 400 sequences of 1,000 nodes, 2,000 clauses, depth 3, on one B200: 1.2 ms; 9.2 ms in the general kernel, a warp per clause
+// walking its include bits with 16 warps per SM.  A CTA that has its SM to itself runs 32 warps.
+//
+// More than 16 classes vote in two passes, which keeps the weights of a pass in registers.  Clause outputs: ones for the
+// clauses that fire, into an array cleared before (500 multigraphs x 5,000 clauses: 13.0 ms in the general kernel, 0.56 here).
+//
 // Shared memory: one buffer of literal rows (transposed literals, then transposed messages) and one that serves as
 // staging area, mark buffer and destination rows in turn.  Global scratch: the survivor lists (L2 traffic
 // proportional to the clauses that are still true).
@@ -35,8 +45,9 @@
 
 namespace gtm {
 
-constexpr int kTileThreads = 512;
-constexpr int kTileMaxK = 16;
+constexpr int kTileThreads = 512, kTileThreadsAlone = 1024;   // threads of a CTA that shares its SM with another / has it to itself
+constexpr int kTileMaxK = 32;
+constexpr int kTileSpanNodes = 1024;  // largest graph of sets whose graphs span quads
 constexpr int kTileMaxTypes = 8;
 constexpr int kTileMaxGraphs = 512;   // graphs per tile: their vote accumulators and node masks live in shared memory
 constexpr int kQuadNodes = 128;
@@ -56,6 +67,8 @@ __device__ __forceinline__ const u32 *include_plane(const DevModel &m, int layer
 // (kernels.py:544-545).  After the literal rows come four rows of ones (list padding, one per residue class).
 __device__ __forceinline__ int tile_row(int p, int W) { return (p & 31) * W + (p >> 5); }
 constexpr int kTilePadRows = 4;
+// Rows of a plane of literal rows, see plane_at.
+__host__ __device__ __forceinline__ int tile_plane_rows(int rows, int TNC, int pw) { return pw < TNC ? rows | 1 : rows; }
 __host__ __device__ __forceinline__ int tile_literal_rows(int layer, int L0, int MW) { return layer == 0 ? 32 * L0 : 64 * MW; }
 
 // Visits the rows of the included literals of a clause layer.
@@ -135,7 +148,10 @@ struct TileArgs {
     int64_t n_graphs;
     int *class_sums;                    // [count][K]
     unsigned *tile_counter;             // tiles handed out beyond the first of every CTA; left at zero
+    int *clause_out;                    // [count][C] clause outputs, zero before the launch, or NULL
     int TNC, PS, words_a, words_b, stage_rows, gmax;
+    int pw;                             // node words of a literal row: TNC, or 8 and TNC/8 planes of rows one after the other
+    int span;                           // a tile is ONE graph, which may span quads
     int rot_step;                       // message transposition: block column j is read rotated by (rot_step * j) & 31
     const TileLayer *layers;            // [D]
     const int *Wt;
@@ -245,29 +261,37 @@ __device__ __forceinline__ uint4 quad_mask(int lo, int n)
 }
 
 template <int KP>
-__global__ void __launch_bounds__(kTileThreads, 2) tile_score_kernel(DevModel m, DevGraphs g, TileArgs a)
+__global__ void __launch_bounds__(kTileThreadsAlone, 1) tile_score_kernel(DevModel m, DevGraphs g, TileArgs a)
 {
     extern __shared__ __align__(16) u32 s_dyn[];
     const int TNC = a.TNC, TN = TNC * 32, Q = TNC >> 2, PS = a.PS;
-    const int rowshift = 31 - __clz(TNC * 4);
+    const int pw = a.pw, pshift = 31 - __clz(pw), rowshift = pshift + 2;
+    const int KS = KP < 16 ? KP : (m.K + KP - 1) / KP * KP;         // class sums of a graph: classes are taken KP at a time
     u32 *bufA = s_dyn;                                              // literal rows / message rows, swapping roles
     u32 *bufB = bufA + a.words_a;                                   // staging of X / message rows, swapping roles
     u32 *TMV = bufB + a.words_b;                                    // [kTileMaxTypes][TNC] valid nodes of each type
     u32 *tnode = TMV + kTileMaxTypes * TNC;                         // [TN] node of each slot, or ~0
     u32 *pinfo = tnode + TN;                                        // [TN] first slot of the slot's graph | nodes << 16
     uint4 *gmask = reinterpret_cast<uint4 *>(pinfo + TN);           // [gmax] node slots of a graph inside its quad
-    int *sums = reinterpret_cast<int *>(gmask + a.gmax);            // [gmax][KP]
-    int *gq_first = sums + a.gmax * KP;                             // [Q+1] first graph of every quad
+    int *sums = reinterpret_cast<int *>(gmask + a.gmax);            // [gmax][KS]
+    int *gq_first = sums + a.gmax * KS;                             // [Q+1] first graph of every quad
     int *cnt = gq_first + 12;                                       // [2][8] survivor counts per list and quad
     int *misc = cnt + 16;                                           // tile number, node range of a staging round
     unsigned long long *mbar_mem = reinterpret_cast<unsigned long long *>(misc + 4);
     unsigned char *gquad = reinterpret_cast<unsigned char *>(mbar_mem + 1);   // [gmax]
     unsigned char *pflag = gquad + ((a.gmax + 3) & ~3);             // [TN] slot's message row has bits
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nwarps = kTileThreads / 32;
+    u32 *fired = reinterpret_cast<u32 *>(pflag + TN);              // span: [cblocks] clauses true on the graph, by position in the last layer's order
+    const int tid = threadIdx.x, lane = tid & 31, nthreads = blockDim.x, warp = tid >> 5, nwarps = nthreads >> 5;
     const unsigned bar = smem_u32(mbar_mem);
+    const int UP = (Q + 1) >> 1;                                                       // quad pairs of a full tile
     const int cblocks = (m.C + 31) >> 5;                                                // blocks of 32 clauses
-    uint4 *surv_r = a.surv_r + (size_t)blockIdx.x * 4 * ((Q + 1) >> 1) * m.C;         // [2][quad pairs][C][2 quads]
+    uint4 *surv_r = a.surv_r + (size_t)blockIdx.x * 4 * UP * m.C;         // [2][quad pairs][C][2 quads]
     const size_t x_words = (size_t)g.total_nodes * m.L0;
+    // Word j of row 0 of a buffer of literal rows; the row's words are pw apart from row to row, a plane of rows is `rows`
+    // long.  One row more than a multiple of four per plane spreads the planes over the banks in the transpositions.
+    auto plane_at = [&](int j, int rows) { return ((j >> pshift) * rows << pshift) + (j & (pw - 1)); };
+    const int rows0 = tile_plane_rows(32 * m.L0 + kTilePadRows, TNC, pw), rowsm = tile_plane_rows(64 * m.MW + kTilePadRows, TNC, pw),
+              mark_rows = tile_plane_rows(32 * m.MW, TNC, pw), mark_words = mark_rows * TNC;
 
     if (tid == 0) mbar_init(bar, 1);
     __syncthreads();
@@ -280,13 +304,18 @@ __global__ void __launch_bounds__(kTileThreads, 2) tile_score_kernel(DevModel m,
         const int ng = g1 - g0;
 
         // ---- slot tables: which node sits where, which slots belong to which graph ----
-        for (int i = tid; i < TN; i += kTileThreads) { tnode[i] = ~0u; pinfo[i] = 0u; }
-        for (int i = tid; i < ng * KP; i += kTileThreads) sums[i] = 0;
+        for (int i = tid; i < TN; i += nthreads) { tnode[i] = ~0u; pinfo[i] = 0u; }
+        for (int i = tid; i < ng * KS; i += nthreads) sums[i] = 0;
+        if (a.span) for (int i = tid; i < cblocks; i += nthreads) fired[i] = 0;
         if (tid < 16) cnt[tid] = 0;
         __syncthreads();
-        {
+        if (a.span) {
+            const int n = (int)g.n_nodes[g0];
+            const u32 nb = g.node_index[g0];
+            for (int i = tid; i < n; i += nthreads) { tnode[i] = nb + i; pinfo[i] = (u32)n << 16; }
+        } else {
             const int gpq = a.uniform_n > 0 ? kQuadNodes / a.uniform_n : 1;
-            for (int gl = tid; gl < ng; gl += kTileThreads) {
+            for (int gl = tid; gl < ng; gl += nthreads) {
                 const int n = (int)g.n_nodes[g0 + gl];
                 const u32 nb = g.node_index[g0 + gl];
                 const int pos = a.uniform_n > 0 ? (gl / gpq) * kQuadNodes + (gl % gpq) * n : (int)a.gpos[g0 + gl];
@@ -296,7 +325,7 @@ __global__ void __launch_bounds__(kTileThreads, 2) tile_score_kernel(DevModel m,
             }
         }
         __syncthreads();
-        for (int gl = tid; gl <= ng; gl += kTileThreads) {      // gq_first[q] = first graph whose quad is >= q
+        if (!a.span) for (int gl = tid; gl <= ng; gl += nthreads) {      // gq_first[q] = first graph whose quad is >= q
             const int qhi = gl < ng ? (int)gquad[gl] : Q, qlo = gl > 0 ? (int)gquad[gl - 1] + 1 : 0;
             for (int qq = qlo; qq <= qhi; ++qq) gq_first[qq] = gl;
         }
@@ -307,7 +336,7 @@ __global__ void __launch_bounds__(kTileThreads, 2) tile_score_kernel(DevModel m,
             const int jend = min(TNC, jr + groups_per_round);
             if (tid == 0) { misc[1] = 0x7fffffff; misc[2] = -1; }
             __syncthreads();
-            for (int p = 32 * jr + tid; p < 32 * jend; p += kTileThreads) {
+            for (int p = 32 * jr + tid; p < 32 * jend; p += nthreads) {
                 const u32 nd = tnode[p];
                 if (nd != ~0u) { atomicMin(&misc[1], (int)nd); atomicMax(&misc[2], (int)nd); }
             }
@@ -328,7 +357,7 @@ __global__ void __launch_bounds__(kTileThreads, 2) tile_score_kernel(DevModel m,
                 parity ^= 1u;
             }
             const int nblk = (jend - jr) * m.L0;
-            for (int blk = tid; blk < nblk; blk += kTileThreads) {
+            for (int blk = tid; blk < nblk; blk += nthreads) {
                 const int jj = blk / m.L0, w = blk - jj * m.L0, j = jr + jj, rot = j & 31;
                 u32 rows[32];
 #pragma unroll
@@ -338,11 +367,11 @@ __global__ void __launch_bounds__(kTileThreads, 2) tile_score_kernel(DevModel m,
                 }
                 transpose32(rows);
 #pragma unroll
-                for (int b = 0; b < 32; ++b) bufA[(size_t)(b * m.L0 + w) * TNC + j] = __funnelshift_l(rows[b], rows[b], rot);
+                for (int b = 0; b < 32; ++b) bufA[plane_at(j, rows0) + ((b * m.L0 + w) << pshift)] = __funnelshift_l(rows[b], rows[b], rot);
             }
             __syncthreads();                          // the staging buffer is rewritten by the next round
         }
-        for (int t = tid; t < kTilePadRows * TNC; t += kTileThreads) bufA[(size_t)(32 * m.L0) * TNC + t] = kFull;   // padding rows
+        for (int t = tid; t < kTilePadRows * TNC; t += nthreads) bufA[plane_at(t % TNC, rows0) + ((32 * m.L0 + t / TNC) << pshift)] = kFull;   // padding rows
         for (int j = warp; j < TNC; j += nwarps) {
             const u32 nd = tnode[32 * j + lane];
             const u32 ty = nd != ~0u ? g.node_type[nd] : ~0u;
@@ -352,14 +381,15 @@ __global__ void __launch_bounds__(kTileThreads, 2) tile_score_kernel(DevModel m,
             }
         }
         if (m.D > 1)
-            for (int i = tid; i < 32 * m.MW * TNC; i += kTileThreads) bufB[i] = 0u;
+            for (int i = tid; i < mark_words; i += nthreads) bufB[i] = 0u;
         __syncthreads();
 
         // ---- layers ----
         // bufA always holds the literal rows of the current layer (the transposed literals, then the transposed
         // messages); bufB takes, in turn, the message bits that the layer's true clauses mark on their nodes (bit-major,
         // the layout of the literal rows) and the node-major destination rows of the edge pass.
-        const int U = (Q + 1) >> 1;                   // quad pairs: a thread evaluates a clause on two quads at a time
+        const int QT = a.span ? ((int)g.n_nodes[g0] + kQuadNodes - 1) / kQuadNodes : Q;     // quads that hold nodes
+        const int U = (QT + 1) >> 1;                  // quad pairs: a thread evaluates a clause on two quads at a time
         const unsigned t32 = smem_u32(bufA);
         for (int d = 0; d < m.D; ++d) {
             const bool last = d == m.D - 1;
@@ -375,7 +405,7 @@ __global__ void __launch_bounds__(kTileThreads, 2) tile_score_kernel(DevModel m,
                 if (r.w & ~old.w) atomicOr(dst + 3, r.w);
             };
             // votes of one quad: per graph, the weights of the lanes that fired, summed over the warp
-            auto vote = [&](int q, const uint4 r, const int (&w)[KP]) {
+            auto vote = [&](int q, const uint4 r, const int (&w)[KP], int c, int kb) {
                 const u32 ax = __reduce_or_sync(kFull, r.x), ay = __reduce_or_sync(kFull, r.y),
                           az = __reduce_or_sync(kFull, r.z), aw = __reduce_or_sync(kFull, r.w);
                 if ((ax | ay | az | aw) == 0) return;
@@ -383,23 +413,42 @@ __global__ void __launch_bounds__(kTileThreads, 2) tile_score_kernel(DevModel m,
                     const uint4 gm = gmask[gl];
                     if (((ax & gm.x) | (ay & gm.y) | (az & gm.z) | (aw & gm.w)) == 0) continue;    // nobody fired on this graph
                     const bool f = ((r.x & gm.x) | (r.y & gm.y) | (r.z & gm.z) | (r.w & gm.w)) != 0;
+                    if (a.clause_out && kb == 0 && f) {
+                        const int64_t gi = (int64_t)g0 + gl;
+                        if (gi >= a.first && gi < a.first + a.count) a.clause_out[(size_t)(gi - a.first) * m.C + c] = 1;
+                    }
                     int mine = 0;
 #pragma unroll
                     for (int k = 0; k < KP; ++k) {
                         const int sk = __reduce_add_sync(kFull, f ? w[k] : 0);
                         if (lane == k) mine = sk;
                     }
-                    if (lane < m.K) atomicAdd(&sums[gl * KP + lane], mine);
+                    if (lane < min(KP, m.K - kb)) atomicAdd(&sums[gl * KS + kb + lane], mine);
+                }
+            };
+            // weights of classes kb .. kb+KP-1 of clause c; zero for a lane whose clause did not fire
+            auto load_weights = [&](int (&w)[KP], bool mine, int c, int kb) {
+#pragma unroll
+                for (int k = 0; k < KP; ++k) w[k] = 0;
+                if (!mine) return;
+                const int4 *wr4 = reinterpret_cast<const int4 *>(a.Wt + (size_t)c * a.KROW + kb);
+#pragma unroll
+                for (int k4 = 0; k4 < (KP + 3) / 4; ++k4) {
+                    const int4 t = __ldg(wr4 + k4);
+                    w[4 * k4] = t.x;
+                    if (4 * k4 + 1 < KP) w[4 * k4 + 1] = t.y;
+                    if (4 * k4 + 2 < KP) w[4 * k4 + 2] = t.z;
+                    if (4 * k4 + 3 < KP) w[4 * k4 + 3] = t.w;
                 }
             };
             // one warp pass over the 32 clauses at positions 32*block .. 32*block+31 of the layer's order (c: the lane's
             // clause, -1: none) and the quads of pair u; ra / rb are the node bits as they were before the layer
             auto pass = [&](int block, int c, uint4 ra, uint4 rb, int u) {
                 const int qa = 2 * u;
-                const bool two = qa + 1 < Q;
+                const bool two = qa + 1 < QT;
                 {
                     const bool flip = two && (lane & 4);                  // lanes 4..7 of every eight take the second quad first
-                    const unsigned ta = t32 + qa * 16;
+                    const unsigned ta = t32 + 4 * plane_at(8 * u, d == 0 ? rows0 : rowsm);
                     uint4 r0 = flip ? rb : ra, r1 = flip ? ra : rb;
                     const unsigned pad = (unsigned)tile_literal_rows(d, m.L0, m.MW);     // padding rows of classes lane, lane+1, ..
                     const uint2 pad4 = make_uint2((pad + (lane & 3)) | ((pad + ((lane + 1) & 3)) << 16),
@@ -414,7 +463,7 @@ __global__ void __launch_bounds__(kTileThreads, 2) tile_score_kernel(DevModel m,
                 if (!last) {
                     // every clause's node bits (zeros included) for the next layer, which takes the clauses in its own order
                     if (c >= 0) {
-                        const size_t at = (size_t)(wr * U + u) * m.C + c;
+                        const size_t at = (size_t)(wr * UP + u) * m.C + c;
                         surv_r[2 * at] = ra;
                         surv_r[2 * at + 1] = rb;
                     }
@@ -423,28 +472,22 @@ __global__ void __launch_bounds__(kTileThreads, 2) tile_score_kernel(DevModel m,
                         // the clause's hypervector bits on every node it is true on (the SOURCE side of kernels.py:571-588):
                         // in the bit-major buffer that is one 128-bit OR per hypervector bit and quad
                         for (int b = 0; b < m.MB; ++b) {
-                            u32 *row = bufB + (size_t)tile_row((int)a.hvm[(size_t)c * m.MB + b], m.MW) * TNC + 4 * qa;
+                            u32 *row = bufB + plane_at(8 * u, mark_rows) + (tile_row((int)a.hvm[(size_t)c * m.MB + b], m.MW) << pshift);
                             mark(row, ra);
                             if (two) mark(row + 4, rb);
                         }
                     }
                 } else if (amask != 0) {
-                    int w[KP];
-#pragma unroll
-                    for (int k = 0; k < KP; ++k) w[k] = 0;
-                    if (alive) {
-                        const int4 *wr4 = reinterpret_cast<const int4 *>(a.Wt + (size_t)c * a.KROW);
-#pragma unroll
-                        for (int k4 = 0; k4 < (KP + 3) / 4; ++k4) {
-                            const int4 t = __ldg(wr4 + k4);
-                            w[4 * k4] = t.x;
-                            if (4 * k4 + 1 < KP) w[4 * k4 + 1] = t.y;
-                            if (4 * k4 + 2 < KP) w[4 * k4 + 2] = t.z;
-                            if (4 * k4 + 3 < KP) w[4 * k4 + 3] = t.w;
-                        }
+                    if (a.span) {
+                        if (lane == 0) atomicOr(&fired[block], amask);
+                        return;
                     }
-                    vote(qa, ra, w);
-                    if (two) vote(qa + 1, rb, w);
+                    for (int kb = 0; kb < m.K; kb += KP) {
+                        int w[KP];
+                        load_weights(w, alive, c, kb);
+                        vote(qa, ra, w, c, kb);
+                        if (two) vote(qa + 1, rb, w, c, kb);
+                    }
                 }
             };
 
@@ -456,9 +499,9 @@ __global__ void __launch_bounds__(kTileThreads, 2) tile_score_kernel(DevModel m,
                     if (d == 0) {
                         const u32 *tm_row = TMV + (c % g.n_types) * TNC + 8 * u;
                         ra = *reinterpret_cast<const uint4 *>(tm_row);
-                        if (2 * u + 1 < Q) rb = *reinterpret_cast<const uint4 *>(tm_row + 4);
+                        if (2 * u + 1 < QT) rb = *reinterpret_cast<const uint4 *>(tm_row + 4);
                     } else {
-                        const size_t at = (size_t)(rd * U + u) * m.C + c;
+                        const size_t at = (size_t)(rd * UP + u) * m.C + c;
                         ra = surv_r[2 * at];
                         rb = surv_r[2 * at + 1];
                     }
@@ -466,7 +509,7 @@ __global__ void __launch_bounds__(kTileThreads, 2) tile_score_kernel(DevModel m,
                 if (d > 0 && !__any_sync(kFull, (ra.x | ra.y | ra.z | ra.w | rb.x | rb.y | rb.z | rb.w) != 0)) {
                     // none of these clauses was true anywhere after the layer below: they stay false
                     if (!last && c >= 0) {
-                        const size_t at = (size_t)(wr * U + u) * m.C + c;
+                        const size_t at = (size_t)(wr * UP + u) * m.C + c;
                         surv_r[2 * at] = ra;
                         surv_r[2 * at + 1] = rb;
                     }
@@ -475,19 +518,40 @@ __global__ void __launch_bounds__(kTileThreads, 2) tile_score_kernel(DevModel m,
                 pass(block, c, ra, rb, u);
             }
             __syncthreads();
-            if (last) break;
+            if (last) {
+                if (a.span)
+                    for (int block = warp; block < cblocks; block += nwarps) {
+                        const u32 word = fired[block];
+                        if (word == 0) continue;
+                        const bool f = (word >> lane) & 1u;
+                        const int c = f ? L.order[block * 32 + lane] : 0;
+                        if (a.clause_out && f && g0 >= a.first && g0 < a.first + a.count) a.clause_out[(size_t)(g0 - a.first) * m.C + c] = 1;
+                        for (int kb = 0; kb < m.K; kb += KP) {
+                            int w[KP], mine = 0;
+                            load_weights(w, f, c, kb);
+#pragma unroll
+                            for (int k = 0; k < KP; ++k) {
+                                const int sk = __reduce_add_sync(kFull, w[k]);
+                                if (lane == k) mine = sk;
+                            }
+                            if (lane < min(KP, m.K - kb)) atomicAdd(&sums[kb + lane], mine);
+                        }
+                    }
+                if (a.span) __syncthreads();
+                break;
+            }
 
             // ---- messages of this layer -> literal rows of the next ----
             int survivors = 0;
             for (int u = 0; u < U; ++u) survivors += cnt[wr * 8 + u];
             if (survivors == 0) break;                // no clause is true anywhere: nothing can fire in later layers
             // (1) marked bits, bit-major in bufB -> node-major source rows in bufA (its literal rows are no longer needed)
-            for (int blk = tid; blk < TNC * m.MW; blk += kTileThreads) {
+            for (int blk = tid; blk < TNC * m.MW; blk += nthreads) {
                 const int j = blk % TNC, w = blk / TNC, rot = (a.rot_step * j) & 31;
                 u32 rows[32];
 #pragma unroll
                 for (int b = 0; b < 32; ++b) {
-                    const u32 x = bufB[(size_t)(b * m.MW + w) * TNC + j];
+                    const u32 x = bufB[plane_at(j, mark_rows) + ((b * m.MW + w) << pshift)];
                     rows[b] = __funnelshift_r(x, x, rot);
                 }
                 transpose32(rows);                    // rows[i] = word w of the node in slot 32j + ((i + rot) & 31)
@@ -497,8 +561,8 @@ __global__ void __launch_bounds__(kTileThreads, 2) tile_score_kernel(DevModel m,
             if (tid < 8) cnt[rd * 8 + tid] = 0;      // the list the next layer writes
             __syncthreads();
             // (2) destination rows start empty; source rows without bits are skipped by the edge pass
-            for (int i = tid; i < TN * PS; i += kTileThreads) bufB[i] = 0u;
-            for (int u = tid; u < TN; u += kTileThreads) {
+            for (int i = tid; i < TN * PS; i += nthreads) bufB[i] = 0u;
+            for (int u = tid; u < TN; u += nthreads) {
                 u32 any = 0;
                 if (tnode[u] != ~0u)
                     for (int w = 0; w < m.MW; ++w) any |= bufA[(size_t)u * PS + w];
@@ -506,7 +570,7 @@ __global__ void __launch_bounds__(kTileThreads, 2) tile_score_kernel(DevModel m,
             }
             __syncthreads();
             // (3) edge pass: a node's bits arrive at the destination rotated by the edge type (kernels.py:581)
-            for (int i = tid; i < TN * m.MW; i += kTileThreads) {
+            for (int i = tid; i < TN * m.MW; i += nthreads) {
                 const int u = i / m.MW, w = i - u * m.MW;
                 if (!pflag[u]) continue;
                 const u32 nd = tnode[u], info = pinfo[u];
@@ -523,7 +587,7 @@ __global__ void __launch_bounds__(kTileThreads, 2) tile_score_kernel(DevModel m,
             __syncthreads();
             // (4) destination rows, node-major in bufB -> literal rows of the next layer, bit-major in bufA: the message
             //     bits and, 32*MW rows further, their complements (the negated message literals)
-            for (int blk = tid; blk < TNC * m.MW; blk += kTileThreads) {
+            for (int blk = tid; blk < TNC * m.MW; blk += nthreads) {
                 const int j = blk % TNC, w = blk / TNC, rot = (a.rot_step * j) & 31;
                 u32 rows[32];
 #pragma unroll
@@ -532,24 +596,24 @@ __global__ void __launch_bounds__(kTileThreads, 2) tile_score_kernel(DevModel m,
 #pragma unroll
                 for (int b = 0; b < 32; ++b) {
                     const u32 x = __funnelshift_l(rows[b], rows[b], rot);
-                    bufA[(size_t)(b * m.MW + w) * TNC + j] = x;
-                    bufA[(size_t)(32 * m.MW + b * m.MW + w) * TNC + j] = ~x;
+                    bufA[plane_at(j, rowsm) + ((b * m.MW + w) << pshift)] = x;
+                    bufA[plane_at(j, rowsm) + ((32 * m.MW + b * m.MW + w) << pshift)] = ~x;
                 }
             }
-            for (int t = tid; t < kTilePadRows * TNC; t += kTileThreads) bufA[(size_t)(64 * m.MW) * TNC + t] = kFull;
+            for (int t = tid; t < kTilePadRows * TNC; t += nthreads) bufA[plane_at(t % TNC, rowsm) + ((64 * m.MW + t / TNC) << pshift)] = kFull;
             __syncthreads();
             // (5) bufB is the mark buffer of the next layer, if that one sends messages too
             if (d + 1 < m.D - 1) {
-                for (int i = tid; i < 32 * m.MW * TNC; i += kTileThreads) bufB[i] = 0u;
+                for (int i = tid; i < mark_words; i += nthreads) bufB[i] = 0u;
                 __syncthreads();
             }
         }
 
         // ---- class sums of the tile's graphs (only those inside the requested range) ----
-        for (int i = tid; i < ng * m.K; i += kTileThreads) {
+        for (int i = tid; i < ng * m.K; i += nthreads) {
             const int gl = i / m.K, k = i - gl * m.K;
             const int64_t gi = (int64_t)g0 + gl;
-            if (gi >= a.first && gi < a.first + a.count) a.class_sums[(size_t)(gi - a.first) * m.K + k] = sums[gl * KP + k];
+            if (gi >= a.first && gi < a.first + a.count) a.class_sums[(size_t)(gi - a.first) * m.K + k] = sums[gl * KS + k];
         }
         // ---- next tile: the CTA whose request is the last of the launch leaves the counter at zero ----
         if (more <= 0) break;
@@ -564,7 +628,7 @@ __global__ void __launch_bounds__(kTileThreads, 2) tile_score_kernel(DevModel m,
 }
 
 // ------------------------------------------------------------------------------------------------ host side
-static int tile_krow(int K) { return (K + 3) & ~3; }
+static int tile_krow(int K) { return K > 16 ? 32 : (K + 3) & ~3; }      // whole passes of classes
 
 template <int KP>
 static const void *tile_kernel_ptr() { return (const void *)tile_score_kernel<KP>; }
@@ -579,7 +643,7 @@ static const void *tile_kernel_for(int K)
     return tile_kernel_ptr<16>();
 }
 
-static int tile_kp(int K) { return K <= 2 ? 2 : K <= 4 ? 4 : K <= 8 ? 8 : K <= 10 ? 10 : K <= 12 ? 12 : 16; }
+static int tile_ks(int K) { return K <= 2 ? 2 : K <= 4 ? 4 : K <= 8 ? 8 : K <= 10 ? 10 : K <= 12 ? 12 : K <= 16 ? 16 : 32; }     // class sums of a graph
 
 int tile_model_create(TileModel *tm, const DevModel &d)
 {
@@ -659,15 +723,15 @@ int tile_model_refresh(TileModel *tm, const DevModel &d, cudaStream_t s)
 // Shared-memory plan for tiles of TNC node words; 0 bytes when the shape cannot be served.
 struct TilePlan { int words_a = 0, words_b = 0, stage_rows = 0, PS = 0; size_t bytes = 0; };
 
-static TilePlan tile_plan(const DevModel &d, int TNC, int gmax)
+static TilePlan tile_plan(const DevModel &d, int TNC, int pw, int gmax, bool span)
 {
     TilePlan p;
     const int TN = TNC * 32;
     p.PS = d.MW | 1;
-    const size_t xt = (size_t)(32 * d.L0 + kTilePadRows) * TNC;
+    const size_t xt = (size_t)tile_plane_rows(32 * d.L0 + kTilePadRows, TNC, pw) * TNC;
     // node-major message rows / bit-major message rows with their complements and the padding rows / mark buffer
-    const size_t pm = d.D > 1 ? (size_t)TN * p.PS : 0, pt = d.D > 1 ? (size_t)(64 * d.MW + kTilePadRows) * TNC : 0;
-    const size_t marks = d.D > 1 ? (size_t)32 * d.MW * TNC : 0;
+    const size_t pm = d.D > 1 ? (size_t)TN * p.PS : 0, pt = d.D > 1 ? (size_t)tile_plane_rows(64 * d.MW + kTilePadRows, TNC, pw) * TNC : 0;
+    const size_t marks = d.D > 1 ? (size_t)tile_plane_rows(32 * d.MW, TNC, pw) * TNC : 0;
     // staging: whole groups of 32 literal rows, up to 16 KB (or whatever the message rows need anyway), + 8 words of slack
     size_t stage = (size_t)32 * d.L0 * std::max<size_t>(1, std::min<size_t>(TNC, 4096 / ((size_t)32 * d.L0))) + 8;
     const size_t wa = (std::max(xt, std::max(pm, pt)) + 3) & ~(size_t)3;
@@ -675,9 +739,9 @@ static TilePlan tile_plan(const DevModel &d, int TNC, int gmax)
     p.words_a = (int)wa;
     p.words_b = (int)wb;
     p.stage_rows = (int)std::min<size_t>(TN, ((wb - 8) / d.L0) / 32 * 32);
-    const size_t words = wa + wb + (size_t)kTileMaxTypes * TNC + 2 * (size_t)TN + 4 * (size_t)gmax + (size_t)gmax * tile_kp(d.K) +
+    const size_t words = wa + wb + (size_t)kTileMaxTypes * TNC + 2 * (size_t)TN + 4 * (size_t)gmax + (size_t)gmax * tile_ks(d.K) +
                          12 + 16 + 4 + 2;
-    p.bytes = words * sizeof(u32) + (size_t)((gmax + 3) & ~3) + (size_t)TN;
+    p.bytes = words * sizeof(u32) + (size_t)((gmax + 3) & ~3) + (size_t)TN + (span ? (size_t)(d.C + 31) / 32 * sizeof(u32) : 0);
     return p;
 }
 
@@ -686,7 +750,7 @@ int tile_data_create(TileData *td, const TileModel &tm, const DevModel &d, const
                      int sm_count, cudaStream_t s)
 {
     td->supported = 0;
-    if (!tm.applicable || v->max_number_of_graph_nodes > kQuadNodes) return GTM_OK;    // a graph must fit one quad
+    if (!tm.applicable || v->max_number_of_graph_nodes > kTileSpanNodes) return GTM_OK;
     const int64_t N = v->number_of_graphs;
     if (n_max == 0) {
         n_min = ~0u;
@@ -696,28 +760,44 @@ int tile_data_create(TileData *td, const TileModel &tm, const DevModel &d, const
             n_max = std::max(n_max, n);
         }
     }
-    if (n_min < 1 || n_max > (u32)kQuadNodes) return GTM_OK;
+    if (n_min < 1 || n_max > (u32)kTileSpanNodes) return GTM_OK;
+    const bool span = n_max > (u32)kQuadNodes;         // graphs that do not fit a quad: a tile each
     const void *fn = tile_kernel_for(d.K);
     // node words per tile: the largest that lets two CTAs share an SM, else the largest that fits at all
     int TNC = 0;
     TilePlan plan;
+    bool shared_sm = true;
+    if (span) {
+        // Node words in planes of eight: a row of a pair of quads is 32 bytes, as for small graphs, whatever the graph's
+        // size.  A CTA with its SM to itself has 32 warps.
+        TNC = n_max <= 256 ? 8 : n_max <= 512 ? 16 : 32;
+        plan = tile_plan(d, TNC, 8, 1, true);
+        if (plan.bytes > (size_t)224 * 1024) return GTM_OK;
+        shared_sm = plan.bytes <= (size_t)112 * 1024;
+    }
     for (int pass = 0; pass < 2 && TNC == 0; ++pass)
         // models with many clauses spend their time in the evaluation, whose shared-memory loads are free of bank
         // conflicts with 32-byte rows (8 node words, see tile_count_kernel); small ones gain more from large tiles
         for (int cand = d.C >= 256 ? 8 : 32; cand >= 4; cand >>= 1) {
             const int gbound = (int)std::min<int64_t>(kTileMaxGraphs, std::min<int64_t>(N, cand * 32 / n_min));
-            const TilePlan p = tile_plan(d, cand, gbound);
-            if (p.bytes <= (pass == 0 ? (size_t)112 * 1024 : (size_t)224 * 1024)) { TNC = cand; plan = p; break; }
+            const TilePlan p = tile_plan(d, cand, cand, gbound, false);
+            if (p.bytes <= (pass == 0 ? (size_t)112 * 1024 : (size_t)224 * 1024)) { TNC = cand; plan = p; shared_sm = pass == 0; break; }
         }
     if (TNC == 0) return GTM_OK;
     const int TN = TNC * 32, Q = TNC / 4;
     td->TNC = TNC;
+    td->span = span;
+    td->pw = span ? 8 : TNC;
+    td->threads = shared_sm ? kTileThreads : kTileThreadsAlone;
     td->uniform_n = n_min == n_max ? (int)n_min : 0;
     td->tile_graph_host.clear();
     td->tile_graph = nullptr;
     td->gpos = nullptr;
     td->stream = s;
-    if (td->uniform_n > 0) {
+    if (span) {
+        td->graphs_per_tile = td->gmax = 1;
+        td->n_tiles = (int)N;
+    } else if (td->uniform_n > 0) {
         td->graphs_per_tile = std::min(kTileMaxGraphs, (kQuadNodes / td->uniform_n) * Q);
         td->n_tiles = (int)((N + td->graphs_per_tile - 1) / td->graphs_per_tile);
         td->gmax = (int)std::min<int64_t>(td->graphs_per_tile, N);
@@ -751,7 +831,7 @@ int tile_data_create(TileData *td, const TileModel &tm, const DevModel &d, const
         GTM_TRY(pool_alloc(&td->gpos, (size_t)N, s));
         GTM_CU(cudaMemcpyAsync(td->gpos, gpos.data(), (size_t)N * sizeof(unsigned short), cudaMemcpyHostToDevice, s));
     }
-    plan = tile_plan(d, TNC, td->gmax);
+    plan = tile_plan(d, TNC, td->pw, td->gmax, span);
     td->PS = plan.PS;
     td->words_a = plan.words_a;
     td->words_b = plan.words_b;
@@ -759,7 +839,7 @@ int tile_data_create(TileData *td, const TileModel &tm, const DevModel &d, const
     td->smem = plan.bytes;
     GTM_CU(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)td->smem));
     int per_sm = 0;
-    GTM_CU(cudaOccupancyMaxActiveBlocksPerMultiprocessorWithFlags(&per_sm, fn, kTileThreads, td->smem, 0));
+    GTM_CU(cudaOccupancyMaxActiveBlocksPerMultiprocessorWithFlags(&per_sm, fn, td->threads, td->smem, 0));
     if (per_sm < 1) { tile_data_destroy(td); return GTM_OK; }
     td->grid = std::max(1, std::min(sm_count * per_sm, td->n_tiles));
     td->n_graphs = N;
@@ -778,7 +858,7 @@ void tile_data_destroy(TileData *td)
 bool tile_supported(const TileData &td, int n_types) { return td.supported != 0 && n_types <= kTileMaxTypes; }
 
 int tile_score(TileModel *model, const TileData &td, const DevModel &d, const DevGraphs &dg, int n_types, int64_t first,
-               int64_t count, int *sums_dev, int *error_dev, int lane, cudaStream_t s)
+               int64_t count, int *sums_dev, int *clause_out_dev, int *error_dev, int lane, cudaStream_t s)
 {
     TileModel &tm = *model;
     DevGraphs g = dg;
@@ -799,7 +879,7 @@ int tile_score(TileModel *model, const TileData &td, const DevModel &d, const De
     }
     a.tile_lo = lo; a.tile_hi = hi;
     a.first = first; a.count = count; a.n_graphs = td.n_graphs;
-    a.class_sums = sums_dev; a.tile_counter = tm.counters + lane;
+    a.class_sums = sums_dev; a.clause_out = clause_out_dev; a.pw = td.pw; a.span = td.span; a.tile_counter = tm.counters + lane;
     a.TNC = td.TNC; a.PS = td.PS; a.words_a = td.words_a; a.words_b = td.words_b; a.stage_rows = td.stage_rows; a.gmax = td.gmax;
     int inv = 1;                                       // inverse of the (odd) message row stride modulo 32
     while ((td.PS * inv) % 32 != 1) inv += 2;
@@ -816,9 +896,10 @@ int tile_score(TileModel *model, const TileData &td, const DevModel &d, const De
     }
     a.surv_r = tm.surv_r[lane];
     a.error = error_dev;
+    if (clause_out_dev) GTM_CU(cudaMemsetAsync(clause_out_dev, 0, (size_t)count * d.C * sizeof(int), s));      // the kernel writes the ones
     DevModel dm = d;
     void *args[] = {&dm, &g, &a};
-    GTM_CU(cudaLaunchKernel(tile_kernel_for(d.K), dim3(grid), dim3(kTileThreads), args, td.smem, s));
+    GTM_CU(cudaLaunchKernel(tile_kernel_for(d.K), dim3(grid), dim3(td.threads), args, td.smem, s));
     return GTM_OK;
 }
 

@@ -1,4 +1,4 @@
-// Tile scoring (gtm_tile.cu): batched inference for ANY depth on graph sets whose graphs have at most 128 nodes.
+// Tile scoring (gtm_tile.cu): batched inference for ANY depth on graph sets whose graphs have at most 1,024 nodes.
 // Types and entry points used by the host runtime.
 #pragma once
 #include <vector>
@@ -41,6 +41,9 @@ struct TileData {
     int words_a = 0, words_b = 0;       // sizes of the two big shared-memory buffers (words)
     int stage_rows = 0;                 // literal rows the staging buffer holds
     int gmax = 0;                       // most graphs in one tile
+    int pw = 0;                         // node words of a literal row: TNC, or planes of 8 (span)
+    bool span = false;                  // graphs of more than 128 nodes: a tile is one graph
+    int threads = 0;                    // of a CTA
     int uniform_n = 0;                  // > 0: every graph has this many nodes: slots follow from the graph number
     int graphs_per_tile = 0;            // uniform sets: graphs per tile (no tile table)
     int n_tiles = 0;
@@ -60,8 +63,9 @@ int tile_data_create(TileData *td, const TileModel &tm, const DevModel &d, const
                      int sm_count, cudaStream_t s);
 void tile_data_destroy(TileData *td);
 bool tile_supported(const TileData &td, int n_types);
+// `clause_out_dev`: clause outputs int32[count][C], or null.
 // `lane` (0 or 1): launches that may run side by side, on disjoint tiles, take different ones.
 int tile_score(TileModel *model, const TileData &td, const DevModel &d, const DevGraphs &dg, int n_types, int64_t first,
-               int64_t count, int *sums_dev, int *error_dev, int lane, cudaStream_t s);
+               int64_t count, int *sums_dev, int *clause_out_dev, int *error_dev, int lane, cudaStream_t s);
 
 }  // namespace gtm
