@@ -117,6 +117,8 @@ void lane_destroy(StageLane *l)
 {
     cudaSetDevice(l->device);
     for (int i = 0; i < kStageSlots; ++i) {
+        if (l->up[i].host) cudaFreeHost(l->up[i].host);
+        if (l->down[i].host) cudaFreeHost(l->down[i].host);
         if (l->up[i].done) cudaEventDestroy(l->up[i].done);
         if (l->down[i].done) cudaEventDestroy(l->down[i].done);
     }
@@ -125,7 +127,6 @@ void lane_destroy(StageLane *l)
     if (l->back) cudaStreamDestroy(l->back);
     if (l->aux) cudaStreamDestroy(l->aux);
     if (l->small) cudaFreeHost(l->small);
-    if (l->big) cudaFreeHost(l->big);
     delete l;
 }
 
@@ -143,14 +144,10 @@ int lane_fill(StageLane *l)
     return GTM_OK;
 }
 
-int lane_big(StageLane *l)
+// The slot's buffer; nothing of the slot is in flight.
+int slot_reserve(StageSlot &slot)
 {
-    if (l->big) return GTM_OK;
-    GTM_CU(cudaMallocHost((void **)&l->big, 2 * kStageSlots * kStagePiece));
-    for (int i = 0; i < kStageSlots; ++i) {
-        l->up[i].host = l->big + (size_t)i * kStagePiece;
-        l->down[i].host = l->big + (size_t)(kStageSlots + i) * kStagePiece;
-    }
+    if (!slot.host) GTM_CU(cudaMallocHost((void **)&slot.host, kStagePiece));
     return GTM_OK;
 }
 
@@ -273,13 +270,13 @@ int stage_up(StageLane *lane, void *dst, const void *src, size_t bytes, bool pin
 {
     if (bytes == 0) return GTM_OK;
     if (pinned) { GTM_CU(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, s)); return GTM_OK; }
-    GTM_TRY(lane_big(lane));
     for (size_t at = 0; at < bytes; at += kStagePiece) {
         const size_t n = std::min(kStagePiece, bytes - at);
         StageSlot &slot = lane->up[lane->up_next];
         lane->up_next = (lane->up_next + 1) % kStageSlots;
         if (slot.busy) GTM_CU(cudaEventSynchronize(slot.done));
         slot.busy = false;
+        GTM_TRY(slot_reserve(slot));
         host_copy(slot.host, (const char *)src + at, n, true);
         GTM_CU(cudaMemcpyAsync((char *)dst + at, slot.host, n, cudaMemcpyHostToDevice, s));
         GTM_CU(cudaEventRecord(slot.done, s));
@@ -306,14 +303,13 @@ int stage_down(StageLane *lane, void *dst, const void *src, size_t bytes, bool p
         GTM_CU(cudaEventRecord(lane->event[3], s));       // stage_down_finish waits for the last of these
         return GTM_OK;
     }
-    GTM_TRY(lane_big(lane));
-    // pieces of a quarter of the result: the host copies a piece while the copy engine brings the next
-    const size_t piece = std::min(kStagePiece, std::max<size_t>((size_t)512 << 10, (bytes / 4 + 4095) & ~(size_t)4095));
-    for (size_t at = 0; at < bytes; at += piece) {
-        const size_t n = std::min(piece, bytes - at);
+    // the host copies a piece while the copy engine brings the next
+    for (size_t at = 0; at < bytes; at += kStagePiece) {
+        const size_t n = std::min(kStagePiece, bytes - at);
         StageSlot &slot = lane->down[lane->down_next];
         lane->down_next = (lane->down_next + 1) % kStageSlots;
         GTM_TRY(slot_land(slot));
+        GTM_TRY(slot_reserve(slot));
         GTM_CU(cudaMemcpyAsync(slot.host, (const char *)src + at, n, cudaMemcpyDeviceToHost, s));
         GTM_CU(cudaEventRecord(slot.done, s));
         slot.busy = true;

@@ -1,8 +1,9 @@
 """Result arrays in recycled page-locked memory.
 
 A result of a few megabytes in a fresh numpy array costs a page fault per page and a copy out of a staging buffer; in
-page-locked memory the copy engine writes it directly, in the time of the transfer.  Page-locking is slow (about a
-millisecond for 4 MB), so the memory of an array that nobody refers to any more is kept for the next result.
+page-locked memory the copy engine writes it directly, in the time of the transfer.  Page-locking is slow (0.5 ms per MB),
+so the memory of an array that nobody refers to any more is kept for the next result, and memory is locked only for a
+size that has been asked for before: a program's first results are ordinary arrays.
 """
 
 import collections
@@ -17,6 +18,9 @@ from . import _lib
 SMALLEST, LARGEST = 64 << 10, 16 << 20      # bytes of an array that is worth it / that is not too much to lock
 MOST = 128 << 20                            # bytes locked at a time, arrays in use included
 
+AT_FIRST = 2                                # arrays of a size class that are ordinary memory
+
+_asked = collections.Counter()                          # size class -> arrays asked for, up to AT_FIRST
 _free = collections.defaultdict(collections.deque)      # size class -> addresses
 _lock = threading.Lock()
 _locked = 0
@@ -65,6 +69,9 @@ def empty(shape, dtype):
     if not SMALLEST <= nbytes <= LARGEST:
         return np.empty(shape, dtype=dtype)
     size = _size_class(nbytes)
+    if _asked[size] < AT_FIRST:
+        _asked[size] += 1
+        return np.empty(shape, dtype=dtype)
     address = _take(size)
     if not address:
         return np.empty(shape, dtype=dtype)
