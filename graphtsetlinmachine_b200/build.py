@@ -10,8 +10,9 @@ import sys
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.path.join(HERE, "libgtm_b200.so")
-SOURCES = [os.path.join(HERE, "csrc", f) for f in ("gtm_api.cu", "gtm_fit_chain.cu", "gtm_fit_chain_rw1.cu", "gtm_fit_chain_rw4.cu", "gtm_fit_chain_rw16.cu",
-                                                   "gtm_fit_chain_rw32.cu", "gtm_fit_global.cu", "gtm_fit_resident.cu", "gtm_stage.cu", "gtm_stream.cu", "gtm_tile.cu")]
+SOURCES = [os.path.join(HERE, "csrc", f) for f in
+           ["gtm_fit_chain_%s_rw%d.cu" % (kind, rw) for kind in ("wide", "narrow") for rw in (1, 4, 16, 32)] +
+           ["gtm_api.cu", "gtm_fit_chain.cu", "gtm_fit_global.cu", "gtm_fit_resident.cu", "gtm_stage.cu", "gtm_stream.cu", "gtm_tile.cu"]]
 NVCC_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17", "-Xcompiler", "-fPIC"]
 
 

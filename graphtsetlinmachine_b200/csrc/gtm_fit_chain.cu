@@ -8,15 +8,22 @@
 #include "gtm_handles.h"
 #include "gtm_fit_chain.cuh"
 
-const void *fit_chain_kernel_rw1(bool one_layer, bool hybrid);
-const void *fit_chain_kernel_rw4(bool one_layer, bool hybrid);
-const void *fit_chain_kernel_rw16(bool one_layer, bool hybrid);
-const void *fit_chain_kernel_rw32(bool one_layer, bool hybrid);
+const void *fit_chain_kernel_narrow_rw1(bool one_layer, bool hybrid);
+const void *fit_chain_kernel_narrow_rw4(bool one_layer, bool hybrid);
+const void *fit_chain_kernel_narrow_rw16(bool one_layer, bool hybrid);
+const void *fit_chain_kernel_narrow_rw32(bool one_layer, bool hybrid);
+const void *fit_chain_kernel_wide_rw1(bool one_layer, bool hybrid);
+const void *fit_chain_kernel_wide_rw4(bool one_layer, bool hybrid);
+const void *fit_chain_kernel_wide_rw16(bool one_layer, bool hybrid);
+const void *fit_chain_kernel_wide_rw32(bool one_layer, bool hybrid);
 
-static const void *chain_kernel_for(int rw, bool one_layer, bool hybrid)
+static const void *chain_kernel_for(int rw, bool one_layer, bool hybrid, bool narrow)
 {
-    return rw == 1 ? fit_chain_kernel_rw1(one_layer, hybrid) : rw == 4 ? fit_chain_kernel_rw4(one_layer, hybrid)
-         : rw == 16 ? fit_chain_kernel_rw16(one_layer, hybrid) : fit_chain_kernel_rw32(one_layer, hybrid);
+    if (narrow)
+        return rw == 1 ? fit_chain_kernel_narrow_rw1(one_layer, hybrid) : rw == 4 ? fit_chain_kernel_narrow_rw4(one_layer, hybrid)
+             : rw == 16 ? fit_chain_kernel_narrow_rw16(one_layer, hybrid) : fit_chain_kernel_narrow_rw32(one_layer, hybrid);
+    return rw == 1 ? fit_chain_kernel_wide_rw1(one_layer, hybrid) : rw == 4 ? fit_chain_kernel_wide_rw4(one_layer, hybrid)
+         : rw == 16 ? fit_chain_kernel_wide_rw16(one_layer, hybrid) : fit_chain_kernel_wide_rw32(one_layer, hybrid);
 }
 
 __global__ void largest_edge_type_kernel(const u32 *edge, size_t edges, u32 *out)
@@ -89,8 +96,10 @@ static ChainPlan plan_chain(const gtm_model *m, const gtm_dataset *ds)
     for (int l = 1; l < d.D; ++l) one_p = one_p && d.p_mask[l] == d.p_mask[0];
     a.narrow = one_p && d.L0 <= 32 && (d.D == 1 || d.M <= 32);
     if (a.narrow) {
-        // the stream of one Type-I class is made in the shadow of the vote exchange; room for up to four classes
-        a.spec_rounds = d.p_mask[0] >= 1.0f ? 0 : (d.K + 3 + 32 * words_all + 127) / 128;
+        // The first rounds of the stream are made in the shadow of the vote exchange, for every clause, wanted or not: two of
+        // them fit the shadow (4,000 images x 2,500 clauses: 24.1 ms without, 23.9 with two, 24.0 with the three that one class
+        // needs; 200 sequences of three layers, 21 rounds: 8.1 ms without or with two, 9.1 with all).  Room for four classes.
+        a.spec_rounds = d.p_mask[0] >= 1.0f ? 0 : std::min(2, (d.K + 3 + 32 * words_all + 127) / 128);
         a.pre_words = (std::max(4 * a.spec_rounds, (d.K + 3) / 32 + 1 + std::min(d.K, 4) * words_all) + 4 + 7) & ~3;
     }
     // One CTA learns a model of few clauses alone: every grid-wide step (about 2,000 cycles; one per graph, and two per
@@ -104,7 +113,7 @@ static ChainPlan plan_chain(const gtm_model *m, const gtm_dataset *ds)
         const int want_warps = a.narrow ? std::max(8, cpc) : 32;
         for (int variant = 0; variant < 4; ++variant) {        // planes resident, then include planes only; with and without staged graphs
             const bool hybrid = variant >= 2, stage = (variant & 1) == 0;
-            const int warps = std::min(want_warps, (hybrid ? kChainThreads : kChainResidentThreads) / 32);
+            const int warps = std::min(want_warps, chain_threads(hybrid, a.narrow != 0) / 32);
             a.stage_nodes = stage ? std::min(ds->max_nodes, 512) : 0;
             a.stage_words = stage ? (std::min(ds->max_nodes * d.L0, 4096) + 3) & ~3 : 0;
             a.stage_edges = stage && D1 > 0 ? 512 : 0;
@@ -114,7 +123,7 @@ static ChainPlan plan_chain(const gtm_model *m, const gtm_dataset *ds)
                                  ((msg + 3) & ~(size_t)3) + (size_t)32 * std::max(d.L0, D1 > 0 ? d.MW : 0) * rw + (size_t)kTransposedTypes * rw4 +
                                  (size_t)cpc * (kChainRec + a.pre_words + a.clause_words);
             const size_t smem = words * sizeof(u32);
-            const void *fn = chain_kernel_for(rw, d.D == 1, hybrid);
+            const void *fn = chain_kernel_for(rw, d.D == 1, hybrid, a.narrow != 0);
             cudaFuncAttributes fa;
             if (cudaFuncGetAttributes(&fa, fn) != cudaSuccess) { cudaGetLastError(); return plan; }
             if (smem + fa.sharedSizeBytes > 227 * 1024 || 32 * warps > fa.maxThreadsPerBlock) continue;
@@ -133,7 +142,7 @@ int launch_fit_chain(gtm_model *m, gtm_dataset *ds, int n_types, const int *Y_de
 {
     const DevModel &d = m->dm;
     *done = 0;
-    if (d.K > 32 || d.SB > 8 || ds->max_nodes > 1024 || n_types > kTransposedTypes) return GTM_OK;
+    if (d.recorded || d.K > 32 || d.SB != kChainStateBits || ds->max_nodes > 1024 || n_types > kTransposedTypes) return GTM_OK;
     ChainPlan plan = plan_chain(m, ds);
     if (!plan.ok) return GTM_OK;
     GTM_TRY(chain_prepare(m, ds, plan.rw));
@@ -149,10 +158,14 @@ int launch_fit_chain(gtm_model *m, gtm_dataset *ds, int n_types, const int *Y_de
     a.missing = m->opt_fit_missing_cta;
     a.node_bits = ds->chain_bits; a.rows_t = ds->chain_rows_t; a.rows_n = ds->chain_rows_n;
     a.bit_off = m->hv_off; a.bit_clause = m->hv_clause; a.tmax = std::max(0, ds->largest_edge_type);
+    for (int r = 0; r < 10; ++r) {
+        a.key[2 * r] = d.seed_lo + (u32)r * 0x9E3779B9u;
+        a.key[2 * r + 1] = d.seed_hi + (u32)r * 0xBB67AE85u;
+    }
     DevGraphs g = ds->dg;
     g.n_types = n_types;
     DevModel dm = d;
-    const void *fn = chain_kernel_for(plan.rw, d.D == 1, plan.hybrid);
+    const void *fn = chain_kernel_for(plan.rw, d.D == 1, plan.hybrid, plan.a.narrow != 0);
     GTM_CU(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)plan.smem));
     void *args[] = {&dm, &g, &a};
     GTM_CU(cudaLaunchCooperativeKernel(fn, dim3(plan.grid), dim3(plan.threads), args, plan.smem, m->stream));

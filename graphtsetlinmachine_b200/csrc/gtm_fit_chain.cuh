@@ -31,8 +31,11 @@
 
 namespace gtm {
 
-constexpr int kChainThreads = 1024, kChainResidentThreads = 768;      // most threads of a CTA with and without planes in global memory;
-                                                                       // they set the register budgets (64 and 80)
+// Most threads of a CTA; they set the register budgets.  80 registers for wide layers, whose work items all warps share (300
+// multigraphs, 20,000 clauses: 36.3 ms with 24 warps of 80, 37.2 with 32 of 64), 96 for narrow ones, where a warp does
+// everything for its clause and there is hardly more than a clause per warp, 64 where many clauses share a CTA's memory.
+constexpr int chain_threads(bool hybrid, bool narrow) { return narrow ? (hybrid ? 1024 : 576) : 768; }
+constexpr int kChainStateBits = 8;       // state bits of an automaton: constant, or every step of an addition is a predicate of its own
 constexpr int kChainStages = 3;          // graphs in shared memory: current, next, next but one (on its way)
 constexpr int kChainRowWise = 3;         // graphs of at most this many nodes are evaluated row-wise
 constexpr int kChainMaxType = 24;        // largest edge type of a set whose messages are pulled: the window is 8 + 24 bits
@@ -52,7 +55,7 @@ struct ChainArgs {
     int missing;                 // test hook: waits expect this many arrivals more than there are CTAs
     int clauses_per_cta, clause_words;
     int solo;                    // one CTA: its barriers replace the grid's, messages stay in shared memory
-    int narrow;                  // a clause's masks come from one packed stream (all layers of one probability, up to 32 words)
+    int narrow;                  // kNarrow: a clause's masks come from one packed stream (all layers of one probability, up to 32 words)
     int pre_words, spec_rounds;  // narrow: words of that stream kept per clause; rounds made in the exchange's shadow
     int stage_words, stage_nodes, stage_edges;       // room for a staged graph: literal words, nodes, edge rows
     int max_nodes;
@@ -61,35 +64,60 @@ struct ChainArgs {
     u32 *rows_n;                 // [D-1][max_nodes][MW] message rows, node-major
     const int *bit_off, *bit_clause;                 // clauses whose hypervector holds message bit b: bit_clause[bit_off[b] ..]
     int tmax;                    // largest edge type
+    u32 key[20];                 // Philox round keys: operands in the constant bank instead of two additions a round
 };
+
+// Four consecutive draws of the stream of clause c (draw_block without recorded draws, which the older kernels serve).
+__device__ __forceinline__ uint4 chain_draws(const ChainArgs &a, u32 c, u64 block)
+{
+    u32 c0 = (u32)block, c1 = (u32)(block >> 32), c2 = c, c3 = 0;
+#pragma unroll
+    for (int r = 0; r < 10; ++r) {
+        const u32 lo0 = 0xD2511F53u * c0, hi0 = __umulhi(0xD2511F53u, c0);
+        const u32 lo1 = 0xCD9E8D57u * c2, hi1 = __umulhi(0xCD9E8D57u, c2);
+        c0 = hi1 ^ c1 ^ a.key[2 * r]; c1 = lo1;
+        c2 = hi0 ^ c3 ^ a.key[2 * r + 1]; c3 = lo0;
+    }
+    return make_uint4(c0, c1, c2, c3);
+}
+
+__device__ __forceinline__ u32 chain_draw_at(const ChainArgs &a, u32 c, u64 i)
+{
+    const uint4 o = chain_draws(a, c, i >> 2);
+    const u32 even = (i & 2) ? o.z : o.x, odd = (i & 2) ? o.w : o.y;
+    return (i & 1) ? odd : even;
+}
 
 // Mask word of a lane in a stretch of 32 words: outcomes [draw <= p] of the 32 draws that start `shift` (0..3) draws into
 // Philox block `block` (the lane's own; the next lane's block is 8 further on).  A lane makes the eight blocks of its own
 // word, so nothing is packed or exchanged but the `shift` bits that spill into the next word.
-__device__ __forceinline__ u32 lane_mask(const DevModel &m, int c, u64 block, int shift, u32 below, int lane)
+__device__ __forceinline__ u32 lane_mask(const ChainArgs &a, int c, u64 block, int shift, u32 below, int lane)
 {
     u32 word = 0;
 #pragma unroll 2
     for (int q = 0; q < 8; ++q) {
-        const uint4 o = draw_block(m.recorded, m.recorded_len, m.seed_lo, m.seed_hi, (u32)c, block + q);
-        const u32 nib = (o.x < below ? 1u : 0u) | (o.y < below ? 2u : 0u) | (o.z < below ? 4u : 0u) | (o.w < below ? 8u : 0u);
-        word |= nib << (4 * q);
+        const uint4 o = chain_draws(a, (u32)c, block + q);
+        word >>= 4;                                     // block q ends up at bits 4q .. 4q+3
+        if (o.x < below) word |= 1u << 28;
+        if (o.y < below) word |= 1u << 29;
+        if (o.z < below) word |= 1u << 30;
+        if (o.w < below) word |= 1u << 31;
     }
     if (shift == 0) return word;
     u32 next = __shfl_down_sync(kFull, word, 1);
     if (lane == 31) {
-        const uint4 o = draw_block(m.recorded, m.recorded_len, m.seed_lo, m.seed_hi, (u32)c, block + 8);
+        const uint4 o = chain_draws(a, (u32)c, block + 8);
         next = (o.x < below ? 1u : 0u) | (o.y < below ? 2u : 0u) | (o.z < below ? 4u : 0u);
     }
     return __funnelshift_r(word, next, shift);
 }
 
 // Rounds [q0, q1) of a clause's packed stream that starts at Philox block `block0`: words 4q .. 4q+3 of dst.
-__device__ __forceinline__ void stream_rounds(const DevModel &m, int c, u64 block0, int q0, int q1, u32 below, u32 *dst, int lane)
+__device__ __forceinline__ void stream_rounds(const ChainArgs &a, int c, u64 block0, int q0, int q1, u32 below, u32 *dst, int lane)
 {
 #pragma unroll 2
     for (int q = q0; q < q1; ++q) {
-        const uint4 o = draw_block(m.recorded, m.recorded_len, m.seed_lo, m.seed_hi, (u32)c, block0 + (u64)q * 32 + lane);
+        const uint4 o = chain_draws(a, (u32)c, block0 + (u64)q * 32 + lane);
         u32 w = (o.x < below ? 1u : 0u) | (o.y < below ? 2u : 0u) | (o.z < below ? 4u : 0u) | (o.w < below ? 8u : 0u);
         w <<= 4 * (lane & 7);
         w |= __shfl_xor_sync(kFull, w, 1);
@@ -109,13 +137,14 @@ __device__ __forceinline__ int nth_set_bit(u32 word, int rank, int lane)
 // the include plane at inc[w].  `masks(rank)` gives the lane's mask word of the Type-I class of that rank.  Returns the
 // change of the lane's include count (bits of `valid`).
 template <class Masks>
-__device__ __forceinline__ int update_words(int SB, int boost, int w, int W, u32 *lo, u32 *inc, u32 x, int upd, bool clause_true, bool within,
+__device__ __forceinline__ int update_words(int boost, int w, int W, u32 *lo, u32 *inc, u32 x, int upd, bool clause_true, bool within,
                                             u32 valid, Masks masks)
 {
+    constexpr int SB = kChainStateBits;
     const bool mine = w < W;
-    u32 pl[8];
+    u32 pl[SB - 1];
 #pragma unroll
-    for (int b = 0; b < 8; ++b) pl[b] = (b < SB - 1 && mine) ? lo[(size_t)b * W + w] : 0u;
+    for (int b = 0; b < SB - 1; ++b) pl[b] = mine ? lo[(size_t)b * W + w] : 0u;
     u32 in = mine ? inc[w] : 0u;
     const u32 before = in;
     bool dirty = false;
@@ -124,25 +153,21 @@ __device__ __forceinline__ int update_words(int SB, int boost, int w, int W, u32
     auto add = [&](u32 active) {
         u32 carry = active;
 #pragma unroll
-        for (int b = 0; b < 8; ++b)
-            if (b < SB - 1) { const u32 nx = pl[b] & carry; pl[b] ^= carry; carry = nx; }
+        for (int b = 0; b < SB - 1; ++b) { const u32 nx = pl[b] & carry; pl[b] ^= carry; carry = nx; }
         const u32 over = in & carry;
         in ^= carry;
 #pragma unroll
-        for (int b = 0; b < 8; ++b)
-            if (b < SB - 1) pl[b] |= over;
+        for (int b = 0; b < SB - 1; ++b) pl[b] |= over;
         in |= over;
     };
     auto sub = [&](u32 active) {
         u32 borrow = active;
 #pragma unroll
-        for (int b = 0; b < 8; ++b)
-            if (b < SB - 1) { const u32 nx = ~pl[b] & borrow; pl[b] ^= borrow; borrow = nx; }
+        for (int b = 0; b < SB - 1; ++b) { const u32 nx = ~pl[b] & borrow; pl[b] ^= borrow; borrow = nx; }
         const u32 under = ~in & borrow;
         in ^= borrow;
 #pragma unroll
-        for (int b = 0; b < 8; ++b)
-            if (b < SB - 1) pl[b] &= ~under;
+        for (int b = 0; b < SB - 1; ++b) pl[b] &= ~under;
         in &= ~under;
     };
     u32 todo = __ballot_sync(kFull, upd != 0);
@@ -167,8 +192,7 @@ __device__ __forceinline__ int update_words(int SB, int boost, int w, int W, u32
     }
     if (mine && dirty) {
 #pragma unroll
-        for (int b = 0; b < 8; ++b)
-            if (b < SB - 1) lo[(size_t)b * W + w] = pl[b];
+        for (int b = 0; b < SB - 1; ++b) lo[(size_t)b * W + w] = pl[b];
         inc[w] = in;
     }
     return mine ? __popc(in & valid) - __popc(before & valid) : 0;
@@ -397,16 +421,18 @@ __device__ __forceinline__ void solo_messages(const DevModel &m, const GraphView
 // [4][4] graph sizes | [2] work list counters .. | [3] staged graphs | message scratch | T: transposed rows, then type rows |
 // [warps] nothing | per clause: record [kChainRec], mask stream [pre_words], state [clause_words] =
 // draw position (2), include count, its pending change, weights [KP], node words [RW], planes (or include planes) of all layers
-template <int RW, bool kOneLayer, bool kHybrid>
-__global__ void __launch_bounds__(kHybrid ? kChainThreads : kChainResidentThreads, 1) fit_chain_kernel(DevModel m_in, DevGraphs g, ChainArgs a)
+template <int RW, bool kOneLayer, bool kHybrid, bool kNarrow>
+__global__ void __launch_bounds__(chain_threads(kHybrid, kNarrow), 1) fit_chain_kernel(DevModel m_in, DevGraphs g, ChainArgs a)
 {
     DevModel m = m_in;
     if (kOneLayer) m.D = 1;
     extern __shared__ __align__(16) u32 s_mem[];
     __shared__ MaskProb s_prob[kMaxDepth];
     __shared__ int s_abort, s_items, s_next_item;
+    __shared__ long long s_lap[9];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
-    const int KP = (m.K + 3) & ~3, SB = m.SB;
+    constexpr int SB = kChainStateBits;
+    const int KP = (m.K + 3) & ~3;
     const bool solo = a.solo != 0;
     int *s_sum = reinterpret_cast<int *>(s_mem), *s_total = s_sum + KP, *s_target = s_total + KP;
     float *s_thr = reinterpret_cast<float *>(s_target + KP);
@@ -582,7 +608,17 @@ __global__ void __launch_bounds__(kHybrid ? kChainThreads : kChainResidentThread
     unsigned long long seen_votes[2] = {0, 0};
     unsigned nb = 0;
     const bool timer = a.timers != 0 && blockIdx.x == 0 && threadIdx.x < 32;
-    long long t_eval = 0, t_bar = 0, t_tot = 0, t_fb = 0, t_x0 = 0, t_x1 = 0, t_x2 = 0, t_x3 = 0, t0 = clock64(), t1;
+    // phase times live in shared memory: as variables they took 20 registers of every thread
+    if (timer && lane < 9) s_lap[lane] = lane == 8 ? clock64() : 0;
+    __syncwarp();
+    auto lap = [&](int phase) {
+        if (timer) {
+            const long long now = clock64(), before = s_lap[8], sum = s_lap[phase];
+            __syncwarp();
+            if (lane == 0) { s_lap[phase] = sum + now - before; s_lap[8] = now; }
+            __syncwarp();
+        }
+    };
 
     int slot = 0;                                                       // staging slot of the current graph
     for (u64 step = 0; step < steps; ++step) {
@@ -593,21 +629,21 @@ __global__ void __launch_bounds__(kHybrid ? kChainThreads : kChainResidentThread
         for (int d = 1; d < m.D; ++d) {
             u32 *bits = a.node_bits + (size_t)(d - 1) * m.C * RW, *rows_t = a.rows_t + (size_t)(d - 1) * 32 * m.MW * RW,
                 *rows_n = a.rows_n + (size_t)(d - 1) * a.max_nodes * m.MW;
-            GTM_LAP(t_eval);
+            lap(0);
             if (solo) {
                 rows_n = s_msg + (size_t)d * a.max_nodes * m.MW;
                 __syncthreads();
                 solo_messages(m, gv, s_msg, rows_n);
                 if (!row_wise(gv.n)) transpose_rows<RW>(rows_n, gv.n, m.MW, s_T);
                 __syncthreads();
-                GTM_LAP(t_x1);
+                lap(5);
             } else {
                 if (!barrier(++nb)) return;
-                GTM_LAP(t_bar);
+                lap(1);
                 pull_messages<RW>(a, m, gv, bits, rows_t, rows_n, s_msg, s_msg + 32 * RW, s_msg + 64 * RW);
-                GTM_LAP(t_x0);
+                lap(4);
                 if (!barrier(++nb)) return;
-                GTM_LAP(t_bar);
+                lap(1);
                 // 32*MW*RW words, a multiple of 128 bytes
                 for (int i = threadIdx.x; i < 8 * m.MW * RW; i += blockDim.x) {
                     const unsigned dst = (unsigned)__cvta_generic_to_shared(s_T + 4 * i);
@@ -615,7 +651,7 @@ __global__ void __launch_bounds__(kHybrid ? kChainThreads : kChainResidentThread
                 }
                 wait_copies();
                 __syncthreads();
-                GTM_LAP(t_x1);
+                lap(5);
             }
             const bool last = d == m.D - 1;
             for (int i = warp; i < mine; i += nwarps) {
@@ -645,7 +681,7 @@ __global__ void __launch_bounds__(kHybrid ? kChainThreads : kChainResidentThread
         if (lane < m.K && vote != 0) atomicAdd(&s_sum[lane], vote);
         vote = 0;
         __syncthreads();
-        GTM_LAP(t_eval);
+        lap(0);
         const int *y = s_y + slot * KP;
         const int set = (int)(step & 1);
         if (warp == 0 && lane < m.K) {
@@ -668,7 +704,7 @@ __global__ void __launch_bounds__(kHybrid ? kChainThreads : kChainResidentThread
             int *rec = record(i);
             const u32 *nd = nodes(i);
             const u64 pos = *reinterpret_cast<const u64 *>(state(i));
-            const u32 draw = draw_at(m, c, pos + lane);
+            const u32 draw = chain_draw_at(a, c, pos + lane);
             // one true node, uniformly: the (draw % count)-th set bit in ascending node order (kernels.py:319-349)
             int count, chosen = -1, pc = 0;
             if (RW == 1) count = __popc(nd[0]);
@@ -692,12 +728,12 @@ __global__ void __launch_bounds__(kHybrid ? kChainThreads : kChainResidentThread
             const u64 after = pos + (count > 0 ? 1 : 0);
             if (lane == 0) { rec[0] = chosen; rec[1] = count > 0; }
             rec[8 + lane] = (int)draw;
-            if (a.narrow) stream_rounds(m, c, (after + (u64)m.K) >> 2, 0, a.spec_rounds, s_prob[0].count, stream(i), lane);
+            if constexpr (kNarrow) stream_rounds(a, c, (after + (u64)m.K) >> 2, 0, a.spec_rounds, s_prob[0].count, stream(i), lane);
         }
         const bool more = step + 1 < steps;
         const GraphView gn = view_of(step + 1, slot1);
         if (more) prepare_graph(gn);
-        GTM_LAP(t_x2);
+        lap(6);
         // ---- votes in ----
         if (!solo && warp == 0) {
             bool gave_up = false;
@@ -720,7 +756,7 @@ __global__ void __launch_bounds__(kHybrid ? kChainThreads : kChainResidentThread
         }
         __syncthreads();
         if (s_abort) return;
-        GTM_LAP(t_tot);
+        lap(2);
         // ---- feedback and the next graph's first layer ----
         const bool final_step = !more;
         for (int i = warp; i < mine; i += nwarps) {
@@ -740,7 +776,7 @@ __global__ void __launch_bounds__(kHybrid ? kChainThreads : kChainResidentThread
             int upd_all = 0;                                            // lane k: feedback type of class k
             for (int kb = 0; kb < m.K; kb += 15) {
                 const int kn = min(15, m.K - kb), at = kb == 0 ? taken : 0;
-                if (kb > 0) draw = draw_at(m, c, pos + lane);
+                if (kb > 0) draw = chain_draw_at(a, c, pos + lane);
                 const float uni = to_uniform(draw);
                 const bool has = lane < kn;
                 int w = 0, sign = 1, t = 1;
@@ -775,7 +811,7 @@ __global__ void __launch_bounds__(kHybrid ? kChainThreads : kChainResidentThread
             const bool any_feedback = positive != 0 || __ballot_sync(kFull, upd_all < 0 && clause_true) != 0;
             const int npos = __popc(positive);
             const int words_all = m.L0 + (m.D - 1) * m.M;
-            if (a.narrow) {
+            if constexpr (kNarrow) {
                 if (any_feedback) {
                     const u64 block0 = (after + (u64)m.K) >> 2;
                     const int off0 = (int)(pos - 4 * block0);
@@ -783,7 +819,7 @@ __global__ void __launch_bounds__(kHybrid ? kChainThreads : kChainResidentThread
                     const int rounds = all_ones ? 0 : (off0 + 32 * npos * words_all + 127) >> 7;
                     u32 *pre = stream(i);
                     const bool packed = 4 * rounds + 1 <= a.pre_words;
-                    if (npos > 0 && packed) stream_rounds(m, c, block0, a.spec_rounds, rounds, s_prob[0].count, pre, lane);
+                    if (npos > 0 && packed) stream_rounds(a, c, block0, a.spec_rounds, rounds, s_prob[0].count, pre, lane);
                     __syncwarp();
                     const bool within = (int)st[2] <= m.max_included;
                     int change = 0, first_word = 0;                     // first_word: stream words of the layers before
@@ -797,7 +833,7 @@ __global__ void __launch_bounds__(kHybrid ? kChainThreads : kChainResidentThread
                         }
                         const u32 valid = lane == W - 1 ? layer_mask(l) : kFull;
                         const int base = first_word;
-                        change += update_words(SB, m.boost, lane, W, planes(i, l), include(i, l), x, upd_all, clause_true, within, valid, [&](int rank) {
+                        change += update_words(m.boost, lane, W, planes(i, l), include(i, l), x, upd_all, clause_true, within, valid, [&](int rank) {
                             if (all_ones) return kFull;
                             const int bit = off0 + 32 * (base + rank * W + lane);
                             if (packed) {
@@ -806,7 +842,7 @@ __global__ void __launch_bounds__(kHybrid ? kChainThreads : kChainResidentThread
                             }
                             // more Type-I classes than the buffer holds: the lane makes its own word
                             const u64 first_draw = pos + (u64)32 * (u64)(base + rank * W);
-                            return lane_mask(m, c, (first_draw >> 2) + (u64)8 * lane, (int)(first_draw & 3), s_prob[0].count, lane);
+                            return lane_mask(a, c, (first_draw >> 2) + (u64)8 * lane, (int)(first_draw & 3), s_prob[0].count, lane);
                         });
                         first_word += npos * W;
                     }
@@ -826,8 +862,8 @@ __global__ void __launch_bounds__(kHybrid ? kChainThreads : kChainResidentThread
                 rec[8 + lane] = upd_all;
             }
         }
-        if (!a.narrow) {
-            GTM_LAP(t_x3);
+        if constexpr (!kNarrow) {
+            lap(7);
             __syncthreads();
             const int per0 = (m.L0 + 31) >> 5, perM = (m.M + 31) >> 5, per = per0 + (m.D - 1) * perM, total = s_items * per;
             while (true) {
@@ -851,11 +887,11 @@ __global__ void __launch_bounds__(kHybrid ? kChainThreads : kChainResidentThread
                     else x = msg_word(a.rows_n + ((size_t)(l - 1) * a.max_nodes + chosen) * m.MW, w, m.MS, m.MW);
                 }
                 const MaskProb mp = s_prob[l];
-                int change = update_words(SB, m.boost, w, W, planes(i, l), include(i, l), x, upd, clause_true, (int)st[2] <= m.max_included,
+                int change = update_words(m.boost, w, W, planes(i, l), include(i, l), x, upd, clause_true, (int)st[2] <= m.max_included,
                                           w == W - 1 ? layer_mask(l) : kFull, [&](int rank) {
                     if (mp.p >= 1.0f) return kFull;
                     const u64 first_draw = layer_pos + (u64)32 * (u64)(rank * W + g0);
-                    return lane_mask(m, c_lo + i, (first_draw >> 2) + (u64)8 * lane, (int)(first_draw & 3), mp.count, lane);
+                    return lane_mask(a, c_lo + i, (first_draw >> 2) + (u64)8 * lane, (int)(first_draw & 3), mp.count, lane);
                 });
                 change = __reduce_add_sync(kFull, change);
                 if (lane == 0 && change != 0) atomicAdd(reinterpret_cast<int *>(st + 3), change);
@@ -870,7 +906,7 @@ __global__ void __launch_bounds__(kHybrid ? kChainThreads : kChainResidentThread
             }
         }
         if (final_step && blockIdx.x == 0 && threadIdx.x < m.K) a.class_sum_tap[threadIdx.x] = s_total[threadIdx.x];
-        GTM_LAP(t_fb);
+        lap(3);
         slot = slot1;
         e2 = e3; e3 = advance(e3);
     }
@@ -888,12 +924,7 @@ __global__ void __launch_bounds__(kHybrid ? kChainThreads : kChainResidentThread
             for (int t = lane; t < (kHybrid ? W : SB * W); t += 32) dst[t] = src[t];
         }
     }
-    if (timer && threadIdx.x == 0) {
-        a.phase_cycles[0] = (unsigned long long)t_eval; a.phase_cycles[1] = (unsigned long long)t_bar;
-        a.phase_cycles[2] = (unsigned long long)t_tot; a.phase_cycles[3] = (unsigned long long)t_fb;
-        a.phase_cycles[4] = (unsigned long long)t_x0; a.phase_cycles[5] = (unsigned long long)t_x1;
-        a.phase_cycles[6] = (unsigned long long)t_x2; a.phase_cycles[7] = (unsigned long long)t_x3;
-    }
+    if (timer && lane < 8) a.phase_cycles[lane] = (unsigned long long)s_lap[lane];
 }
 
 }  // namespace gtm

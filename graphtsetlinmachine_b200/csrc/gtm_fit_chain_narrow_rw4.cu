@@ -1,0 +1,9 @@
+// fit_chain_kernel, narrow layers, transposed rows of 4 node words.
+#include "gtm_fit_chain.cuh"
+
+const void *fit_chain_kernel_narrow_rw4(bool one_layer, bool hybrid)
+{
+    using namespace gtm;
+    if (one_layer) return hybrid ? (const void *)fit_chain_kernel<4, true, true, true> : (const void *)fit_chain_kernel<4, true, false, true>;
+    return hybrid ? (const void *)fit_chain_kernel<4, false, true, true> : (const void *)fit_chain_kernel<4, false, false, true>;
+}
