@@ -118,7 +118,7 @@ static ChainPlan plan_chain(const gtm_model *m, const gtm_dataset *ds)
             a.stage_words = stage ? (std::min(ds->max_nodes * d.L0, 4096) + 3) & ~3 : 0;
             a.stage_edges = stage && D1 > 0 ? 512 : 0;
             a.clause_words = (4 + KP + rw4 + words_all * (hybrid ? 1 : d.SB) + 3) & ~3;
-            const size_t msg = D1 == 0 ? 0 : solo ? (size_t)d.D * ds->max_nodes * d.MW : (size_t)96 * rw;
+            const size_t msg = D1 == 0 ? 0 : solo ? (size_t)(d.D + 1) * ds->max_nodes * d.MW : (size_t)96 * rw;
             const size_t words = (size_t)7 * KP + 16 + (size_t)kChainStages * ((a.stage_words + 3 * a.stage_nodes + 2 * a.stage_edges + 3) & ~3) +
                                  ((msg + 3) & ~(size_t)3) + (size_t)32 * std::max(d.L0, D1 > 0 ? d.MW : 0) * rw + (size_t)kTransposedTypes * rw4 +
                                  (size_t)cpc * (kChainRec + a.pre_words + a.clause_words);

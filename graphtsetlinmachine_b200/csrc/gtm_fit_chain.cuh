@@ -112,6 +112,20 @@ __device__ __forceinline__ u32 lane_mask(const ChainArgs &a, int c, u64 block, i
     return __funnelshift_r(word, next, shift);
 }
 
+// The same for a lane whose neighbour's word is elsewhere in the stream.
+__device__ __forceinline__ u32 own_mask(const ChainArgs &a, int c, u64 block, int shift, u32 below)
+{
+    u32 word = 0, next = 0;
+#pragma unroll 1
+    for (int q = 0; q < (shift ? 9 : 8); ++q) {
+        const uint4 o = chain_draws(a, (u32)c, block + q);
+        const u32 nib = (o.x < below ? 1u : 0u) | (o.y < below ? 2u : 0u) | (o.z < below ? 4u : 0u) | (o.w < below ? 8u : 0u);
+        if (q < 8) word |= nib << (4 * q);
+        else next = nib;
+    }
+    return __funnelshift_r(word, next, shift);
+}
+
 // Rounds [q0, q1) of a clause's packed stream that starts at Philox block `block0`: words 4q .. 4q+3 of dst.
 __device__ __forceinline__ void stream_rounds(const ChainArgs &a, int c, u64 block0, int q0, int q1, u32 below, u32 *dst, int lane)
 {
@@ -133,15 +147,15 @@ __device__ __forceinline__ int nth_set_bit(u32 word, int rank, int lane)
     return __ffs(__ballot_sync(kFull, ((word >> lane) & 1u) != 0 && __popc(word & ((1u << lane) - 1u)) == rank)) - 1;
 }
 
-// Automata of 32 words of one layer of one clause, all classes in order (kernels.py:98-183): planes 0..SB-2 at lo[b * W],
-// the include plane at inc[w].  `masks(rank)` gives the lane's mask word of the Type-I class of that rank.  Returns the
+// Automata of up to 32 words of one clause, a word per lane that has one (`mine`; w, W, lo and inc belong to the word's layer
+// and may differ from lane to lane), all classes in order (kernels.py:98-183): planes 0..SB-2 at lo[b * W + w], the include
+// plane at inc[w].  `masks(rank)` gives the lane's mask word of the Type-I class of that rank.  Returns the
 // change of the lane's include count (bits of `valid`).
 template <class Masks>
-__device__ __forceinline__ int update_words(int boost, int w, int W, u32 *lo, u32 *inc, u32 x, int upd, bool clause_true, bool within,
+__device__ __forceinline__ int update_words(int boost, int w, int W, bool mine, u32 *lo, u32 *inc, u32 x, int upd, bool clause_true, bool within,
                                             u32 valid, Masks masks)
 {
     constexpr int SB = kChainStateBits;
-    const bool mine = w < W;
     u32 pl[SB - 1];
 #pragma unroll
     for (int b = 0; b < SB - 1; ++b) pl[b] = mine ? lo[(size_t)b * W + w] : 0u;
@@ -394,26 +408,34 @@ __device__ __forceinline__ void pull_messages(const ChainArgs &a, const DevModel
     }
 }
 
-// One CTA with the whole model: message rows in shared memory, node-major.  `src` holds the clauses' marks on the source
-// nodes (complete: call after a CTA barrier) and is left cleared; rows [v][MW] are made in `out`.
-__device__ __forceinline__ void solo_messages(const DevModel &m, const GraphView &gv, u32 *src, u32 *out)
+// One CTA with the whole model: message rows [v][MW] in shared memory, node-major, from the clauses' marks on the source
+// nodes `src` (complete: call after a CTA barrier; the rows are complete on return).  Graphs of a few nodes: a thread per row
+// word looks through all edges, so that nothing is cleared first and nothing merged - a barrier instead of three.
+__device__ __forceinline__ void solo_messages(const DevModel &m, const GraphView &gv, const u32 *src, u32 *out)
 {
     const int n = gv.n, MW = m.MW;
-    for (int i = threadIdx.x; i < n * MW; i += blockDim.x) out[i] = 0;
-    __syncthreads();
+    const bool gather = n <= kChainRowWise;
+    if (!gather) {
+        for (int i = threadIdx.x; i < n * MW; i += blockDim.x) out[i] = 0;
+        __syncthreads();
+    }
     for (int i = threadIdx.x; i < n * MW; i += blockDim.x) {
-        const int u = i / MW, w = i - u * MW;
-        const u32 *row = src + u * MW;
-        const u32 e0 = gv.eidx[u] - gv.e_off, deg = gv.degree[u];
-        for (u32 k = 0; k < deg && e0 + k < gv.e_cnt; ++k) {
-            const u32 dst = gv.edge[2 * (size_t)(e0 + k)], ty = gv.edge[2 * (size_t)(e0 + k) + 1];
-            if (dst >= (u32)n) continue;
-            const u32 v = rotated_word(row, w, ty >= (u32)m.MS ? ty % (u32)m.MS : ty, m.MS, MW);
-            if (v) atomicOr(out + dst * MW + w, v);
+        const int v0 = i / MW, w = i - v0 * MW;
+        u32 acc = 0;
+        for (int u = gather ? 0 : v0; u < (gather ? n : v0 + 1); ++u) {
+            const u32 *row = src + u * MW;
+            const u32 e0 = gv.eidx[u] - gv.e_off, deg = gv.degree[u];
+            for (u32 k = 0; k < deg && e0 + k < gv.e_cnt; ++k) {
+                const u32 dst = gv.edge[2 * (size_t)(e0 + k)], ty = gv.edge[2 * (size_t)(e0 + k) + 1];
+                if (gather ? dst != (u32)v0 : dst >= (u32)n) continue;       // malformed edges are ignored
+                const u32 v = rotated_word(row, w, ty >= (u32)m.MS ? ty % (u32)m.MS : ty, m.MS, MW);
+                if (gather) acc |= v;
+                else if (v) atomicOr(out + dst * MW + w, v);
+            }
         }
+        if (gather) out[i] = acc;
     }
     __syncthreads();
-    for (int i = threadIdx.x; i < n * MW; i += blockDim.x) src[i] = 0;
 }
 
 // ------------------------------------------------------------------------------------------------ the kernel
@@ -441,8 +463,8 @@ __global__ void __launch_bounds__(chain_threads(kHybrid, kNarrow), 1) fit_chain_
     u32 *s_stage = reinterpret_cast<u32 *>(s_size + 16);
     const int stage_total = (a.stage_words + 3 * a.stage_nodes + 2 * a.stage_edges + 3) & ~3;
     u32 *s_msg = s_stage + kChainStages * stage_total;
-    // message scratch: solo [n][MW] marks, [D-1][n][MW] rows; else window rows [32][RW], window words and destinations [32*RW] each
-    const int msg_words = kOneLayer ? 0 : solo ? m.D * a.max_nodes * m.MW : 96 * RW;
+    // message scratch: solo [n][MW] marks, [D-1][n][MW] rows, [n][MW] marks; else window rows [32][RW], window words and destinations [32*RW] each
+    const int msg_words = kOneLayer ? 0 : solo ? (m.D + 1) * a.max_nodes * m.MW : 96 * RW;
     u32 *s_T = s_msg + ((msg_words + 3) & ~3);
     const int t_rows = 32 * max(m.L0, kOneLayer ? 0 : m.MW);
     u32 *s_types = s_T + (size_t)t_rows * RW;
@@ -464,6 +486,19 @@ __global__ void __launch_bounds__(chain_threads(kHybrid, kNarrow), 1) fit_chain_
     auto include = [&](int i, int l) -> u32 * {
         if (kHybrid) return nodes(i) + max(RW, 4) + (l == 0 ? 0 : m.L0 + (l - 1) * m.M);
         return planes(i, l) + (SB - 1) * layer_words(l);
+    };
+    // solo: the clauses mark one buffer while the other, which the last messages were made from, is cleared
+    int turn = 0;
+    auto marks = [&](int t) { return s_msg + (size_t)(t ? m.D : 0) * a.max_nodes * m.MW; };
+    auto mark = [&](int i, int n) {
+        u32 *to = marks(turn);
+        for (int j = 0; j < (n + 31) >> 5; ++j)
+            if ((nodes(i)[j] >> lane) & 1u)
+                for (int b = 0; b < m.MB; ++b) {
+                    u32 bit = __ldg(m.hv + (size_t)(c_lo + i) * m.MB + b);
+                    if (bit >= (u32)m.MS) bit %= (u32)m.MS;
+                    atomicOr(to + (32 * j + lane) * m.MW + (bit >> 5), 1u << (bit & 31));
+                }
     };
     auto layer_mask = [&](int l) { return l == 0 ? m.lit_mask : m.msg_mask; };
 
@@ -557,12 +592,7 @@ __global__ void __launch_bounds__(chain_threads(kHybrid, kNarrow), 1) fit_chain_
             if (lane < RW) a.node_bits[(size_t)(c_lo + i) * RW + lane] = nodes(i)[lane];
         } else if (any) {
             __syncwarp();
-            for (int j = 0; j < (gv.n + 31) >> 5; ++j)
-                if ((nodes(i)[j] >> lane) & 1u)
-                    for (int b = 0; b < m.MB; ++b) {
-                        const u32 bit = __ldg(m.hv + (size_t)(c_lo + i) * m.MB + b) % (u32)m.MS;
-                        atomicOr(s_msg + (32 * j + lane) * m.MW + (bit >> 5), 1u << (bit & 31));
-                    }
+            mark(i, gv.n);
         }
     };
 
@@ -570,7 +600,7 @@ __global__ void __launch_bounds__(chain_threads(kHybrid, kNarrow), 1) fit_chain_
     if (threadIdx.x < kMaxDepth) s_prob[threadIdx.x] = mask_prob(m_in.p_mask[threadIdx.x]);
     if (threadIdx.x == 0) { s_abort = 0; s_items = 0; s_next_item = 0; }
     if (threadIdx.x < m.K) s_sum[threadIdx.x] = 0;
-    if (!kOneLayer && solo) for (int i = threadIdx.x; i < a.max_nodes * m.MW; i += blockDim.x) s_msg[i] = 0;
+    if (!kOneLayer && solo) for (int i = threadIdx.x; i < a.max_nodes * m.MW; i += blockDim.x) marks(0)[i] = marks(1)[i] = 0;
     for (int i = warp; i < mine; i += nwarps) {
         const int c = c_lo + i;
         u32 *st = state(i);
@@ -633,9 +663,11 @@ __global__ void __launch_bounds__(chain_threads(kHybrid, kNarrow), 1) fit_chain_
             if (solo) {
                 rows_n = s_msg + (size_t)d * a.max_nodes * m.MW;
                 __syncthreads();
-                solo_messages(m, gv, s_msg, rows_n);
-                if (!row_wise(gv.n)) transpose_rows<RW>(rows_n, gv.n, m.MW, s_T);
-                __syncthreads();
+                u32 *sent = marks(turn);
+                solo_messages(m, gv, sent, rows_n);
+                if (!row_wise(gv.n)) { transpose_rows<RW>(rows_n, gv.n, m.MW, s_T); __syncthreads(); }
+                turn ^= 1;
+                for (int i = threadIdx.x; i < gv.n * m.MW; i += blockDim.x) sent[i] = 0;
                 lap(5);
             } else {
                 if (!barrier(++nb)) return;
@@ -668,12 +700,7 @@ __global__ void __launch_bounds__(chain_threads(kHybrid, kNarrow), 1) fit_chain_
                     if (lane < RW) bits[(size_t)m.C * RW + (size_t)(c_lo + i) * RW + lane] = nodes(i)[lane];
                 } else if (any) {
                     __syncwarp();
-                    for (int j = 0; j < (gv.n + 31) >> 5; ++j)
-                        if ((nodes(i)[j] >> lane) & 1u)
-                            for (int b = 0; b < m.MB; ++b) {
-                                const u32 bit = __ldg(m.hv + (size_t)(c_lo + i) * m.MB + b) % (u32)m.MS;
-                                atomicOr(s_msg + (32 * j + lane) * m.MW + (bit >> 5), 1u << (bit & 31));
-                            }
+                    mark(i, gv.n);
                 }
             }
         }
@@ -822,29 +849,29 @@ __global__ void __launch_bounds__(chain_threads(kHybrid, kNarrow), 1) fit_chain_
                     if (npos > 0 && packed) stream_rounds(a, c, block0, a.spec_rounds, rounds, s_prob[0].count, pre, lane);
                     __syncwarp();
                     const bool within = (int)st[2] <= m.max_included;
-                    int change = 0, first_word = 0;                     // first_word: stream words of the layers before
-                    for (int l = 0; l < m.D; ++l) {
-                        const int W = layer_words(l);
+                    int change = 0;
+                    // the words of all layers, 32 at a time
+                    for (int f0 = 0; f0 < words_all; f0 += 32) {
+                        int l = 0, w = f0 + lane, W = m.L0;
+                        if (!kOneLayer) while (w >= W && l < m.D - 1) { w -= W; W = m.M; ++l; }
+                        const int before = f0 + lane - w;                    // words of the layers before
+                        const bool in_layer = w < W;
+                        if (!in_layer) w = 0;
                         u32 x = 0;
-                        if (clause_true && lane < W) {
-                            if (l == 0) x = gv.X[(size_t)chosen * m.L0 + lane];
-                            else if (solo) x = msg_word(s_msg + ((size_t)l * a.max_nodes + chosen) * m.MW, lane, m.MS, m.MW);
-                            else x = msg_word(a.rows_n + ((size_t)(l - 1) * a.max_nodes + chosen) * m.MW, lane, m.MS, m.MW);
+                        if (clause_true && in_layer) {
+                            if (l == 0) x = gv.X[(size_t)chosen * m.L0 + w];
+                            else if (solo) x = msg_word(s_msg + ((size_t)l * a.max_nodes + chosen) * m.MW, w, m.MS, m.MW);
+                            else x = msg_word(a.rows_n + ((size_t)(l - 1) * a.max_nodes + chosen) * m.MW, w, m.MS, m.MW);
                         }
-                        const u32 valid = lane == W - 1 ? layer_mask(l) : kFull;
-                        const int base = first_word;
-                        change += update_words(m.boost, lane, W, planes(i, l), include(i, l), x, upd_all, clause_true, within, valid, [&](int rank) {
-                            if (all_ones) return kFull;
-                            const int bit = off0 + 32 * (base + rank * W + lane);
-                            if (packed) {
-                                if (lane >= W) return 0u;
-                                return __funnelshift_r(pre[bit >> 5], pre[(bit >> 5) + 1], bit & 31);
-                            }
+                        const u32 valid = w == W - 1 ? layer_mask(l) : kFull;
+                        change += update_words(m.boost, w, W, in_layer, planes(i, l), include(i, l), x, upd_all, clause_true, within, valid, [&](int rank) {
+                            if (all_ones || !in_layer) return kFull;
+                            const int bit = off0 + 32 * (npos * before + rank * W + w);
+                            if (packed) return __funnelshift_r(pre[bit >> 5], pre[(bit >> 5) + 1], bit & 31);
                             // more Type-I classes than the buffer holds: the lane makes its own word
-                            const u64 first_draw = pos + (u64)32 * (u64)(base + rank * W);
-                            return lane_mask(a, c, (first_draw >> 2) + (u64)8 * lane, (int)(first_draw & 3), s_prob[0].count, lane);
+                            const u64 first_draw = 4 * block0 + (u64)(u32)bit;
+                            return own_mask(a, c, first_draw >> 2, (int)(first_draw & 3), s_prob[0].count);
                         });
-                        first_word += npos * W;
                     }
                     change = __reduce_add_sync(kFull, change);
                     if (lane == 0) st[2] += (u32)change;
@@ -887,7 +914,7 @@ __global__ void __launch_bounds__(chain_threads(kHybrid, kNarrow), 1) fit_chain_
                     else x = msg_word(a.rows_n + ((size_t)(l - 1) * a.max_nodes + chosen) * m.MW, w, m.MS, m.MW);
                 }
                 const MaskProb mp = s_prob[l];
-                int change = update_words(m.boost, w, W, planes(i, l), include(i, l), x, upd, clause_true, (int)st[2] <= m.max_included,
+                int change = update_words(m.boost, w, W, w < W, planes(i, l), include(i, l), x, upd, clause_true, (int)st[2] <= m.max_included,
                                           w == W - 1 ? layer_mask(l) : kFull, [&](int rank) {
                     if (mp.p >= 1.0f) return kFull;
                     const u64 first_draw = layer_pos + (u64)32 * (u64)(rank * W + g0);
