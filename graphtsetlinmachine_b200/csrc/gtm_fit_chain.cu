@@ -41,11 +41,16 @@ static int chain_prepare(gtm_model *m, gtm_dataset *ds, int rw)
     if (!m->chain_sync) GTM_TRY(dev_alloc(&m->chain_sync, (size_t)2 * d.K + 1));
     if (d.D == 1) return GTM_OK;
     if (!m->hv_lists_valid) {
-        std::vector<int> off((size_t)d.MS + 1, 0), list((size_t)d.C * d.MB);
+        std::vector<int> off((size_t)d.MS + 1, 0), list((size_t)2 * d.C * d.MB);
         for (u32 h : m->hv_host) ++off[h % (u32)d.MS + 1];
         for (int b = 0; b < d.MS; ++b) off[(size_t)b + 1] += off[(size_t)b];
         std::vector<int> at(off.begin(), off.end() - 1);
-        for (size_t i = 0; i < m->hv_host.size(); ++i) list[(size_t)at[m->hv_host[i] % (u32)d.MS]++] = (int)(i / (size_t)d.MB);
+        for (size_t i = 0; i < m->hv_host.size(); ++i) {
+            const int bit = (int)(m->hv_host[i] % (u32)d.MS);
+            const size_t entry = (size_t)at[(size_t)bit]++;
+            list[2 * entry] = (int)(i / (size_t)d.MB);
+            list[2 * entry + 1] = bit;
+        }
         if (!m->hv_off) {
             GTM_TRY(dev_alloc(&m->hv_off, off.size()));
             GTM_TRY(dev_alloc(&m->hv_clause, list.size()));
@@ -110,10 +115,15 @@ static ChainPlan plan_chain(const gtm_model *m, const gtm_dataset *ds)
         const int grid = (d.C + cpc - 1) / cpc;
         const bool solo = grid == 1;
         if (grid > m->sm_count) return plan;
-        const int want_warps = a.narrow ? std::max(8, cpc) : 32;
+        const int want_warps = a.narrow ? std::max(D1 > 0 && !solo ? 16 : 8, cpc) : 32;
         for (int variant = 0; variant < 4; ++variant) {        // planes resident, then include planes only; with and without staged graphs
             const bool hybrid = variant >= 2, stage = (variant & 1) == 0;
-            const int warps = std::min(want_warps, chain_threads(hybrid, a.narrow != 0) / 32);
+            const int most = chain_threads(hybrid, a.narrow != 0) / 32;
+            // Graphs that are tested as they are: a warp without clauses stages them and exchanges the votes (4,000 images x 2,500
+            // clauses 24.1 -> 21.6 ms, 10,000 Noisy-XOR graphs 55.8 -> 54.2).  Transposing a graph of 90 nodes took that warp longer
+            // than the exchange (700 graphs 15.6 -> 16.0 ms).
+            a.helper = a.narrow && want_warps < most && ds->max_nodes <= kChainRowWise;
+            const int warps = std::min(want_warps + a.helper, most);
             a.stage_nodes = stage ? std::min(ds->max_nodes, 512) : 0;
             a.stage_words = stage ? (std::min(ds->max_nodes * d.L0, 4096) + 3) & ~3 : 0;
             a.stage_edges = stage && D1 > 0 ? 512 : 0;
@@ -157,7 +167,7 @@ int launch_fit_chain(gtm_model *m, gtm_dataset *ds, int n_types, const int *Y_de
     a.wait_ns = (unsigned long long)m->opt_fit_wait_ms * 1000000ull;
     a.missing = m->opt_fit_missing_cta;
     a.node_bits = ds->chain_bits; a.rows_t = ds->chain_rows_t; a.rows_n = ds->chain_rows_n;
-    a.bit_off = m->hv_off; a.bit_clause = m->hv_clause; a.tmax = std::max(0, ds->largest_edge_type);
+    a.bit_off = m->hv_off; a.bit_clause = reinterpret_cast<const int2 *>(m->hv_clause); a.tmax = std::max(0, ds->largest_edge_type);
     for (int r = 0; r < 10; ++r) {
         a.key[2 * r] = d.seed_lo + (u32)r * 0x9E3779B9u;
         a.key[2 * r + 1] = d.seed_hi + (u32)r * 0xBB67AE85u;

@@ -21,6 +21,11 @@
 //   (the positions of these draws do not depend on the class sums), and the transposition of the next graph.
 //   Feedback and the next graph's first layer are one pass: a clause's warp decides, updates and evaluates.
 //
+// What bounds it: instructions of few warps.  One epoch and the way back of the state on one B200, ms, here / in
+// fit_resident_kernel or fit_kernel: 10,000 Noisy-XOR graphs (one CTA) 57 / 109; 4,000 images x 2,500 clauses 22 / 44; 200
+// sequences of 1,000 nodes 8.1 / 26.7; 300 multigraphs x 20,000 clauses 51 / 160, 36 of them in the kernel, half of that for the
+// Philox draws and the automata of some 95 clauses per CTA and graph.
+//
 // State: automaton planes in shared memory while they fit; otherwise (kHybrid) only the include planes, which the
 // evaluation reads, and the other planes are read and written in global memory for the clauses that get feedback.
 #pragma once
@@ -54,6 +59,7 @@ struct ChainArgs {
     unsigned long long wait_ns;
     int missing;                 // test hook: waits expect this many arrivals more than there are CTAs
     int clauses_per_cta, clause_words;
+    int helper;                  // the last warp has no clauses: it stages graphs and exchanges votes
     int solo;                    // one CTA: its barriers replace the grid's, messages stay in shared memory
     int narrow;                  // kNarrow: a clause's masks come from one packed stream (all layers of one probability, up to 32 words)
     int pre_words, spec_rounds;  // narrow: words of that stream kept per clause; rounds made in the exchange's shadow
@@ -62,7 +68,8 @@ struct ChainArgs {
     u32 *node_bits;              // [D-1][C][RW] node words of every clause after each layer but the last
     u32 *rows_t;                 // [D-1][32*MW][RW] message rows, transposed
     u32 *rows_n;                 // [D-1][max_nodes][MW] message rows, node-major
-    const int *bit_off, *bit_clause;                 // clauses whose hypervector holds message bit b: bit_clause[bit_off[b] ..]
+    const int *bit_off;          // clauses whose hypervector holds message bit b: bit_clause[bit_off[b] ..]
+    const int2 *bit_clause;      // (clause, b)
     int tmax;                    // largest edge type
     u32 key[20];                 // Philox round keys: operands in the constant bank instead of two additions a round
 };
@@ -321,13 +328,13 @@ __device__ __forceinline__ bool eval_clause_rowwise(const u32 *inc, int W, u32 l
     return r != 0;
 }
 
-// Rows [v][0..W) of n nodes -> T, all threads of the CTA: a thread takes 32 nodes x 32 literals; the 32 lanes of a warp take
+// Rows [v][0..W) of n nodes -> T, by `threads` threads (whole warps): a thread takes 32 nodes x 32 literals; the 32 lanes of a warp take
 // 8 words x 4 node words, which keeps reads in 32-byte sectors and the bank conflicts of the stores at eight.
 template <int RW>
-__device__ __forceinline__ void transpose_rows(const u32 *rows, int n, int W, u32 *T)
+__device__ __forceinline__ void transpose_rows(const u32 *rows, int n, int W, u32 *T, int thread, int threads)
 {
     const int nw = (n + 31) >> 5, wb = (W + 7) >> 3, jb = (nw + 3) >> 2;
-    for (int i = threadIdx.x; i < wb * jb * 32; i += blockDim.x) {
+    for (int i = thread; i < wb * jb * 32; i += threads) {
         const int b8 = i >> 5, w = (b8 % wb) * 8 + (i & 7), j = (b8 / wb) * 4 + ((i >> 3) & 3);
         if (w >= W || j >= nw) continue;
         u32 r[32];
@@ -354,24 +361,40 @@ __device__ __forceinline__ void pull_messages(const ChainArgs &a, const DevModel
     const int nw = (gv.n + 31) >> 5, units = (m.MS + 7) >> 3;
     for (int unit = blockIdx.x; unit < units; unit += gridDim.x) {
         const int b0 = 8 * unit, nb = min(8, m.MS - b0), win = nb + a.tmax;
-        // (1) node words of the window's bits b0 - tmax .. b0 + nb - 1
-        for (int i = warp; i < win; i += nwarps) {
-            int bit = (b0 - a.tmax + i) % m.MS;
-            if (bit < 0) bit += m.MS;
-            const int lo = __ldg(a.bit_off + bit), hi = __ldg(a.bit_off + bit + 1);
-            u32 acc = 0;
-            const int j = lane % RW;
-            for (int s = lo + lane / RW; s < hi; s += 32 / RW)
-                if (j < nw) acc |= __ldcg(node_bits + (size_t)__ldg(a.bit_clause + s) * RW + j);
-            __syncwarp();
+        // (1) node words of the window's bits b0 - tmax .. b0 + nb - 1.  Their clauses are one stretch of the list, or several
+        //     where the bits wrap around; groups of RW lanes take entries of it, four loads of node words in flight each.
+        for (int i = threadIdx.x; i < win * RW; i += blockDim.x) s_row[i] = 0;
+        __syncthreads();
+        const int j = lane % RW, group = warp * (32 / RW) + lane / RW, groups = nwarps * (32 / RW);
+        const int start = (((b0 - a.tmax) % m.MS) + m.MS) % m.MS;       // bit of window row 0
+        for (int row0 = 0; row0 < win;) {
+            const int bit0 = (start + row0) % m.MS, rows = min(win - row0, m.MS - bit0);
+            const int lo = __ldg(a.bit_off + bit0), hi = __ldg(a.bit_off + bit0 + rows);
+            for (int s0 = lo + group; s0 < hi; s0 += 4 * groups) {
+                u32 word[4];
+                int row[4];
 #pragma unroll
-            for (int d = RW; d < 32; d <<= 1) acc |= __shfl_xor_sync(kFull, acc, d);
-            if (lane < RW) s_row[i * RW + lane] = acc;
+                for (int t = 0; t < 4; ++t) {
+                    const int s = s0 + t * groups;
+                    word[t] = 0;
+                    row[t] = 0;
+                    if (s < hi) {
+                        const int2 entry = __ldg(a.bit_clause + s);     // clause, bit
+                        row[t] = row0 + entry.y - bit0;
+                        if (j < nw) word[t] = __ldcg(node_bits + (size_t)entry.x * RW + j);
+                    }
+                }
+#pragma unroll
+                for (int t = 0; t < 4; ++t)
+                    if (word[t]) atomicOr(s_row + row[t] * RW + j, word[t]);
+            }
+            row0 += rows;
         }
         __syncthreads();
         // (2) the window of every source node as one word
         for (int j = warp; j < nw; j += nwarps) {
             u32 s = 0;
+#pragma unroll 4
             for (int i = 0; i < win; ++i) s |= ((s_row[i * RW + j] >> lane) & 1u) << i;
             s_win[32 * j + lane] = s;
             s_dst[32 * j + lane] = 0;
@@ -470,7 +493,10 @@ __global__ void __launch_bounds__(chain_threads(kHybrid, kNarrow), 1) fit_chain_
     u32 *s_types = s_T + (size_t)t_rows * RW;
     u32 *s_clause = s_types + kTransposedTypes * max(RW, 4);
     const int per_clause = kChainRec + a.pre_words + a.clause_words;
+    const int clause_warps = nwarps - a.helper, vote_warp = a.helper ? clause_warps : 0;
+    const int stage_thread = a.helper ? (int)threadIdx.x - 32 * clause_warps : (int)threadIdx.x, stage_threads = a.helper ? 32 : (int)blockDim.x;
     const int c_lo = min(m.C, (int)blockIdx.x * a.clauses_per_cta), c_hi = min(m.C, c_lo + a.clauses_per_cta), mine = c_hi - c_lo;
+    const int clause0 = warp < clause_warps ? warp : mine;               // first of the warp's clauses
 
     auto record = [&](int i) { return reinterpret_cast<int *>(s_clause + (size_t)i * per_clause); };
     auto stream = [&](int i) { return s_clause + (size_t)i * per_clause + kChainRec; };
@@ -507,20 +533,20 @@ __global__ void __launch_bounds__(chain_threads(kHybrid, kNarrow), 1) fit_chain_
     auto advance = [&](int64_t e) { return e + 1 < a.first + a.count ? e + 1 : a.first; };
     auto fits = [&](const int *sz) { return sz[0] <= a.stage_nodes && sz[0] * m.L0 <= a.stage_words && (kOneLayer || sz[3] <= a.stage_edges); };
     auto fetch_sizes = [&](u64 st, int64_t e) {
-        if (threadIdx.x < 4 && st < steps) {
-            const u32 *src = threadIdx.x == 0 ? g.n_nodes : threadIdx.x == 1 ? g.node_index : threadIdx.x == 2 ? g.graph_edge0 : g.graph_edges;
-            async_copy_word(reinterpret_cast<u32 *>(s_size + (int)(st & 3) * 4 + threadIdx.x), src + e);
+        if (stage_thread >= 0 && stage_thread < 4 && st < steps) {
+            const u32 *src = stage_thread == 0 ? g.n_nodes : stage_thread == 1 ? g.node_index : stage_thread == 2 ? g.graph_edge0 : g.graph_edges;
+            async_copy_word(reinterpret_cast<u32 *>(s_size + (int)(st & 3) * 4 + stage_thread), src + e);
         }
     };
     auto fetch_graph = [&](u64 st, int64_t e, int slot) {               // sizes of step st are there
-        if (st >= steps) return;
-        if (threadIdx.x < m.K) async_copy_word(reinterpret_cast<u32 *>(s_y + slot * KP + threadIdx.x), reinterpret_cast<const u32 *>(a.Y + (size_t)e * m.K + threadIdx.x));
+        if (st >= steps || stage_thread < 0) return;
+        if (stage_thread < m.K) async_copy_word(reinterpret_cast<u32 *>(s_y + slot * KP + stage_thread), reinterpret_cast<const u32 *>(a.Y + (size_t)e * m.K + stage_thread));
         const int *sz = s_size + (int)(st & 3) * 4;
         if (!fits(sz)) return;
         const int n = sz[0], base = sz[1], e0 = sz[2], ne = sz[3];
         u32 *x = s_stage + slot * stage_total, *t = x + a.stage_words;
-        for (int i = threadIdx.x; i < n * m.L0; i += blockDim.x) async_copy_word(x + i, g.X + (size_t)base * m.L0 + i);
-        for (int i = threadIdx.x; i < n; i += blockDim.x) {
+        for (int i = stage_thread; i < n * m.L0; i += stage_threads) async_copy_word(x + i, g.X + (size_t)base * m.L0 + i);
+        for (int i = stage_thread; i < n; i += stage_threads) {
             async_copy_word(t + i, g.node_type + base + i);
             if (!kOneLayer) {
                 async_copy_word(t + a.stage_nodes + i, g.degree + base + i);
@@ -528,7 +554,7 @@ __global__ void __launch_bounds__(chain_threads(kHybrid, kNarrow), 1) fit_chain_
             }
         }
         if (!kOneLayer)
-            for (int i = threadIdx.x; i < 2 * ne; i += blockDim.x) async_copy_word(t + 3 * a.stage_nodes + i, g.edge + 2 * (size_t)e0 + i);
+            for (int i = stage_thread; i < 2 * ne; i += stage_threads) async_copy_word(t + 3 * a.stage_nodes + i, g.edge + 2 * (size_t)e0 + i);
     };
     auto wait_copies = [&]() { asm volatile("cp.async.wait_all;" ::: "memory"); };
     auto view_of = [&](u64 st, int slot) {
@@ -549,7 +575,8 @@ __global__ void __launch_bounds__(chain_threads(kHybrid, kNarrow), 1) fit_chain_
     auto row_wise = [&](int n) { return RW == 1 && n <= kChainRowWise; };
     // transposed rows of the first layer and type rows of a graph
     auto prepare_graph = [&](const GraphView &gv) {
-        for (int j = warp; j < (RW == 1 ? 1 : RW); j += nwarps) {
+        if (stage_thread < 0) return;
+        for (int j = stage_thread >> 5; j < (RW == 1 ? 1 : RW); j += stage_threads >> 5) {
             const int v = 32 * j + lane;
             const u32 ty = v < gv.n ? gv.type[v] : ~0u;
             for (int t = 0; t < g.n_types; ++t) {
@@ -557,7 +584,7 @@ __global__ void __launch_bounds__(chain_threads(kHybrid, kNarrow), 1) fit_chain_
                 if (lane == 0) s_types[t * RW + j] = col;
             }
         }
-        if (!row_wise(gv.n)) transpose_rows<RW>(gv.X, gv.n, m.L0, s_T);
+        if (!row_wise(gv.n)) transpose_rows<RW>(gv.X, gv.n, m.L0, s_T, stage_thread, stage_threads);
     };
 
     // ---- waits ----
@@ -601,7 +628,7 @@ __global__ void __launch_bounds__(chain_threads(kHybrid, kNarrow), 1) fit_chain_
     if (threadIdx.x == 0) { s_abort = 0; s_items = 0; s_next_item = 0; }
     if (threadIdx.x < m.K) s_sum[threadIdx.x] = 0;
     if (!kOneLayer && solo) for (int i = threadIdx.x; i < a.max_nodes * m.MW; i += blockDim.x) marks(0)[i] = marks(1)[i] = 0;
-    for (int i = warp; i < mine; i += nwarps) {
+    for (int i = clause0; i < mine; i += clause_warps) {
         const int c = c_lo + i;
         u32 *st = state(i);
         if (lane == 0) { *reinterpret_cast<u64 *>(st) = m.draw_pos[c]; st[3] = 0; }
@@ -632,9 +659,9 @@ __global__ void __launch_bounds__(chain_threads(kHybrid, kNarrow), 1) fit_chain_
     __syncthreads();
     {
         const GraphView gv = view_of(0, 0);
-        for (int i = warp; i < mine; i += nwarps) first_layer(i, gv);
+        for (int i = clause0; i < mine; i += clause_warps) first_layer(i, gv);
     }
-    // accumulators only grow: what this CTA read last from each of the two sets (lane k of warp 0)
+    // accumulators only grow: what this CTA read last from each of the two sets (lane k of the voting warp)
     unsigned long long seen_votes[2] = {0, 0};
     unsigned nb = 0;
     const bool timer = a.timers != 0 && blockIdx.x == 0 && threadIdx.x < 32;
@@ -650,10 +677,10 @@ __global__ void __launch_bounds__(chain_threads(kHybrid, kNarrow), 1) fit_chain_
         }
     };
 
+    GraphView gv = view_of(0, 0);                                       // the current graph
     int slot = 0;                                                       // staging slot of the current graph
     for (u64 step = 0; step < steps; ++step) {
         const int slot1 = slot == 2 ? 0 : slot + 1, slot2 = slot1 == 2 ? 0 : slot1 + 1;
-        const GraphView gv = view_of(step, slot);
         wait_copies();                                                  // issued a step ago; seen by all after the next barrier
         // ---- message layers ----
         for (int d = 1; d < m.D; ++d) {
@@ -665,7 +692,7 @@ __global__ void __launch_bounds__(chain_threads(kHybrid, kNarrow), 1) fit_chain_
                 __syncthreads();
                 u32 *sent = marks(turn);
                 solo_messages(m, gv, sent, rows_n);
-                if (!row_wise(gv.n)) { transpose_rows<RW>(rows_n, gv.n, m.MW, s_T); __syncthreads(); }
+                if (!row_wise(gv.n)) { transpose_rows<RW>(rows_n, gv.n, m.MW, s_T, threadIdx.x, blockDim.x); __syncthreads(); }
                 turn ^= 1;
                 for (int i = threadIdx.x; i < gv.n * m.MW; i += blockDim.x) sent[i] = 0;
                 lap(5);
@@ -686,7 +713,7 @@ __global__ void __launch_bounds__(chain_threads(kHybrid, kNarrow), 1) fit_chain_
                 lap(5);
             }
             const bool last = d == m.D - 1;
-            for (int i = warp; i < mine; i += nwarps) {
+            for (int i = clause0; i < mine; i += clause_warps) {
                 const int ct = (c_lo + i) % g.n_types;
                 const u32 *inc = include(i, d);
                 bool any;
@@ -711,7 +738,7 @@ __global__ void __launch_bounds__(chain_threads(kHybrid, kNarrow), 1) fit_chain_
         lap(0);
         const int *y = s_y + slot * KP;
         const int set = (int)(step & 1);
-        if (warp == 0 && lane < m.K) {
+        if (warp == vote_warp && lane < m.K) {
             const int sum = s_sum[lane];
             s_sum[lane] = 0;
             if (solo) {
@@ -726,7 +753,7 @@ __global__ void __launch_bounds__(chain_threads(kHybrid, kNarrow), 1) fit_chain_
         // ---- in the shadow of the exchange: the graph after next, what decisions need besides the class sums, the next graph ----
         fetch_sizes(step + 3, e3);
         fetch_graph(step + 2, e2, slot2);
-        for (int i = warp; i < mine; i += nwarps) {
+        for (int i = clause0; i < mine; i += clause_warps) {
             const int c = c_lo + i;
             int *rec = record(i);
             const u32 *nd = nodes(i);
@@ -762,7 +789,7 @@ __global__ void __launch_bounds__(chain_threads(kHybrid, kNarrow), 1) fit_chain_
         if (more) prepare_graph(gn);
         lap(6);
         // ---- votes in ----
-        if (!solo && warp == 0) {
+        if (!solo && warp == vote_warp) {
             bool gave_up = false;
             if (lane < m.K) {
                 const unsigned long long want = (unsigned long long)gridDim.x + (unsigned long long)a.missing;
@@ -786,7 +813,7 @@ __global__ void __launch_bounds__(chain_threads(kHybrid, kNarrow), 1) fit_chain_
         lap(2);
         // ---- feedback and the next graph's first layer ----
         const bool final_step = !more;
-        for (int i = warp; i < mine; i += nwarps) {
+        for (int i = clause0; i < mine; i += clause_warps) {
             const int c = c_lo + i;
             int *rec = record(i);
             u32 *st = state(i);
@@ -925,7 +952,7 @@ __global__ void __launch_bounds__(chain_threads(kHybrid, kNarrow), 1) fit_chain_
             }
             __syncthreads();
             if (threadIdx.x == 0) { s_items = 0; s_next_item = 0; }
-            for (int i = warp; i < mine; i += nwarps) {
+            for (int i = clause0; i < mine; i += clause_warps) {
                 u32 *st = state(i);
                 if (lane == 0) { st[2] += st[3]; st[3] = 0; }
                 __syncwarp();
@@ -935,11 +962,12 @@ __global__ void __launch_bounds__(chain_threads(kHybrid, kNarrow), 1) fit_chain_
         if (final_step && blockIdx.x == 0 && threadIdx.x < m.K) a.class_sum_tap[threadIdx.x] = s_total[threadIdx.x];
         lap(3);
         slot = slot1;
+        gv = gn;
         e2 = e3; e3 = advance(e3);
     }
 
     // ---- state out ----
-    for (int i = warp; i < mine; i += nwarps) {
+    for (int i = clause0; i < mine; i += clause_warps) {
         const int c = c_lo + i;
         if (lane == 0) m.draw_pos[c] = *reinterpret_cast<u64 *>(state(i));
         for (int k = lane; k < m.K; k += 32) m.weights[(size_t)k * m.C + c] = weights(i)[k];
