@@ -761,9 +761,11 @@ static bool scores_by_stream(gtm_model *m, gtm_dataset *ds, int n_types)
     return (m->opt_score_kernel == 0 || m->opt_score_kernel == 2) && stream_supported(ds->sd, n_types);
 }
 
+// The option that forces the tile kernel stands for tiles of several graphs and one pass of the votes, and is an error beyond.
 static bool scores_by_tile(gtm_model *m, gtm_dataset *ds, int n_types)
 {
-    return (m->opt_score_kernel == 0 || m->opt_score_kernel == 3) && tile_supported(ds->td, n_types);
+    if (!tile_supported(ds->td, n_types)) return false;
+    return m->opt_score_kernel == 0 || (m->opt_score_kernel == 3 && !ds->td.span && m->dm.K <= 16);
 }
 
 extern "C" int gtm_score_device(gtm_model *m, gtm_dataset *ds, int n_types, int64_t first, int64_t count,
@@ -775,7 +777,7 @@ extern "C" int gtm_score_device(gtm_model *m, gtm_dataset *ds, int n_types, int6
     if (!sums_dev) return fail(GTM_ERR_ARG, "class_sums_device is null");
     if (m->opt_score_kernel == 2 && !stream_supported(ds->sd, n_types))
         return fail(GTM_ERR_ARG, "the node-stream scoring kernel does not cover this model / graph set");
-    if (m->opt_score_kernel == 3 && !tile_supported(ds->td, n_types))
+    if (m->opt_score_kernel == 3 && !scores_by_tile(m, ds, n_types))
         return fail(GTM_ERR_ARG, "the tile scoring kernel does not cover this model / graph set");
     if (scores_by_stream(m, ds, n_types)) {
         GTM_TRY(refresh_lists(m));

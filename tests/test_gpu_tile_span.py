@@ -10,7 +10,7 @@ from util import EngineTM, encode_labels, random_graphs
 pytestmark = pytest.mark.gpu
 
 
-def compare(n, seed, *, clauses, classes, hv, depth, ms, mb=2, max_nodes, node_types=2, edge_types=3, fixed=None, options=None):
+def compare(n, seed, *, clauses, classes, hv, depth, ms, mb=2, max_nodes, node_types=2, edge_types=3, fixed=None):
     rng = np.random.default_rng(seed)
     np.random.seed(seed)
     graphs = random_graphs(n, rng, hv_size=hv, hv_bits=2, max_nodes=max_nodes, node_types=node_types, edge_types=edge_types,
@@ -19,7 +19,7 @@ def compare(n, seed, *, clauses, classes, hv, depth, ms, mb=2, max_nodes, node_t
     hvs = np.stack([rng.choice(ms, size=mb, replace=False) for _ in range(clauses)]).astype(np.uint32)
     kw = dict(clauses=clauses, classes=classes, literals=2 * hv, threshold=15, s=2.0, depth=depth, message_size=ms,
               message_bits=mb, max_nodes=max_nodes, hypervectors=hvs, seed=seed)
-    cpu, gpu = OracleTM(**kw), EngineTM(**kw, options=options or {})
+    cpu, gpu = OracleTM(**kw), EngineTM(**kw)
     for tm in (cpu, gpu):
         tm.set_graphs(graphs)
         tm.prepare()
@@ -41,18 +41,18 @@ def compare(n, seed, *, clauses, classes, hv, depth, ms, mb=2, max_nodes, node_t
 
 @pytest.mark.parametrize("nodes", [129, 256, 257, 383, 512, 513, 900, 1024])
 def test_graphs_that_span_quads(engine_lib, nodes):
-    compare(5, nodes, clauses=70, classes=3, hv=40, depth=3, ms=50, max_nodes=nodes, fixed=nodes, options={"score_kernel": 3})
+    compare(5, nodes, clauses=70, classes=3, hv=40, depth=3, ms=50, max_nodes=nodes, fixed=nodes)
 
 
 @pytest.mark.parametrize("max_nodes,depth,ms", [(140, 2, 64), (300, 4, 33), (1000, 1, 32)])
 def test_ragged_sets_with_graphs_that_span_quads(engine_lib, max_nodes, depth, ms):
-    compare(9, max_nodes, clauses=333, classes=2, hv=31, depth=depth, ms=ms, max_nodes=max_nodes, node_types=3, options={"score_kernel": 3})
+    compare(9, max_nodes, clauses=333, classes=2, hv=31, depth=depth, ms=ms, max_nodes=max_nodes, node_types=3)
 
 
 @pytest.mark.parametrize("classes", [16, 17, 20, 31, 32])
 @pytest.mark.parametrize("max_nodes", [30, 200])
 def test_class_counts(engine_lib, classes, max_nodes):
-    compare(12, classes, clauses=90, classes=classes, hv=20, depth=2, ms=40, max_nodes=max_nodes, options={"score_kernel": 3})
+    compare(12, classes, clauses=90, classes=classes, hv=20, depth=2, ms=40, max_nodes=max_nodes)
 
 
 @pytest.mark.parametrize("fixed", [1, 4, None])
