@@ -10,7 +10,7 @@
 //   one to three nodes are tested row-wise, lane = include word.
 //   Messages (depth > 1) are PULLED.  Clauses publish their node words (plain stores); after a grid barrier CTA b makes
 //   the message bits 8b .. 8b+7 of every node: it ORs the node words of the clauses whose hypervectors hold a bit of the
-//   window (lists per bit, made once), walks the edges once with the window as one word per node - a rotation by the edge
+//   window (lists per bit, made once), walks the edges once, a packed word each, with the window as one word per node - a rotation by the edge
 //   type (kernels.py:581) is a shift of the window - and stores the bits both transposed, the next layer's rows as the
 //   evaluation reads them, and node-major for the feedback.  A second barrier, and every CTA copies the rows.  Nothing is
 //   merged with atomics: sending source-node marks to shared rows (fit_resident_kernel) took 40,000 cycles per layer on
@@ -46,6 +46,8 @@ constexpr int kChainRowWise = 3;         // graphs of at most this many nodes ar
 constexpr int kChainMaxType = 24;        // largest edge type of a set whose messages are pulled: the window is 8 + 24 bits
 constexpr int kChainRec = 40;            // words per clause of a step: chosen, pos (2), taken, -, -, -, -, draws / feedback [32]
 
+constexpr u32 kNoEdge = ~0u;
+
 struct ChainArgs {
     const int *Y;                // [N][K] +-T targets, absolute graph ids
     int64_t first, count;
@@ -68,6 +70,7 @@ struct ChainArgs {
     u32 *node_bits;              // [D-1][C][RW] node words of every clause after each layer but the last
     u32 *rows_t;                 // [D-1][32*MW][RW] message rows, transposed
     u32 *rows_n;                 // [D-1][max_nodes][MW] message rows, node-major
+    const u32 *packed;           // [edges] source | destination << 10 | type << 20 of every edge row; kNoEdge: malformed
     const int *bit_off;          // clauses whose hypervector holds message bit b: bit_clause[bit_off[b] ..]
     const int2 *bit_clause;      // (clause, b)
     int tmax;                    // largest edge type
@@ -354,7 +357,7 @@ __device__ __forceinline__ void transpose_rows(const u32 *rows, int n, int W, u3
 // this CTA.  All threads; the node words are complete (grid barrier); the rows are complete after another grid barrier.
 // s_row [32][RW], s_win / s_dst [32*RW]: scratch.
 template <int RW>
-__device__ __forceinline__ void pull_messages(const ChainArgs &a, const DevModel &m, const GraphView &gv, const u32 *node_bits, u32 *rows_t,
+__device__ __forceinline__ void pull_messages(const ChainArgs &a, const DevModel &m, const GraphView &gv, const u32 *packed, int edges, const u32 *node_bits, u32 *rows_t,
                                               u32 *rows_n, u32 *s_row, u32 *s_win, u32 *s_dst)
 {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
@@ -363,6 +366,12 @@ __device__ __forceinline__ void pull_messages(const ChainArgs &a, const DevModel
         const int b0 = 8 * unit, nb = min(8, m.MS - b0), win = nb + a.tmax;
         // (1) node words of the window's bits b0 - tmax .. b0 + nb - 1.  Their clauses are one stretch of the list, or several
         //     where the bits wrap around; groups of RW lanes take entries of it, four loads of node words in flight each.
+        u32 ahead[4];                                                   // the thread's first edges, on their way meanwhile
+#pragma unroll
+        for (int t = 0; t < 4; ++t) {
+            const int e = threadIdx.x + t * blockDim.x;
+            ahead[t] = e < edges ? __ldg(packed + e) : kNoEdge;
+        }
         for (int i = threadIdx.x; i < win * RW; i += blockDim.x) s_row[i] = 0;
         __syncthreads();
         const int j = lane % RW, group = warp * (32 / RW) + lane / RW, groups = nwarps * (32 / RW);
@@ -402,17 +411,14 @@ __device__ __forceinline__ void pull_messages(const ChainArgs &a, const DevModel
         __syncthreads();
         // (3) bit b of a destination is bit b - t of a source: the window shifted by the edge type
         const u32 keep = (1u << nb) - 1u;
-        for (int u = threadIdx.x; u < gv.n; u += blockDim.x) {
-            const u32 s = s_win[u];
-            if (s == 0) continue;
-            const u32 e0 = gv.eidx[u] - gv.e_off, deg = gv.degree[u];
-            for (u32 k = 0; k < deg && e0 + k < gv.e_cnt; ++k) {
-                const u32 dst = gv.edge[2 * (size_t)(e0 + k)], ty = gv.edge[2 * (size_t)(e0 + k) + 1];
-                if (dst >= (u32)gv.n) continue;                        // malformed edge: ignore, never fault
-                const u32 v = (s >> (a.tmax - (int)min(ty, (u32)a.tmax))) & keep;
-                if (v) atomicOr(s_dst + dst, v);
-            }
-        }
+        auto send = [&](u32 e) {
+            if (e == kNoEdge) return;
+            const u32 v = (s_win[e & 1023u] >> (a.tmax - (int)(e >> 20))) & keep;
+            if (v) atomicOr(s_dst + ((e >> 10) & 1023u), v);
+        };
+#pragma unroll
+        for (int t = 0; t < 4; ++t) send(ahead[t]);
+        for (int e = threadIdx.x + 4 * blockDim.x; e < edges; e += blockDim.x) send(__ldg(packed + e));
         __syncthreads();
         // (4) out: node-major bytes, and the transposed rows of the unit's bits
         for (int j = warp; j < nw; j += nwarps) {
@@ -699,7 +705,7 @@ __global__ void __launch_bounds__(chain_threads(kHybrid, kNarrow), 1) fit_chain_
             } else {
                 if (!barrier(++nb)) return;
                 lap(1);
-                pull_messages<RW>(a, m, gv, bits, rows_t, rows_n, s_msg, s_msg + 32 * RW, s_msg + 64 * RW);
+                pull_messages<RW>(a, m, gv, a.packed + (u32)s_size[(int)(step & 3) * 4 + 2], s_size[(int)(step & 3) * 4 + 3], bits, rows_t, rows_n, s_msg, s_msg + 32 * RW, s_msg + 64 * RW);
                 lap(4);
                 if (!barrier(++nb)) return;
                 lap(1);

@@ -74,7 +74,7 @@ struct gtm_dataset {
     unsigned *rank_barrier = nullptr;      // arrival counter of the barriers among one rank's CTAs
     // learning on one GPU: message buffers (gtm_fit_chain.cu)
     bool chain_msg = false;
-    u32 *chain_bits = nullptr, *chain_rows_t = nullptr, *chain_rows_n = nullptr;
+    u32 *chain_bits = nullptr, *chain_rows_t = nullptr, *chain_rows_n = nullptr, *chain_packed = nullptr;
     int largest_edge_type = -1;            // -1: not known yet
     // scoring scratch of the general path: one slice per CTA
     EvalScratch score_sc;
