@@ -128,7 +128,7 @@ NCU_BINDING = {
     1: "tile_score_kernel<2>: short barrier-separated phases per tile (barrier stall 17.7 warps per issue); shared-memory wavefronts 27 % of peak, DRAM 1.2 %",
     2: "stream_score_kernel<10>: shared memory (wavefronts 64 % of peak, short-scoreboard stall 5.7 warps per issue); DRAM 0.5 %",
     3: "stream_score_kernel<10>: shared memory (wavefronts 62 % of peak); DRAM 0.5 %",
-    4: "score_graphs_kernel<1>: latency at 16 warps per SM with find-first-set loops on the quarter-rate pipe (XU 30 %, issue slots 43 %); DRAM 0.4 %",
+    4: "tile_score_kernel<2>, a graph per tile: shared-memory reads, 128 bytes per included literal and graph (not captured for this shape)",
     5: "tile_score_kernel<10>: shared memory (wavefronts 76 % of peak, 4.8 % of them from bank conflicts, issue slots 53 %); DRAM 7.9 %",
 }
 
