@@ -705,7 +705,7 @@ static int ensure_score_scratch(gtm_dataset *ds)
 {
     if (ds->score_sc.cno) return GTM_OK;
     const void *fn = score_kernel_for(ds->max_nodes, ds->score_units);
-    if (ds->score_smem > 48 * 1024) GTM_CU(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ds->score_smem));
+    if (ds->score_smem > 48 * 1024) GTM_CU(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, 224 * 1024));   // not the set's own: another set may need more
     int per_sm = 0;
     GTM_CU(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, ds->score_block, ds->score_smem));
     ds->score_grid = (int)std::max<int64_t>(1, std::min<int64_t>((int64_t)ds->model->sm_count * std::max(1, per_sm), ds->n_graphs));

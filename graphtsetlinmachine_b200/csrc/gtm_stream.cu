@@ -430,7 +430,7 @@ int stream_data_create(StreamData *sd, const StreamModel &sm, const DevModel &d,
     if (TNC == 0) return GTM_OK;
     const size_t smem = stream_smem_bytes(d.literals, TNC, kStreamMaxTypes);
     const void *fn = stream_kernel_for(d.K);
-    GTM_CU(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    GTM_CU(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, 224 * 1024));      // not the set's own: another set may need more
     int per_sm = 0;
     GTM_CU(cudaOccupancyMaxActiveBlocksPerMultiprocessorWithFlags(&per_sm, fn, kStreamThreads, smem, 0));
     if (per_sm < 1) return GTM_OK;

@@ -837,7 +837,8 @@ int tile_data_create(TileData *td, const TileModel &tm, const DevModel &d, const
     td->words_b = plan.words_b;
     td->stage_rows = plan.stage_rows;
     td->smem = plan.bytes;
-    GTM_CU(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)td->smem));
+    // the limit belongs to the kernel, not to the set: a set of a smaller plan must not lower it under another one's launches
+    GTM_CU(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
     int per_sm = 0;
     GTM_CU(cudaOccupancyMaxActiveBlocksPerMultiprocessorWithFlags(&per_sm, fn, td->threads, td->smem, 0));
     if (per_sm < 1) { tile_data_destroy(td); return GTM_OK; }
