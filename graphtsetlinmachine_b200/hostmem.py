@@ -2,8 +2,9 @@
 
 A result of a few megabytes in a fresh numpy array costs a page fault per page and a copy out of a staging buffer; in
 page-locked memory the copy engine writes it directly, in the time of the transfer.  Page-locking is slow (0.5 ms per MB),
-so the memory of an array that nobody refers to any more is kept for the next result, and memory is locked only for a
-size that has been asked for before: a program's first results are ordinary arrays.
+so the memory of an array that nobody refers to any more is kept for the next result, and a block is locked only for
+every eighth array of a size that is asked for: a program's first results are ordinary arrays, and what locking costs is
+spread over many.
 """
 
 import collections
@@ -18,9 +19,10 @@ from . import _lib
 SMALLEST, LARGEST = 64 << 10, 16 << 20      # bytes of an array that is worth it / that is not too much to lock
 MOST = 128 << 20                            # bytes locked at a time, arrays in use included
 
-AT_FIRST = 2                                # arrays of a size class that are ordinary memory
+PER_BLOCK = 8                               # arrays of a size class asked for, for every block that may be locked
 
-_asked = collections.Counter()                          # size class -> arrays asked for, up to AT_FIRST
+_asked = collections.Counter()                          # size class -> arrays asked for
+_blocks = collections.Counter()                         # size class -> blocks locked
 _free = collections.defaultdict(collections.deque)      # size class -> addresses
 _lock = threading.Lock()
 _locked = 0
@@ -45,6 +47,8 @@ def _take(size):
         pass
     lib = _lib.load()
     with _lock:
+        if (_blocks[size] + 1) * PER_BLOCK > _asked[size]:
+            return 0
         if _locked + size > MOST:           # free blocks of other sizes make room
             for other, blocks in list(_free.items()):
                 while blocks and _locked + size > MOST:
@@ -54,12 +58,14 @@ def _take(size):
                         break
                     lib.gtm_host_free(address)
                     _locked -= other
+                    _blocks[other] -= 1
         if _locked + size > MOST:
             return 0
         out = C.c_void_p()
         if lib.gtm_host_alloc(size, C.byref(out)) != 0:
             return 0
         _locked += size
+        _blocks[size] += 1
         return out.value
 
 
@@ -69,9 +75,7 @@ def empty(shape, dtype):
     if not SMALLEST <= nbytes <= LARGEST:
         return np.empty(shape, dtype=dtype)
     size = _size_class(nbytes)
-    if _asked[size] < AT_FIRST:
-        _asked[size] += 1
-        return np.empty(shape, dtype=dtype)
+    _asked[size] += 1
     address = _take(size)
     if not address:
         return np.empty(shape, dtype=dtype)

@@ -98,7 +98,7 @@ def test_pipelined_chunks(engine_lib, n, nodes, depth):
 
 def test_results_outlive_the_pool(engine_lib):
     """An array in recycled page-locked memory keeps its memory while it, or a view of it, is alive."""
-    for _ in range(hostmem.AT_FIRST):                            # a size's first arrays are ordinary memory
+    for _ in range(4 * hostmem.PER_BLOCK):                       # a size's first arrays are ordinary memory
         hostmem.empty((1000, 100), np.int32)
     a = hostmem.empty((1000, 100), np.int32)
     a[...] = 7
