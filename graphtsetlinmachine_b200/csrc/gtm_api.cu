@@ -768,6 +768,32 @@ static bool scores_by_tile(gtm_model *m, gtm_dataset *ds, int n_types)
     return m->opt_score_kernel == 0 || (m->opt_score_kernel == 3 && !ds->td.span && m->dm.K <= 16);
 }
 
+// One launch of a tiled kernel; clause_out_dev: the tile kernel only.  Its scratch belongs to the launch alone: kept with the
+// model or the set, launches on two streams would share it.
+static int launch_score_tiled(gtm_model *m, gtm_dataset *ds, bool by_stream, int n_types, int64_t first, int64_t count, int *sums_dev,
+                              int *clause_out_dev, char *scratch, cudaStream_t s)
+{
+    if (by_stream) return stream_score(m->sm, ds->sd, m->dm, ds->dg, n_types, first, count, sums_dev, scratch, s);
+    return tile_score(m->tm, ds->td, m->dm, ds->dg, n_types, first, count, sums_dev, clause_out_dev, m->score_error, scratch, s);
+}
+
+static size_t tiled_scratch_bytes(const gtm_model *m, const gtm_dataset *ds, bool by_stream, int64_t first, int64_t count)
+{
+    return by_stream ? stream_scratch_bytes(ds->sd, m->dm, first, count) : tile_scratch_bytes(ds->td, m->dm, first, count);
+}
+
+// The same on the model's stream, with lists and scratch.
+static int score_tiled(gtm_model *m, gtm_dataset *ds, bool by_stream, int n_types, int64_t first, int64_t count, int *sums_dev,
+                       int *clause_out_dev = nullptr)
+{
+    GTM_TRY(by_stream ? refresh_lists(m) : refresh_tile_lists(m));
+    char *scratch;
+    GTM_TRY(pool_alloc(&scratch, tiled_scratch_bytes(m, ds, by_stream, first, count), m->stream));
+    const int st = launch_score_tiled(m, ds, by_stream, n_types, first, count, sums_dev, clause_out_dev, scratch, m->stream);
+    cudaFreeAsync(scratch, m->stream);
+    return st;
+}
+
 extern "C" int gtm_score_device(gtm_model *m, gtm_dataset *ds, int n_types, int64_t first, int64_t count,
                                 int32_t *sums_dev)
 {
@@ -779,14 +805,8 @@ extern "C" int gtm_score_device(gtm_model *m, gtm_dataset *ds, int n_types, int6
         return fail(GTM_ERR_ARG, "the node-stream scoring kernel does not cover this model / graph set");
     if (m->opt_score_kernel == 3 && !scores_by_tile(m, ds, n_types))
         return fail(GTM_ERR_ARG, "the tile scoring kernel does not cover this model / graph set");
-    if (scores_by_stream(m, ds, n_types)) {
-        GTM_TRY(refresh_lists(m));
-        return stream_score(&m->sm, ds->sd, m->dm, ds->dg, n_types, first, count, sums_dev, 0, m->stream);
-    }
-    if (scores_by_tile(m, ds, n_types)) {
-        GTM_TRY(refresh_tile_lists(m));
-        return tile_score(&m->tm, ds->td, m->dm, ds->dg, n_types, first, count, sums_dev, nullptr, m->score_error, 0, m->stream);
-    }
+    const bool by_stream = scores_by_stream(m, ds, n_types);
+    if (by_stream || scores_by_tile(m, ds, n_types)) return score_tiled(m, ds, by_stream, n_types, first, count, sums_dev);
     return launch_score_general(m, ds, n_types, first, count, sums_dev, nullptr);
 }
 
@@ -821,21 +841,23 @@ static int score_in_chunks(gtm_model *m, gtm_dataset *ds, const gtm_graphs_view 
     }
     if (!by_stream) chunk_tiles = (chunk_tiles + m->sm_count - 1) / m->sm_count * m->sm_count;
     const bool pinned_out = host_is_pinned(out);
+    auto chunk_lo = [&](int t0) { return std::max(first, tile_first(t0)); };
+    auto chunk_hi = [&](int t0) { return std::min(first + count, tile_first(t0 + chunk_tiles)); };
     int *dev = nullptr;
+    char *scratch[2] = {nullptr, nullptr};              // of the launches on either stream
     auto body = [&]() -> int {
-        if (by_stream) {
-            GTM_TRY(refresh_lists(m));
-            GTM_TRY(stream_reserve(&m->sm, ds->sd, d, std::min(chunk_tiles, tiles)));
-        } else {
-            GTM_TRY(refresh_tile_lists(m));
-        }
+        GTM_TRY(by_stream ? refresh_lists(m) : refresh_tile_lists(m));
+        size_t need = 0;
+        for (int t0 = t_lo; t0 < t_hi; t0 += chunk_tiles)
+            if (chunk_hi(t0) > chunk_lo(t0)) need = std::max(need, tiled_scratch_bytes(m, ds, by_stream, chunk_lo(t0), chunk_hi(t0) - chunk_lo(t0)));
+        for (int i = 0; i < (chunk_tiles < tiles ? 2 : 1); ++i) GTM_TRY(pool_alloc(&scratch[i], need, m->stream));
         GTM_TRY(pool_alloc(&dev, (size_t)count * d.K, m->stream));
         GTM_CU(cudaEventRecord(lane->event[0], m->stream));       // allocations, tile tables and literal lists are in stream order
         GTM_CU(cudaStreamWaitEvent(lane->in, lane->event[0], 0));
         GTM_CU(cudaStreamWaitEvent(lane->aux, lane->event[0], 0));
         int turn = 0;
         for (int t0 = t_lo; t0 < t_hi; t0 += chunk_tiles, turn ^= 1) {
-            const int64_t g0 = std::max(first, tile_first(t0)), g1 = std::min(first + count, tile_first(t0 + chunk_tiles));
+            const int64_t g0 = chunk_lo(t0), g1 = chunk_hi(t0);
             if (g1 <= g0) continue;
             const size_t cnt = (size_t)(g1 - g0), at = (size_t)(g0 - first) * d.K;
             cudaStream_t cs = turn ? lane->aux : m->stream;
@@ -848,8 +870,7 @@ static int score_in_chunks(gtm_model *m, gtm_dataset *ds, const gtm_graphs_view 
                 GTM_CU(cudaStreamWaitEvent(cs, lane->event[1], 0));
                 GTM_TRY(fill_range(f, cs));
             }
-            if (by_stream) GTM_TRY(stream_score(&m->sm, ds->sd, d, ds->dg, n_types, g0, (int64_t)cnt, dev + at, turn, cs));
-            else GTM_TRY(tile_score(&m->tm, ds->td, d, ds->dg, n_types, g0, (int64_t)cnt, dev + at, nullptr, m->score_error, turn, cs));
+            GTM_TRY(launch_score_tiled(m, ds, by_stream, n_types, g0, (int64_t)cnt, dev + at, nullptr, scratch[turn], cs));
             GTM_CU(cudaEventRecord(lane->event[2], cs));
             GTM_CU(cudaStreamWaitEvent(lane->back, lane->event[2], 0));
             GTM_TRY(stage_down(lane, out + at, dev + at, cnt * d.K * sizeof(int), pinned_out, lane->back));
@@ -867,6 +888,7 @@ static int score_in_chunks(gtm_model *m, gtm_dataset *ds, const gtm_graphs_view 
         cudaStreamSynchronize(m->stream);
     }
     if (dev) cudaFreeAsync(dev, m->stream);
+    for (char *p : scratch) if (p) cudaFreeAsync(p, m->stream);
     return st;
 }
 
@@ -987,8 +1009,7 @@ static int transform_common(gtm_model *m, gtm_dataset *ds, int n_types, int64_t 
         // clause outputs of whole graphs come out of the tile kernel too; outputs per node only out of the general one
         if (!node_out && clause_out && m->opt_score_kernel != 1) st = ensure_tiles(m, ds);
         if (st == GTM_OK && !node_out && clause_out && m->opt_score_kernel != 1 && tile_supported(ds->td, n_types)) {
-            st = refresh_tile_lists(m);
-            if (st == GTM_OK) st = tile_score(&m->tm, ds->td, m->dm, ds->dg, n_types, first, count, sums_dev, co_dev, m->score_error, 0, m->stream);
+            st = score_tiled(m, ds, false, n_types, first, count, sums_dev, co_dev);
         } else if (st == GTM_OK) {
             st = launch_score_general(m, ds, n_types, first, count, sums_dev, co_dev, no_dev, node_stride);
         }

@@ -110,11 +110,11 @@ struct StreamArgs {
     int64_t first, count;               // graphs written: [first, first+count)
     int64_t n_graphs, total_nodes;
     int *class_sums;                    // [count][K]
-    unsigned *unit_counter;             // units handed out beyond the first of every CTA; left at zero
+    unsigned *unit_counter;             // units handed out beyond the first of every CTA, zero before the launch
     int splits;                         // shares of a tile's clauses
     int blocks_per_split;               // clause blocks of a share
     int *part;                          // [splits][n_graphs][K] partial sums (splits > 1)
-    int *ticket;                        // [tiles of the launch] shares of a tile that are done (splits > 1); left at zero
+    int *ticket;                        // [tiles of the launch] shares of a tile that are done (splits > 1), zero before the launch
     int TNC;
     const int *lit_cnt;
     const unsigned short *lit_list;
@@ -336,7 +336,6 @@ __global__ void __launch_bounds__(kStreamThreads, 2) stream_score_kernel(DevMode
             write = s_last != 0;
             if (write) {
                 __threadfence();
-                if (tid == 0) a.ticket[tile - a.tile_lo] = 0;
                 for (int i = tid; i < ng * m.K; i += kStreamThreads) {
                     int v = sums[i];
                     for (int s = 0; s < a.splits; ++s)
@@ -351,13 +350,9 @@ __global__ void __launch_bounds__(kStreamThreads, 2) stream_score_kernel(DevMode
                 const int64_t gi = (int64_t)g0 + i / m.K;
                 if (gi >= a.first && gi < a.first + a.count) a.class_sums[((int64_t)g0 - a.first) * m.K + i] = sums[i];
             }
-        // ---- next unit: the CTA whose request is the last of the launch leaves the counter at zero ----
+        // ---- next unit ----
         if (more <= 0) break;
-        if (tid == 0) {
-            const int got = (int)atomicAdd(a.unit_counter, 1u);
-            if (got == more + (int)gridDim.x - 1) *a.unit_counter = 0u;
-            s_unit = (int)gridDim.x + got;
-        }
+        if (tid == 0) s_unit = (int)gridDim.x + (int)atomicAdd(a.unit_counter, 1u);
         __syncthreads();       // s_unit; the shared buffers are reused by the next unit
         unit = s_unit;
     }
@@ -389,24 +384,23 @@ int stream_model_create(StreamModel *sm, const DevModel &d)
     GTM_TRY(dev_alloc(&sm->lit_cnt, (size_t)d.C));
     GTM_TRY(dev_alloc(&sm->lit_list, (size_t)d.C * sm->list_stride));
     GTM_TRY(dev_alloc(&sm->wf, wf));
-    GTM_TRY(dev_alloc(&sm->sync, (size_t)3 + 2 * kStreamMaxSplitTiles));
+    GTM_TRY(dev_alloc(&sm->limbs, 1));
     GTM_CU(cudaMemset(sm->wf, 0, wf));
-    GTM_CU(cudaMemset(sm->sync, 0, ((size_t)3 + 2 * kStreamMaxSplitTiles) * sizeof(int)));
     sm->applicable = true;
     return GTM_OK;
 }
 
 void stream_model_destroy(StreamModel *sm)
 {
-    cudaFree(sm->lit_cnt); cudaFree(sm->lit_list); cudaFree(sm->wf); cudaFree(sm->sync); cudaFree(sm->part);
+    cudaFree(sm->lit_cnt); cudaFree(sm->lit_list); cudaFree(sm->wf); cudaFree(sm->limbs);
     *sm = StreamModel();
 }
 
 int stream_model_refresh(StreamModel *sm, const DevModel &d, cudaStream_t s)
 {
     if (!sm->applicable) return GTM_OK;
-    GTM_CU(cudaMemsetAsync(sm->sync + 2, 0, sizeof(int), s));
-    stream_lists_kernel<<<(d.C + 7) / 8, 256, 0, s>>>(d, sm->lit_cnt, sm->lit_list, sm->list_stride, sm->wf, stream_kt(d.K), sm->sync + 2);
+    GTM_CU(cudaMemsetAsync(sm->limbs, 0, sizeof(int), s));
+    stream_lists_kernel<<<(d.C + 7) / 8, 256, 0, s>>>(d, sm->lit_cnt, sm->lit_list, sm->list_stride, sm->wf, stream_kt(d.K), sm->limbs);
     GTM_CU(cudaGetLastError());
     return GTM_OK;
 }
@@ -507,22 +501,19 @@ static void stream_tiles(const StreamData &sd, int64_t first, int64_t count, int
     }
 }
 
-int stream_reserve(StreamModel *sm, const StreamData &sd, const DevModel &d, int tiles)
+// Scratch of a launch: the unit counter, a ticket per tile when the clauses are split, then the shares' partial sums.
+static size_t stream_sync_bytes(int tiles, int splits) { return (((size_t)1 + (splits > 1 ? tiles : 0)) * sizeof(int) + 255) & ~(size_t)255; }
+
+size_t stream_scratch_bytes(const StreamData &sd, const DevModel &d, int64_t first, int64_t count)
 {
-    int per;
-    const int splits = stream_splits(sd, d, tiles, &per);
-    const size_t need = splits > 1 ? (size_t)splits * sd.n_graphs * d.K : 0;
-    if (need > sm->part_cap) {
-        cudaFree(sm->part);                            // waits for the kernels that use it
-        sm->part = nullptr; sm->part_cap = 0;
-        GTM_TRY(dev_alloc(&sm->part, need + need / 2));
-        sm->part_cap = need + need / 2;
-    }
-    return GTM_OK;
+    int lo, hi, per;
+    stream_tiles(sd, first, count, &lo, &hi);
+    const int splits = stream_splits(sd, d, hi - lo, &per);
+    return stream_sync_bytes(hi - lo, splits) + (splits > 1 ? (size_t)splits * sd.n_graphs * d.K * sizeof(int) : 0);
 }
 
-int stream_score(StreamModel *sm, const StreamData &sd, const DevModel &d, const DevGraphs &dg, int n_types,
-                 int64_t first, int64_t count, int *sums_dev, int lane, cudaStream_t s)
+int stream_score(const StreamModel &sm, const StreamData &sd, const DevModel &d, const DevGraphs &dg, int n_types,
+                 int64_t first, int64_t count, int *sums_dev, char *scratch, cudaStream_t s)
 {
     DevGraphs g = dg;
     g.n_types = n_types;
@@ -530,15 +521,16 @@ int stream_score(StreamModel *sm, const StreamData &sd, const DevModel &d, const
     a.tile_graph = sd.tile_graph;
     stream_tiles(sd, first, count, &a.tile_lo, &a.tile_hi);          // tiles that overlap [first, first+count)
     const int tiles = a.tile_hi - a.tile_lo;
-    GTM_TRY(stream_reserve(sm, sd, d, tiles));
     a.splits = stream_splits(sd, d, tiles, &a.blocks_per_split);
-    a.part = sm->part; a.ticket = sm->sync + 3 + lane * kStreamMaxSplitTiles;
+    const size_t sync_bytes = stream_sync_bytes(tiles, a.splits);
+    a.unit_counter = (unsigned *)scratch; a.ticket = (int *)scratch + 1; a.part = (int *)(scratch + sync_bytes);
     a.graphs_per_tile = sd.graphs_per_tile;
     a.first = first; a.count = count; a.n_graphs = sd.n_graphs; a.total_nodes = sd.total_nodes;
-    a.class_sums = sums_dev; a.unit_counter = (unsigned *)sm->sync + lane; a.TNC = sd.TNC;
-    a.lit_cnt = sm->lit_cnt; a.lit_list = sm->lit_list; a.list_stride = sm->list_stride;
-    a.wf = sm->wf; a.limbs = sm->sync + 2;
+    a.class_sums = sums_dev; a.TNC = sd.TNC;
+    a.lit_cnt = sm.lit_cnt; a.lit_list = sm.lit_list; a.list_stride = sm.list_stride;
+    a.wf = sm.wf; a.limbs = sm.limbs;
     const int grid = std::max(1, std::min(sd.grid, tiles * a.splits));
+    if (a.splits > 1 || tiles > grid) GTM_CU(cudaMemsetAsync(scratch, 0, sync_bytes, s));      // else the kernel reads none of it
     DevModel dm = d;
     void *args[] = {&dm, &g, &a};
     GTM_CU(cudaLaunchKernel(stream_kernel_for(d.K), dim3(grid), dim3(kStreamThreads), args, stream_smem_bytes(d.literals, sd.TNC, n_types), s));

@@ -13,9 +13,7 @@ struct StreamModel {
     unsigned short *lit_list = nullptr; // [C][list_stride] row numbers of the included literals
     int list_stride = 0;
     signed char *wf = nullptr;          // weights as tensor-core fragments, see stream_weight_at
-    int *sync = nullptr;                // unit counters of two launches side by side, limbs in use, share tickets
-    int *part = nullptr;                // partial class sums of launches that split the clauses; grows on demand
-    size_t part_cap = 0;
+    int *limbs = nullptr;               // signed bytes that the largest weight needs
 };
 
 struct StreamData {
@@ -38,10 +36,10 @@ int stream_data_create(StreamData *sd, const StreamModel &sm, const DevModel &d,
                        int sm_count, cudaStream_t s);
 void stream_data_destroy(StreamData *sd);
 bool stream_supported(const StreamData &sd, int n_types);
-// Makes room for the partial sums of launches over `tiles` tiles (before launches on two streams).
-int stream_reserve(StreamModel *sm, const StreamData &sd, const DevModel &d, int tiles);
-// `lane` (0 or 1): launches that may run side by side, on disjoint tiles, take different ones.
-int stream_score(StreamModel *sm, const StreamData &sd, const DevModel &d, const DevGraphs &dg, int n_types,
-                 int64_t first, int64_t count, int *sums_dev, int lane, cudaStream_t s);
+// Bytes of scratch (256-byte aligned device memory, no contents expected) that a launch over graphs [first, first+count)
+// needs.  The scratch belongs to one launch: launches on different streams share nothing.
+size_t stream_scratch_bytes(const StreamData &sd, const DevModel &d, int64_t first, int64_t count);
+int stream_score(const StreamModel &sm, const StreamData &sd, const DevModel &d, const DevGraphs &dg, int n_types,
+                 int64_t first, int64_t count, int *sums_dev, char *scratch, cudaStream_t s);
 
 }  // namespace gtm

@@ -147,7 +147,7 @@ struct TileArgs {
     int64_t first, count;               // graphs written: [first, first+count)
     int64_t n_graphs;
     int *class_sums;                    // [count][K]
-    unsigned *tile_counter;             // tiles handed out beyond the first of every CTA; left at zero
+    unsigned *tile_counter;             // tiles handed out beyond the first of every CTA, zero before the launch
     int *clause_out;                    // [count][C] clause outputs, zero before the launch, or NULL
     int TNC, PS, words_a, words_b, stage_rows, gmax;
     int pw;                             // node words of a literal row: TNC, or 8 and TNC/8 planes of rows one after the other
@@ -615,13 +615,9 @@ __global__ void __launch_bounds__(kTileThreadsAlone, 1) tile_score_kernel(DevMod
             const int64_t gi = (int64_t)g0 + gl;
             if (gi >= a.first && gi < a.first + a.count) a.class_sums[(size_t)(gi - a.first) * m.K + k] = sums[gl * KS + k];
         }
-        // ---- next tile: the CTA whose request is the last of the launch leaves the counter at zero ----
+        // ---- next tile ----
         if (more <= 0) break;
-        if (tid == 0) {
-            const int got = (int)atomicAdd(a.tile_counter, 1u);
-            if (got == more + (int)gridDim.x - 1) *a.tile_counter = 0u;
-            misc[0] = a.tile_lo + (int)gridDim.x + got;
-        }
+        if (tid == 0) misc[0] = a.tile_lo + (int)gridDim.x + (int)atomicAdd(a.tile_counter, 1u);
         __syncthreads();                              // misc; the shared tables are rewritten by the next tile
         tile = misc[0];
     }
@@ -660,15 +656,13 @@ int tile_model_create(TileModel *tm, const DevModel &d)
         GTM_TRY(dev_alloc(&tm->order[l], (size_t)d.C));
         GTM_TRY(dev_alloc(&tm->blk_off[l], (size_t)((d.C + 31) / 32) + 1));
     }
-    GTM_TRY(dev_alloc(&tm->counters, 2));
-    GTM_CU(cudaMemset(tm->counters, 0, 2 * sizeof(unsigned)));
     tm->applicable = true;
     return GTM_OK;
 }
 
 void tile_model_destroy(TileModel *tm)
 {
-    cudaFree(tm->Wt); cudaFree(tm->hvm); cudaFree(tm->layers); cudaFree(tm->counters); cudaFree(tm->surv_r[0]); cudaFree(tm->surv_r[1]);
+    cudaFree(tm->Wt); cudaFree(tm->hvm); cudaFree(tm->layers);
     for (int l = 0; l < kMaxDepth; ++l) { cudaFree(tm->cnt[l]); cudaFree(tm->order[l]); cudaFree(tm->blk_off[l]); cudaFree(tm->list[l]); }
     *tm = TileModel();
 }
@@ -858,10 +852,34 @@ void tile_data_destroy(TileData *td)
 
 bool tile_supported(const TileData &td, int n_types) { return td.supported != 0 && n_types <= kTileMaxTypes; }
 
-int tile_score(TileModel *model, const TileData &td, const DevModel &d, const DevGraphs &dg, int n_types, int64_t first,
-               int64_t count, int *sums_dev, int *clause_out_dev, int *error_dev, int lane, cudaStream_t s)
+// Tiles [lo, hi) that overlap graphs [first, first+count).
+static void tile_range(const TileData &td, int64_t first, int64_t count, int *lo, int *hi)
 {
-    TileModel &tm = *model;
+    if (td.graphs_per_tile > 0) {
+        *lo = (int)(first / td.graphs_per_tile);
+        *hi = (int)((first + count + td.graphs_per_tile - 1) / td.graphs_per_tile);
+    } else {
+        const std::vector<int> &tg = td.tile_graph_host;
+        *lo = (int)(std::upper_bound(tg.begin(), tg.end(), (int)first) - tg.begin()) - 1;
+        *hi = (int)(std::lower_bound(tg.begin(), tg.end(), (int)(first + count)) - tg.begin());
+    }
+}
+
+static int tile_grid(const TileData &td, int lo, int hi) { return std::max(1, std::min(td.grid, hi - lo)); }
+
+constexpr size_t kTileCounterBytes = 256;              // the tile counter; then the node bits of every clause between layers
+
+size_t tile_scratch_bytes(const TileData &td, const DevModel &d, int64_t first, int64_t count)
+{
+    int lo, hi;
+    tile_range(td, first, count, &lo, &hi);
+    const size_t pairs = (size_t)(td.TNC / 4 + 1) / 2;
+    return kTileCounterBytes + 2 * (size_t)tile_grid(td, lo, hi) * 2 * pairs * d.C * sizeof(uint4);
+}
+
+int tile_score(const TileModel &tm, const TileData &td, const DevModel &d, const DevGraphs &dg, int n_types, int64_t first,
+               int64_t count, int *sums_dev, int *clause_out_dev, int *error_dev, char *scratch, cudaStream_t s)
+{
     DevGraphs g = dg;
     g.n_types = n_types;
     TileArgs a;
@@ -870,33 +888,19 @@ int tile_score(TileModel *model, const TileData &td, const DevModel &d, const De
     a.uniform_n = td.uniform_n;
     a.graphs_per_tile = td.graphs_per_tile;
     int lo, hi;
-    if (td.graphs_per_tile > 0) {
-        lo = (int)(first / td.graphs_per_tile);
-        hi = (int)((first + count + td.graphs_per_tile - 1) / td.graphs_per_tile);
-    } else {
-        const std::vector<int> &tg = td.tile_graph_host;
-        lo = (int)(std::upper_bound(tg.begin(), tg.end(), (int)first) - tg.begin()) - 1;
-        hi = (int)(std::lower_bound(tg.begin(), tg.end(), (int)(first + count)) - tg.begin());
-    }
+    tile_range(td, first, count, &lo, &hi);
     a.tile_lo = lo; a.tile_hi = hi;
     a.first = first; a.count = count; a.n_graphs = td.n_graphs;
-    a.class_sums = sums_dev; a.clause_out = clause_out_dev; a.pw = td.pw; a.span = td.span; a.tile_counter = tm.counters + lane;
+    a.class_sums = sums_dev; a.clause_out = clause_out_dev; a.pw = td.pw; a.span = td.span; a.tile_counter = (unsigned *)scratch;
     a.TNC = td.TNC; a.PS = td.PS; a.words_a = td.words_a; a.words_b = td.words_b; a.stage_rows = td.stage_rows; a.gmax = td.gmax;
     int inv = 1;                                       // inverse of the (odd) message row stride modulo 32
     while ((td.PS * inv) % 32 != 1) inv += 2;
     a.rot_step = ((32 / td.TNC) * inv) & 31;
     a.layers = tm.layers; a.Wt = tm.Wt; a.KROW = tm.KROW; a.hvm = tm.hvm;
-    const int grid = std::max(1, std::min(td.grid, hi - lo)), U = (td.TNC / 4 + 1) / 2;
-    // node bits of every clause between layers, per CTA, layer parity and quad pair: kept by the model, grows on demand
-    const size_t need = 2 * (size_t)grid * 2 * U * d.C;
-    if (need > tm.surv_cap[lane]) {
-        cudaFree(tm.surv_r[lane]);                     // waits for the kernels that use it
-        tm.surv_r[lane] = nullptr; tm.surv_cap[lane] = 0;
-        GTM_TRY(dev_alloc(&tm.surv_r[lane], need));
-        tm.surv_cap[lane] = need;
-    }
-    a.surv_r = tm.surv_r[lane];
+    const int grid = tile_grid(td, lo, hi);
+    a.surv_r = (uint4 *)(scratch + kTileCounterBytes);
     a.error = error_dev;
+    if (hi - lo > grid) GTM_CU(cudaMemsetAsync(a.tile_counter, 0, sizeof(unsigned), s));       // else no CTA asks for a tile
     if (clause_out_dev) GTM_CU(cudaMemsetAsync(clause_out_dev, 0, (size_t)count * d.C * sizeof(int), s));      // the kernel writes the ones
     DevModel dm = d;
     void *args[] = {&dm, &g, &a};

@@ -29,9 +29,6 @@ struct TileModel {
     int *Wt = nullptr;            // [C][KROW] weights, clause-major
     u32 *hvm = nullptr;           // [C][MB] hypervector bits reduced modulo the message size
     TileLayer *layers = nullptr;  // [D] device copy of the pointers above
-    unsigned *counters = nullptr; // [2] tile counters of two launches side by side
-    uint4 *surv_r[2] = {};        // per launch: [grid][2][quad pairs][C][2] node bits of every clause on the pair's two quads after a layer
-    size_t surv_cap[2] = {};
 };
 
 struct TileData {
@@ -63,9 +60,11 @@ int tile_data_create(TileData *td, const TileModel &tm, const DevModel &d, const
                      int sm_count, cudaStream_t s);
 void tile_data_destroy(TileData *td);
 bool tile_supported(const TileData &td, int n_types);
+// Bytes of scratch (256-byte aligned device memory, no contents expected) that a launch over graphs [first, first+count)
+// needs.  The scratch belongs to one launch: launches on different streams share nothing.
+size_t tile_scratch_bytes(const TileData &td, const DevModel &d, int64_t first, int64_t count);
 // `clause_out_dev`: clause outputs int32[count][C], or null.
-// `lane` (0 or 1): launches that may run side by side, on disjoint tiles, take different ones.
-int tile_score(TileModel *model, const TileData &td, const DevModel &d, const DevGraphs &dg, int n_types, int64_t first,
-               int64_t count, int *sums_dev, int *clause_out_dev, int *error_dev, int lane, cudaStream_t s);
+int tile_score(const TileModel &tm, const TileData &td, const DevModel &d, const DevGraphs &dg, int n_types, int64_t first,
+               int64_t count, int *sums_dev, int *clause_out_dev, int *error_dev, char *scratch, cudaStream_t s);
 
 }  // namespace gtm
