@@ -30,6 +30,23 @@ static int bind(gtm_model *m)
     return GTM_OK;
 }
 
+static bool is_capturing(cudaStream_t s)
+{
+    cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(s, &status) != cudaSuccess) { cudaGetLastError(); return true; }
+    return status != cudaStreamCaptureStatusNone;
+}
+
+// For calls that return with work in flight: gtm_set_stream orders the next stream behind it.  Work that is recorded into a
+// graph is not in flight; its replays are the caller's to order.
+static int note_queued(gtm_model *m)
+{
+    if (is_capturing(m->stream)) return GTM_OK;
+    GTM_CU(cudaEventRecord(m->queued, m->stream));
+    m->in_flight = true;
+    return GTM_OK;
+}
+
 // largest float that is <= d
 static float float_round_down(double d)
 {
@@ -129,6 +146,7 @@ extern "C" int gtm_create(const gtm_config *cfg, gtm_model **out)
     if (st == GTM_OK) st = dev_alloc(&m->error, 1);
     if (st == GTM_OK && cudaMallocHost((void **)&m->score_error, sizeof(int)) != cudaSuccess) st = fail(GTM_ERR_OOM, "page-locked host allocation failed");
     if (st == GTM_OK) st = dev_alloc(&m->phase_cycles, 8);
+    if (st == GTM_OK && cudaEventCreateWithFlags(&m->queued, cudaEventDisableTiming) != cudaSuccess) st = fail(GTM_ERR_CUDA, "an event could not be created");
     if (st != GTM_OK) { gtm_destroy(m); return st; }
     d.hv = hv;
     m->hv_host.assign((size_t)d.C * d.MB, 0);
@@ -159,6 +177,7 @@ extern "C" int gtm_destroy(gtm_model *m)
     stream_model_destroy(&m->sm);
     tile_model_destroy(&m->tm);
     if (m->score_error) cudaFreeHost(m->score_error);
+    if (m->queued) cudaEventDestroy(m->queued);
     delete m;
     stage_drop();
     return GTM_OK;
@@ -167,6 +186,10 @@ extern "C" int gtm_destroy(gtm_model *m)
 extern "C" int gtm_set_stream(gtm_model *m, void *stream)
 {
     GTM_TRY(bind(m));
+    // Lists, weights and automata are the model's: what is in flight on the old stream makes or reads them.  (The old stream
+    // itself may be gone by now, the event is not.)
+    if (m->in_flight && (cudaStream_t)stream != m->stream && !is_capturing((cudaStream_t)stream))
+        GTM_CU(cudaStreamWaitEvent((cudaStream_t)stream, m->queued, 0));
     m->stream = (cudaStream_t)stream;
     return GTM_OK;
 }
@@ -794,8 +817,7 @@ static int score_tiled(gtm_model *m, gtm_dataset *ds, bool by_stream, int n_type
     return st;
 }
 
-extern "C" int gtm_score_device(gtm_model *m, gtm_dataset *ds, int n_types, int64_t first, int64_t count,
-                                int32_t *sums_dev)
+static int score_device(gtm_model *m, gtm_dataset *ds, int n_types, int64_t first, int64_t count, int32_t *sums_dev)
 {
     GTM_TRY(bind(m));
     GTM_TRY(check_range(m, ds, n_types, first, count));
@@ -808,6 +830,13 @@ extern "C" int gtm_score_device(gtm_model *m, gtm_dataset *ds, int n_types, int6
     const bool by_stream = scores_by_stream(m, ds, n_types);
     if (by_stream || scores_by_tile(m, ds, n_types)) return score_tiled(m, ds, by_stream, n_types, first, count, sums_dev);
     return launch_score_general(m, ds, n_types, first, count, sums_dev, nullptr);
+}
+
+extern "C" int gtm_score_device(gtm_model *m, gtm_dataset *ds, int n_types, int64_t first, int64_t count,
+                                int32_t *sums_dev)
+{
+    GTM_TRY(score_device(m, ds, n_types, first, count, sums_dev));
+    return note_queued(m);
 }
 
 // Scoring of graphs [first, first+count) into host memory by a tiled kernel, pipelined: chunks of whole tiles are scored
@@ -899,7 +928,7 @@ static int score_to_host(gtm_model *m, gtm_dataset *ds, int n_types, int64_t fir
     // a few results: the kernel writes them to page-locked host memory itself, which takes less than starting a copy
     if (bytes <= 16 * 1024) {
         int *direct = (int *)(lane->small + kStageSmall);
-        GTM_TRY(gtm_score_device(m, ds, n_types, first, count, direct));
+        GTM_TRY(score_device(m, ds, n_types, first, count, direct));
         GTM_CU(cudaStreamSynchronize(m->stream));
         GTM_TRY(score_flag_status(m));
         memcpy(out, direct, bytes);
@@ -912,7 +941,7 @@ static int score_to_host(gtm_model *m, gtm_dataset *ds, int n_types, int64_t fir
     }
     int *dev;
     GTM_TRY(pool_alloc(&dev, (size_t)count * m->dm.K, m->stream));
-    int st = gtm_score_device(m, ds, n_types, first, count, dev);
+    int st = score_device(m, ds, n_types, first, count, dev);
     if (st == GTM_OK) st = stage_down(lane, out, dev, bytes, host_is_pinned(out), m->stream);
     cudaFreeAsync(dev, m->stream);
     if (st == GTM_OK) st = stage_down_finish(lane);
@@ -1281,7 +1310,7 @@ extern "C" int gtm_score_static_scratch(gtm_model *m, const gtm_graphs_view *v, 
     a.part_words = 0; a.t_stride = 0;
     score_graphs_kernel<true><<<grid, 256, (size_t)d.K * sizeof(int), m->stream>>>(d, g, sc, a);
     GTM_CU(cudaGetLastError());
-    return GTM_OK;
+    return note_queued(m);
 }
 
 extern "C" int gtm_check_skipped_graphs(gtm_model *m, int *skipped_out)

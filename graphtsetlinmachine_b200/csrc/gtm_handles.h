@@ -14,6 +14,8 @@ struct gtm_model {
     gtm_config cfg;
     DevModel dm;
     cudaStream_t stream = nullptr;
+    cudaEvent_t queued = nullptr;             // behind the last work that a call left in flight on `stream`
+    bool in_flight = false;                   // `queued` was recorded
     int sm_count = 0;
     bool has_state = false;
     u32 *recorded = nullptr;

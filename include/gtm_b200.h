@@ -83,7 +83,8 @@ int gtm_create(const gtm_config *config, gtm_model **model_out);
 int gtm_destroy(gtm_model *model);
 
 /* All device work of a model is issued on this CUDA stream (a cudaStream_t passed as void*; NULL = the legacy
- * default stream, which is also the default). */
+ * default stream, which is also the default).  Work that earlier calls left in flight on the stream before comes first on
+ * the new one, unless the new one is being captured into a graph: then the caller orders the two. */
 int gtm_set_stream(gtm_model *model, void *cuda_stream);
 
 /* Kernel selection (the reference has one code path; its only launch knobs are grid/block, tm.py:53-54).

@@ -103,3 +103,33 @@ def test_captured_launch(engine_lib, depth):
     del graph
     tm.lib.gtm_dataset_destroy(ds)
     tm.close()
+
+
+@pytest.mark.parametrize("depth", [1, 2])
+def test_lists_of_one_stream_on_the_next(engine_lib, depth):
+    """The first launch after new automata makes the literal lists; a launch on another stream right behind it waits for them.
+    Later automata on a third stream leave launches in flight alone."""
+    tm, base = learned(depth, clauses=4000)
+    large, _ = resident(tm, base[np.arange(40000) % 200])
+    small, old_want = resident(tm, base[:100])
+    planes = [tm.get_ta(d) for d in range(depth)]
+    streams = [torch.cuda.Stream() for _ in range(3)]
+    out_large, out_small, out_last = sums(40000, tm), sums(100, tm), sums(100, tm)
+    for turn in range(4):
+        changed = turn % 2 == 0                            # include planes shifted by a clause, then as they were
+        for d, p in enumerate(planes):
+            tm.set_ta(d, np.roll(p, 1, axis=0) if changed else p)
+        queue(tm, large, streams[0], out_large)
+        queue(tm, small, streams[1], out_small)
+        queue(tm, small, streams[2], out_last)
+        torch.cuda.synchronize()
+        got = out_small.cpu().numpy()
+        tm.ds, keep = small, tm.ds
+        want = tm.score(0, 100)
+        tm.ds = keep
+        assert np.array_equal(got, want) and np.array_equal(out_last.cpu().numpy(), want)
+        assert np.array_equal(out_large.cpu().numpy()[:100], want)
+        assert changed or np.array_equal(want, old_want)
+    for ds in (large, small):
+        tm.lib.gtm_dataset_destroy(ds)
+    tm.close()
