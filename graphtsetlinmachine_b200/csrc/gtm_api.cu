@@ -672,8 +672,8 @@ extern "C" int gtm_dataset_destroy(gtm_dataset *ds)
     cudaSetDevice(ds->model->cfg.device);
     for (void *p : ds->owned) cudaFreeAsync(p, ds->model->stream);        // in stream order, behind the kernels that use them
     if (ds->Y) cudaFree(ds->Y);
-    stream_data_destroy(&ds->sd);
-    tile_data_destroy(&ds->td);
+    stream_data_destroy(&ds->sd, ds->model->stream);
+    tile_data_destroy(&ds->td, ds->model->stream);
     if (ds->comm.block) cudaStreamSynchronize(ds->model->stream);
     fit_comm_release(ds);
     delete ds;

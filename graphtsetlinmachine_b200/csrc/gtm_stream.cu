@@ -453,7 +453,6 @@ int stream_data_create(StreamData *sd, const StreamModel &sm, const DevModel &d,
         GTM_TRY(pool_alloc(&sd->tile_graph, tg.size(), s));
         GTM_CU(cudaMemcpyAsync(sd->tile_graph, tg.data(), tg.size() * sizeof(int), cudaMemcpyHostToDevice, s));
     }
-    sd->stream = s;
     sd->TNC = TNC;
     sd->grid = sm_count * per_sm;
     sd->total_nodes = v->total_nodes;
@@ -462,9 +461,10 @@ int stream_data_create(StreamData *sd, const StreamModel &sm, const DevModel &d,
     return GTM_OK;
 }
 
-void stream_data_destroy(StreamData *sd)
+// s: a stream behind every kernel that reads the tables (the model's, which may not be the one they were made on).
+void stream_data_destroy(StreamData *sd, cudaStream_t s)
 {
-    if (sd->tile_graph) cudaFreeAsync(sd->tile_graph, sd->stream);
+    if (sd->tile_graph) cudaFreeAsync(sd->tile_graph, s);
     sd->tile_graph = nullptr; sd->supported = 0;
 }
 

@@ -22,7 +22,6 @@ struct StreamData {
     int n_tiles = 0;
     int *tile_graph = nullptr;          // [n_tiles+1] first graph of every tile (NULL for sets of equally large graphs)
     int graphs_per_tile = 0;            // > 0: every tile holds this many graphs
-    cudaStream_t stream = nullptr;      // stream the pooled buffers were allocated on
     std::vector<int> tile_graph_host;
     int grid = 0;
     int64_t total_nodes = 0, n_graphs = 0;
@@ -34,7 +33,7 @@ void stream_model_destroy(StreamModel *sm);
 int stream_model_refresh(StreamModel *sm, const DevModel &d, cudaStream_t s);
 int stream_data_create(StreamData *sd, const StreamModel &sm, const DevModel &d, const gtm_graphs_view *v, u32 n_min, u32 n_max,
                        int sm_count, cudaStream_t s);
-void stream_data_destroy(StreamData *sd);
+void stream_data_destroy(StreamData *sd, cudaStream_t s);
 bool stream_supported(const StreamData &sd, int n_types);
 // Bytes of scratch (256-byte aligned device memory, no contents expected) that a launch over graphs [first, first+count)
 // needs.  The scratch belongs to one launch: launches on different streams share nothing.

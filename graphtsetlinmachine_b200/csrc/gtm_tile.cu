@@ -787,7 +787,6 @@ int tile_data_create(TileData *td, const TileModel &tm, const DevModel &d, const
     td->tile_graph_host.clear();
     td->tile_graph = nullptr;
     td->gpos = nullptr;
-    td->stream = s;
     if (span) {
         td->graphs_per_tile = td->gmax = 1;
         td->n_tiles = (int)N;
@@ -835,17 +834,18 @@ int tile_data_create(TileData *td, const TileModel &tm, const DevModel &d, const
     GTM_CU(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
     int per_sm = 0;
     GTM_CU(cudaOccupancyMaxActiveBlocksPerMultiprocessorWithFlags(&per_sm, fn, td->threads, td->smem, 0));
-    if (per_sm < 1) { tile_data_destroy(td); return GTM_OK; }
+    if (per_sm < 1) { tile_data_destroy(td, s); return GTM_OK; }
     td->grid = std::max(1, std::min(sm_count * per_sm, td->n_tiles));
     td->n_graphs = N;
     td->supported = 1;
     return GTM_OK;
 }
 
-void tile_data_destroy(TileData *td)
+// s: a stream behind every kernel that reads the tables (the model's, which may not be the one they were made on).
+void tile_data_destroy(TileData *td, cudaStream_t s)
 {
-    if (td->tile_graph) cudaFreeAsync(td->tile_graph, td->stream);
-    if (td->gpos) cudaFreeAsync(td->gpos, td->stream);
+    if (td->tile_graph) cudaFreeAsync(td->tile_graph, s);
+    if (td->gpos) cudaFreeAsync(td->gpos, s);
     td->tile_graph = nullptr; td->gpos = nullptr;
     td->supported = 0;
 }

@@ -47,7 +47,6 @@ struct TileData {
     int *tile_graph = nullptr;          // [n_tiles+1] first graph of every tile (NULL for uniform sets)
     unsigned short *gpos = nullptr;     // [N] first node slot of every graph inside its tile (NULL for uniform sets)
     std::vector<int> tile_graph_host;
-    cudaStream_t stream = nullptr;
     int grid = 0;
     size_t smem = 0;
     int64_t n_graphs = 0;
@@ -58,7 +57,7 @@ void tile_model_destroy(TileModel *tm);
 int tile_model_refresh(TileModel *tm, const DevModel &d, cudaStream_t s);
 int tile_data_create(TileData *td, const TileModel &tm, const DevModel &d, const gtm_graphs_view *v, u32 n_min, u32 n_max,
                      int sm_count, cudaStream_t s);
-void tile_data_destroy(TileData *td);
+void tile_data_destroy(TileData *td, cudaStream_t s);
 bool tile_supported(const TileData &td, int n_types);
 // Bytes of scratch (256-byte aligned device memory, no contents expected) that a launch over graphs [first, first+count)
 // needs.  The scratch belongs to one launch: launches on different streams share nothing.

@@ -133,3 +133,30 @@ def test_lists_of_one_stream_on_the_next(engine_lib, depth):
     for ds in (large, small):
         tm.lib.gtm_dataset_destroy(ds)
     tm.close()
+
+
+@pytest.mark.parametrize("depth,max_nodes", [(1, 9), (2, 9)])
+def test_set_destroyed_behind_its_launch(engine_lib, depth, max_nodes):
+    """A set of ragged graphs, made on one stream, scored on another and destroyed at once: its tile tables outlive the launch,
+    although the next set is made on the first stream in the memory that became free."""
+    tm, base = learned(depth, clauses=3000, max_nodes=max_nodes)
+    first, second = torch.cuda.Stream(), torch.cuda.Stream()
+    order = [(np.arange(30000) * 13 + k) % 200 for k in range(2)]
+    want = resident(tm, base)[1]
+    outs = [sums(30000, tm) for _ in order]
+    torch.cuda.synchronize()
+    for _ in range(3):
+        for k, out in zip(order, outs):
+            _lib.check(tm.lib.gtm_set_stream(tm.model, C.c_void_p(first.cuda_stream)))
+            tm.ds, keep = C.c_void_p(), (tm.ds, tm.graphs, tm.number_of_graphs)
+            tm.set_graphs(base[k])
+            ds = tm.ds
+            tm.ds, tm.graphs, tm.number_of_graphs = keep
+            queue(tm, ds, second, out)
+            tm.lib.gtm_dataset_destroy(ds)
+        torch.cuda.synchronize()
+        for k, out in zip(order, outs):
+            assert np.array_equal(out.cpu().numpy(), want[k])
+            out.fill_(-77)
+        torch.cuda.synchronize()
+    tm.close()
