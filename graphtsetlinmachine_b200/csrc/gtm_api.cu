@@ -386,13 +386,16 @@ static void check_graph_span(const gtm_graphs_view *v, int64_t g_lo, int64_t g_h
         c.n_min = std::min(c.n_min, n);
         c.n_max = std::max(c.n_max, n);
     }
+    // a span is consistent in itself wherever it starts: its nodes and edges have to lie inside the arrays as well
+    const int64_t v_lo = v->node_index[g_lo], v_hi = g_hi < N ? (int64_t)v->node_index[g_hi] : v->total_nodes;
+    c.bad_index |= (u32)(v_hi > v->total_nodes);
     if (!c.bad_count && !c.bad_index) {          // node ranges are sound: the span's nodes
-        const int64_t v_lo = v->node_index[g_lo], v_hi = g_hi < N ? (int64_t)v->node_index[g_hi] : v->total_nodes;
         for (int64_t vi = v_lo; vi < v_hi; ++vi) {
             const uint64_t end = (uint64_t)v->edge_index[vi] + v->number_of_graph_node_edges[vi];
             const uint64_t want = vi + 1 < v->total_nodes ? (uint64_t)v->edge_index[vi + 1] : (uint64_t)v->total_edges;
             c.bad_edges |= (u32)(end != want);
         }
+        c.bad_edges |= (u32)(v_hi < v->total_nodes && (int64_t)v->edge_index[v_hi] > v->total_edges);
         for (int64_t vi = v_lo; vi < v_hi; ++vi) c.types |= v->node_type[vi];
     }
     *out = c;

@@ -94,6 +94,30 @@ def test_graph_arrays_are_validated_on_the_host():
     assert lib.gtm_validate_graphs(None) == 1
 
 
+def test_shifted_ranges_of_large_sets_are_refused():
+    """Spans of a large set are checked side by side.  Ranges that are shifted from some graph on are consistent within the
+    spans behind it, whose nodes must not be looked up where they say."""
+    lib = _lib.load()
+    graphs, per = 1200, 500                                       # 600,000 nodes: sixteen spans
+    nodes = graphs * per
+
+    def arrays():
+        return [np.zeros((nodes, 1), dtype=np.uint32), np.zeros(nodes, dtype=np.uint32), np.ones(nodes, dtype=np.uint32),
+                np.arange(nodes, dtype=np.uint32), np.zeros((nodes, 2), dtype=np.uint32),
+                (np.arange(graphs) * per).astype(np.uint32), np.full(graphs, per, dtype=np.uint32)]
+
+    assert lib.gtm_validate_graphs(C.byref(_view(arrays(), graphs, per))) == 0
+    for first, shift in [(1, 2 ** 30), (40, nodes), (graphs // 2, 2 ** 31), (graphs - 1, 2 ** 30)]:
+        bad = arrays()
+        bad[5][first:] += np.uint32(shift)
+        assert lib.gtm_validate_graphs(C.byref(_view(bad, graphs, per))) == 1
+        assert b"node_index" in lib.gtm_last_error()
+        bad = arrays()
+        bad[3][first * per:] += np.uint32(shift)
+        assert lib.gtm_validate_graphs(C.byref(_view(bad, graphs, per))) == 1
+        assert b"edge_index" in lib.gtm_last_error()
+
+
 def test_reference_graphs_pass_validation():
     import sys
     sys.path.insert(0, os.path.join(ROOT, "tests"))

@@ -96,6 +96,32 @@ def test_pipelined_chunks(engine_lib, n, nodes, depth):
     gpu.close()
 
 
+@pytest.mark.parametrize("depth", [1, 2])
+@pytest.mark.parametrize("first", [3, 8000])
+def test_shifted_ranges_are_refused_chunk_by_chunk(engine_lib, depth, first):
+    """A set that goes up in chunks is checked chunk by chunk, each before it is copied; the model scores on."""
+    rng = np.random.default_rng(first)
+    np.random.seed(6)
+    base = random_graphs(300, rng, hv_size=128, max_nodes=4, max_degree=2)
+    base.edge[:, 0] = 0
+    kw = dict(clauses=200, classes=9, literals=256, threshold=50, s=3.0, depth=depth, message_size=64, max_nodes=4, seed=2,
+              hypervectors=np.stack([rng.choice(64, size=2, replace=False) for _ in range(200)]).astype(np.uint32))
+    gpu = EngineTM(**kw)
+    gpu.set_graphs(base)
+    gpu.prepare()
+    want = np.resize(gpu.score(), (16000, 9))
+    for name, shift in [("node_index", 2 ** 30), ("edge_index", 2 ** 30)]:
+        graphs = base[np.arange(16000) % 300]
+        at = first if name == "node_index" else int(graphs.node_index[first])
+        array = np.array(getattr(graphs, name))
+        array[at:] += np.uint32(shift)
+        setattr(graphs, name, array)
+        with pytest.raises(Exception, match=name):
+            scored_create(gpu, graphs)
+    assert np.array_equal(scored_create(gpu, base[np.arange(16000) % 300]), want)
+    gpu.close()
+
+
 def test_results_outlive_the_pool(engine_lib):
     """An array in recycled page-locked memory keeps its memory while it, or a view of it, is alive."""
     for _ in range(4 * hostmem.PER_BLOCK):                       # a size's first arrays are ordinary memory
