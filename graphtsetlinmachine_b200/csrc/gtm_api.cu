@@ -75,17 +75,29 @@ extern "C" int gtm_device_count(int *count_out)
     return GTM_OK;
 }
 
+// Calls without a model, from a thread that may be new to CUDA: on a device that a model lives on, if there is one, instead of
+// on device 0, where a context would be made.
+static int bind_any()
+{
+    const int device = stage_device();
+    if (device >= 0) GTM_CU(cudaSetDevice(device));
+    return GTM_OK;
+}
+
 extern "C" int gtm_host_alloc(uint64_t bytes, void **out)
 {
     if (!out) return fail(GTM_ERR_ARG, "out is null");
     *out = nullptr;
+    GTM_TRY(bind_any());
     GTM_CU(cudaHostAlloc(out, (size_t)std::max<uint64_t>(bytes, 1), cudaHostAllocPortable));
     return GTM_OK;
 }
 
 extern "C" int gtm_host_free(void *p)
 {
-    if (p) GTM_CU(cudaFreeHost(p));
+    if (!p) return GTM_OK;
+    GTM_TRY(bind_any());
+    GTM_CU(cudaFreeHost(p));
     return GTM_OK;
 }
 
@@ -130,7 +142,7 @@ extern "C" int gtm_create(const gtm_config *cfg, gtm_model **out)
     GTM_CU(cudaGetDeviceProperties(&prop, cfg->device));
     m->sm_count = prop.multiProcessorCount;
     { int st0 = pool_prepare(cfg->device); if (st0 != GTM_OK) { delete m; return st0; } }
-    stage_retain();                  // given back by gtm_destroy
+    stage_retain(cfg->device);       // given back by gtm_destroy
 
     int st = GTM_OK;
     st = dev_alloc(&d.ta0, (size_t)d.C * d.SB * d.L0);
@@ -144,9 +156,9 @@ extern "C" int gtm_create(const gtm_config *cfg, gtm_model **out)
     if (st == GTM_OK) st = dev_alloc(&m->class_sum_tap, (size_t)d.K);
     if (st == GTM_OK) st = dev_alloc(&m->barrier, 1);
     if (st == GTM_OK) st = dev_alloc(&m->error, 1);
-    if (st == GTM_OK && cudaMallocHost((void **)&m->score_error, sizeof(int)) != cudaSuccess) st = fail(GTM_ERR_OOM, "page-locked host allocation failed");
+    if (st == GTM_OK && cudaMallocHost((void **)&m->score_error, sizeof(int)) != cudaSuccess) { cudaGetLastError(); st = fail(GTM_ERR_OOM, "page-locked host allocation failed"); }
     if (st == GTM_OK) st = dev_alloc(&m->phase_cycles, 8);
-    if (st == GTM_OK && cudaEventCreateWithFlags(&m->queued, cudaEventDisableTiming) != cudaSuccess) st = fail(GTM_ERR_CUDA, "an event could not be created");
+    if (st == GTM_OK && cudaEventCreateWithFlags(&m->queued, cudaEventDisableTiming) != cudaSuccess) { cudaGetLastError(); st = fail(GTM_ERR_CUDA, "an event could not be created"); }
     if (st != GTM_OK) { gtm_destroy(m); return st; }
     d.hv = hv;
     m->hv_host.assign((size_t)d.C * d.MB, 0);
@@ -443,7 +455,7 @@ static int check_view(const gtm_graphs_view *v)
 extern "C" int gtm_validate_graphs(const gtm_graphs_view *v)
 {
     GTM_TRY(check_view(v));
-    struct Keep { Keep() { stage_retain(); } ~Keep() { stage_drop(); } } keep;      // the copy threads stay while they check
+    struct Keep { Keep() { stage_retain(-1); } ~Keep() { stage_drop(); } } keep;      // the copy threads stay while they check
     return validate_graphs(v, 0, v->number_of_graphs);
 }
 

@@ -26,12 +26,16 @@ inline int fail(int code, const char *fmt, ...)
     return code;
 }
 
+// A failed call is reported here and nowhere else: cudaGetLastError() takes it back, or the check behind the next kernel
+// launch would report it again.
 #define GTM_CU(call)                                                                              \
     do {                                                                                          \
         cudaError_t e_ = (call);                                                                  \
-        if (e_ != cudaSuccess)                                                                    \
+        if (e_ != cudaSuccess) {                                                                  \
+            cudaGetLastError();                                                                   \
             return fail(e_ == cudaErrorMemoryAllocation ? GTM_ERR_OOM : GTM_ERR_CUDA, "%s failed: %s", #call, \
                         cudaGetErrorString(e_));                                                  \
+        }                                                                                         \
     } while (0)
 
 #define GTM_TRY(call)            \

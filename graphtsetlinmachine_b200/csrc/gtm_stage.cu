@@ -97,7 +97,7 @@ struct CopyPool {
 constexpr int kLanesKept = 2;
 
 std::mutex g_lock;                               // guards what follows
-int g_users = 0;
+int g_users = 0, g_device = -1;
 CopyPool *g_pool = nullptr;                      // plain pointers: nothing is torn down behind a process that just exits
 std::vector<StageLane *> *g_lanes = nullptr;     // free lanes
 
@@ -238,10 +238,17 @@ void lane_release(StageLane *lane)
     lane_destroy(lane);
 }
 
-void stage_retain()
+void stage_retain(int device)
 {
     std::lock_guard<std::mutex> hold(g_lock);
     ++g_users;
+    if (device >= 0) g_device = device;
+}
+
+int stage_device()
+{
+    std::lock_guard<std::mutex> hold(g_lock);
+    return g_device;
 }
 
 void stage_drop()
@@ -251,6 +258,7 @@ void stage_drop()
     {
         std::lock_guard<std::mutex> hold(g_lock);
         if (--g_users > 0) return;
+        g_device = -1;
         if (g_lanes) lanes.swap(*g_lanes);
         pool = g_pool;
         g_pool = nullptr;

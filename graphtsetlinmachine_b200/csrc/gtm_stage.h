@@ -42,11 +42,13 @@ struct StageLane {
 };
 
 // A lane of the device, from the free list or new.  At most kLanesKept lanes per device stay on the list; all of them,
-// and the copy threads, are given back when the last model is destroyed (stage_retain / stage_drop).
+// and the copy threads, are given back when the last model is destroyed (stage_retain / stage_drop).  stage_device: the
+// device of the model made last, -1 when there is none; stage_retain(-1) names no device.
 int lane_acquire(int device, StageLane **out);
 void lane_release(StageLane *lane);
-void stage_retain();
+void stage_retain(int device);
 void stage_drop();
+int stage_device();
 
 struct LaneGuard {
     StageLane *lane = nullptr;

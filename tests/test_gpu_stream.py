@@ -136,3 +136,20 @@ def test_results_outlive_the_pool(engine_lib):
     assert b.ctypes.data != address and (view == 7).all()
     del view
     assert hostmem.empty((1000, 100), np.int32).ctypes.data == address
+
+
+def test_memory_that_cannot_be_locked(engine_lib):
+    """A failed page-lock is an error of its own call; the calls behind it, whose launches succeed, are not blamed for it."""
+    rng = np.random.default_rng(3)
+    np.random.seed(3)
+    graphs = random_graphs(40, rng, hv_size=20, max_nodes=3)
+    gpu = EngineTM(clauses=30, classes=3, literals=40, threshold=50, s=3.0, max_nodes=3)
+    gpu.set_graphs(graphs)
+    gpu.prepare()
+    want = gpu.score()
+    p = C.c_void_p()
+    assert engine_lib.gtm_host_alloc(1 << 50, C.byref(p)) in (2, 3) and not p.value
+    gpu.prepare()                                                 # a launch with a check behind it
+    assert engine_lib.gtm_host_alloc(1 << 50, C.byref(p)) in (2, 3)
+    assert np.array_equal(scored_create(gpu, graphs), gpu.score()) and gpu.score().shape == want.shape
+    gpu.close()
