@@ -103,7 +103,6 @@ void stage_drop()
     {
         std::lock_guard<std::mutex> hold(g_lock);
         if (--g_users > 0) return;
-        g_device = -1;
         lanes = g_lanes;
         g_lanes = nullptr;
     }

@@ -34,7 +34,7 @@ struct StageLane {
 
 // A lane of the device, from the free list or new.  At most kLanesKept lanes per device stay on the list; all of them are
 // given back when the last model is destroyed (stage_retain / stage_drop).  stage_device: the device of the model made
-// last, -1 when there is none.
+// last, -1 before the first.
 int lane_acquire(int device, StageLane **out);
 void lane_release(StageLane *lane);
 void stage_retain(int device);

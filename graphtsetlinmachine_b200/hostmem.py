@@ -4,7 +4,10 @@ A result of a few megabytes in a fresh numpy array costs a page fault per page a
 page-locked memory the copy engine writes it directly, in the time of the transfer.  Page-locking is slow (0.5 ms per MB),
 so the memory of an array that nobody refers to any more is kept for the next result, and a block is locked only for
 every eighth array of a size that is asked for: a program's first results are ordinary arrays, and what locking costs is
-spread over many.
+spread over many.  Free blocks are given back when the last model is closed, blocks in use when their arrays go after that.
+
+An array in a block does not own its data, which shows in ``flags.owndata`` and in that it cannot be resized in place; a copy
+of it can.
 """
 
 import collections
@@ -26,6 +29,8 @@ _blocks = collections.Counter()                         # size class -> blocks l
 _free = collections.defaultdict(collections.deque)      # size class -> addresses
 _lock = threading.Lock()
 _locked = 0
+_models = set()                                         # handles of open models (set operations are atomic)
+_keep = True                                            # blocks that come back are kept: not once the last model has closed
 
 
 def _size_class(nbytes):
@@ -36,11 +41,50 @@ def _size_class(nbytes):
 
 def _give_back(address, size):
     _free[size].append(address)             # atomic: may run in the garbage collector of any thread
+    if not _keep:
+        _drain()
+
+
+def _drain():
+    """Frees unused blocks.  Not while another thread, or the code that the garbage collector interrupted, is at it: they then
+    wait for the next occasion."""
+    if _lock.acquire(blocking=False):
+        try:
+            _drain_locked(0)
+        finally:
+            _lock.release()
+
+
+def _drain_locked(limit):
+    """Frees unused blocks until at most `limit` bytes are locked; the caller holds the lock."""
+    global _locked
+    for size, blocks in list(_free.items()):
+        while blocks and _locked > limit:
+            try:
+                address = blocks.popleft()
+            except IndexError:
+                break
+            _lib.load().gtm_host_free(address)
+            _locked -= size
+            _blocks[size] -= 1
+
+
+def model_opened(handle):
+    _models.add(handle)
+
+
+def model_closed(handle):
+    """May run in the garbage collector of any thread."""
+    global _keep
+    _models.discard(handle)
+    if not _models:
+        _keep = False
+        _drain()
 
 
 def _take(size):
     """Address of a free block, or a newly locked one while the limit allows; 0 when it does not."""
-    global _locked
+    global _locked, _keep
     try:
         return _free[size].popleft()
     except IndexError:
@@ -49,16 +93,7 @@ def _take(size):
     with _lock:
         if (_blocks[size] + 1) * PER_BLOCK > _asked[size]:
             return 0
-        if _locked + size > MOST:           # free blocks of other sizes make room
-            for other, blocks in list(_free.items()):
-                while blocks and _locked + size > MOST:
-                    try:
-                        address = blocks.popleft()
-                    except IndexError:
-                        break
-                    lib.gtm_host_free(address)
-                    _locked -= other
-                    _blocks[other] -= 1
+        _drain_locked(MOST - size)          # free blocks of other sizes make room
         if _locked + size > MOST:
             return 0
         out = C.c_void_p()
@@ -66,6 +101,7 @@ def _take(size):
             return 0
         _locked += size
         _blocks[size] += 1
+        _keep = True
         return out.value
 
 

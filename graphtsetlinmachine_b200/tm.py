@@ -170,6 +170,7 @@ class CommonTsetlinMachine:
                 ds.close()
         self._train_set = self._test_set = None
         if self._model:
+            hostmem.model_closed(self._model.value)
             self._lib.gtm_destroy(self._model)
             self._model = C.c_void_p()
 
@@ -256,6 +257,7 @@ class CommonTsetlinMachine:
             cfg.s[d] = float(v)
         cfg.seed = self.seed
         _lib.check(self._lib.gtm_create(C.byref(cfg), C.byref(self._model)))
+        hostmem.model_opened(self._model.value)
         _lib.check(self._lib.gtm_set_hypervectors(self._model, _ptr(_u32(self.hypervectors))))
 
     def _init(self, graphs):
@@ -338,7 +340,8 @@ class CommonTsetlinMachine:
 
     def _score(self, graphs, out=None):
         """tm.py:786-812: raw class sums int32[N][outputs]; one batched launch instead of a per-graph loop.
-        `out` (optional, C-contiguous int32[N][outputs], e.g. page-locked) receives the result in place."""
+        `out` (optional, C-contiguous int32[N][outputs], e.g. page-locked) receives the result in place; an array made here may
+        lie in recycled page-locked memory (see hostmem): copy it to resize it in place."""
         if not self.initialized:
             print("Error: Model not trained.")
             sys.exit(-1)

@@ -153,3 +153,34 @@ def test_memory_that_cannot_be_locked(engine_lib):
     assert engine_lib.gtm_host_alloc(1 << 50, C.byref(p)) in (2, 3)
     assert np.array_equal(scored_create(gpu, graphs), gpu.score()) and gpu.score().shape == want.shape
     gpu.close()
+
+
+def test_locked_memory_goes_with_the_last_model(engine_lib):
+    """Free blocks are given back when the last model is closed; a block in use stays until its array goes."""
+    import gc
+
+    from graphtsetlinmachine_b200.tm import MultiClassGraphTsetlinMachine
+    gc.collect()
+    np.random.seed(4)
+    graphs = random_graphs(8, np.random.default_rng(4), hv_size=16, max_nodes=3)
+    models = [MultiClassGraphTsetlinMachine(20, 50, 2.0, depth=1) for _ in range(2)]
+    for tm in models:
+        tm.fit(graphs, np.arange(8, dtype=np.uint32) % 2, epochs=1)
+    others = len(hostmem._models) - 2
+    shape = (1 << 17, 3)
+    kept = [hostmem.empty(shape, np.int32) for _ in range(3 * hostmem.PER_BLOCK)]
+    locked = hostmem._locked
+    assert locked >= 3 * kept[0].nbytes
+    held = next(a for a in kept if not a.flags.owndata)
+    held[...] = 5
+    del kept
+    models[0]._release()
+    assert hostmem._locked == locked
+    models[1]._release()
+    models[1]._release()                                         # once is enough
+    if others == 0:
+        assert held.nbytes <= hostmem._locked < 2 * held.nbytes and (held == 5).all()
+        del held
+        assert hostmem._locked == 0 and not any(hostmem._free.values())
+    a = hostmem.empty(shape, np.int32)                           # and the module serves on
+    a[...] = 1
