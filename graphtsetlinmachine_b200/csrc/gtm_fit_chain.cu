@@ -112,6 +112,24 @@ static int chain_prepare(gtm_model *m, gtm_dataset *ds, int rw)
 
 struct ChainPlan { bool ok = false, hybrid = false; int rw = 0, grid = 0, threads = 0; size_t smem = 0; ChainArgs a; };
 
+// Whether one CTA learns the model alone.  It saves the grid-wide steps (one per graph, two per message layer, about 2,000
+// cycles each) and the rounds of a few CTAs over many message bits, and pays with more than a clause per warp (16 warps) and
+// with graphs that grow.  Measured on one B200, us a graph, one CTA / a CTA per clause:
+//   messages, up to 16 clauses: 10 clauses, 12 nodes 10.0 / 12.4; 16 clauses, 90 nodes 11.8 / 11.6; 16 clauses, 200 nodes, 64
+//     message bits 13.4 / 12.8, 512 bits 19.8 / 20.3; 16 clauses, 500 nodes 17.2 / 12.9 and 33.9 / 20.3;
+//   messages, more clauses: 24 clauses, 3 nodes 11.8 / 10.9, 12 nodes 13.9 / 12.6; 60 clauses, 500 nodes 38.4 / 12.4;
+//   the same on graphs of a few nodes when s = 1, which leaves no masks to draw: 20 clauses 8.5 / 11.4, 32 clauses 9.2 / 9.5, 48
+//     clauses 11.9 / 9.5;
+//   no messages: 4 clauses 3.5 / 3.5 (images), 4.3 / 4.8 (90 nodes); 8 clauses 3.9 / 3.6, 4.6 / 4.8; 32 clauses 8.5 / 3.9, 9.4 / 5.3.
+static bool learned_by_one_cta(const DevModel &d, int max_nodes)
+{
+    if (d.D == 1) return d.C <= 4;
+    bool no_masks = true;
+    for (int l = 0; l < d.D; ++l) no_masks = no_masks && d.p_mask[l] >= 1.0f;
+    if (no_masks && max_nodes <= kChainRowWise) return d.C <= 32;
+    return d.C <= 16 && max_nodes <= 256;
+}
+
 static ChainPlan plan_chain(const gtm_model *m, const gtm_dataset *ds)
 {
     const DevModel &d = m->dm;
@@ -132,10 +150,8 @@ static ChainPlan plan_chain(const gtm_model *m, const gtm_dataset *ds)
         a.spec_rounds = d.p_mask[0] >= 1.0f ? 0 : std::min(2, (d.K + 3 + 32 * words_all + 127) / 128);
         a.pre_words = (std::max(4 * a.spec_rounds, (d.K + 3) / 32 + 1 + std::min(d.K, 4) * words_all) + 4 + 7) & ~3;
     }
-    // One CTA learns a model of few clauses alone: every grid-wide step (about 2,000 cycles; one per graph, and two per
-    // message layer) costs more than a second or third clause per warp.
     int cpc = m->opt_fit_block_clauses;
-    if (cpc <= 0) cpc = d.C <= (d.D > 1 ? 64 : 32) ? d.C : (d.C + m->sm_count - 1) / m->sm_count;
+    if (cpc <= 0) cpc = learned_by_one_cta(d, ds->max_nodes) ? d.C : (d.C + m->sm_count - 1) / m->sm_count;
     for (int attempt = 0; attempt < 2; ++attempt) {
         const int grid = (d.C + cpc - 1) / cpc;
         const bool solo = grid == 1;

@@ -98,3 +98,17 @@ def test_clause_ranges(engine_lib, per_cta):
     graphs = random_graphs(20, rng, hv_size=30, max_nodes=12, edge_types=2)
     kw = model(rng, clauses=60, classes=3, hv=30, depth=2, ms=64, max_nodes=12, seed=4)
     agree(kw, graphs, 3, 8, options={"fit_block_clauses": per_cta})
+
+
+@pytest.mark.parametrize("clauses,depth,nodes,s", [
+    (4, 1, 3, 2.5), (5, 1, 3, 2.5),                             # no messages
+    (16, 2, 30, 2.5), (17, 2, 30, 2.5), (16, 3, 256, 2.5), (16, 2, 257, 2.5),
+    (32, 2, 3, 1.0), (33, 2, 3, 1.0), (32, 2, 4, 1.0),          # few nodes and no masks to draw
+])
+def test_one_cta_or_many(engine_lib, clauses, depth, nodes, s):
+    """Both sides of the lines of the rule that has one CTA learn a model alone."""
+    rng = np.random.default_rng(nodes)
+    np.random.seed(clauses)
+    graphs = random_graphs(6, rng, hv_size=20, fixed_nodes=nodes, max_nodes=nodes, edge_types=2, max_degree=2)
+    kw = model(rng, clauses=clauses, classes=3, hv=20, depth=depth, ms=70, s=s, max_nodes=nodes, seed=9)
+    agree(kw, graphs, 3, 7)
