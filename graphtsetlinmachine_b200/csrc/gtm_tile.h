@@ -41,6 +41,7 @@ struct TileData {
     int pw = 0;                         // node words of a literal row: TNC, or planes of 8 (span)
     bool span = false;                  // graphs of more than 128 nodes: a tile is one graph
     int threads = 0;                    // of a CTA
+    bool plain = false;                 // class sums are the plain kernel's work (see tile_score_kernel)
     int uniform_n = 0;                  // > 0: every graph has this many nodes: slots follow from the graph number
     int graphs_per_tile = 0;            // uniform sets: graphs per tile (no tile table)
     int n_tiles = 0;
