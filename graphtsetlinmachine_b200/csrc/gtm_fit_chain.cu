@@ -217,7 +217,10 @@ int launch_fit_chain(gtm_model *m, gtm_dataset *ds, int n_types, const int *Y_de
     g.n_types = n_types;
     DevModel dm = d;
     const void *fn = chain_kernel_for(plan.rw, d.D == 1, plan.hybrid, plan.a.narrow != 0);
-    GTM_CU(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)plan.smem));
+    // the limit belongs to the kernel: set to this plan's size, another model's fit in another thread could lower it before the launch
+    cudaFuncAttributes fa;
+    GTM_CU(cudaFuncGetAttributes(&fa, fn));
+    GTM_CU(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024 - (int)fa.sharedSizeBytes));
     void *args[] = {&dm, &g, &a};
     GTM_CU(cudaLaunchCooperativeKernel(fn, dim3(plan.grid), dim3(plan.threads), args, plan.smem, m->stream));
     *done = 1;

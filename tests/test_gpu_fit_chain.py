@@ -112,3 +112,44 @@ def test_one_cta_or_many(engine_lib, clauses, depth, nodes, s):
     graphs = random_graphs(6, rng, hv_size=20, fixed_nodes=nodes, max_nodes=nodes, edge_types=2, max_degree=2)
     kw = model(rng, clauses=clauses, classes=3, hv=20, depth=depth, ms=70, s=s, max_nodes=nodes, seed=9)
     agree(kw, graphs, 3, 7)
+
+
+def test_two_models_in_two_threads(engine_lib):
+    """Models of one kernel variant and different shared-memory plans, learned in two threads: as each learns alone."""
+    import threading
+
+    rng = np.random.default_rng(12)
+    np.random.seed(12)
+    jobs = []
+    for clauses in (150, 900):
+        graphs = random_graphs(12, rng, hv_size=60, max_nodes=3, max_degree=2)
+        kw = model(rng, clauses=clauses, classes=3, hv=60, depth=2, ms=60, max_nodes=3, seed=clauses)
+        encY = encode_labels(rng.integers(0, 3, size=12), 3, kw["threshold"])
+        tms = [EngineTM(**kw) for _ in range(2)]
+        for tm in tms:
+            tm.set_graphs(graphs)
+            tm.prepare()
+        for _ in range(60):
+            tms[0].fit(encY)
+        jobs.append((tms, encY))
+    errors = []
+
+    def learn(tm, encY):
+        try:
+            for _ in range(60):
+                tm.fit(encY)
+        except Exception as e:
+            errors.append(e)
+
+    threads = [threading.Thread(target=learn, args=(tms[1], encY)) for tms, encY in jobs]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not errors
+    for (alone, beside), _ in jobs:
+        a, b = state_of(alone, 2), state_of(beside, 2)
+        assert np.array_equal(a["ta_state"], b["ta_state"]) and np.array_equal(a["message_ta_state"][0], b["message_ta_state"][0])
+        assert np.array_equal(a["clause_weights"], b["clause_weights"]) and np.array_equal(a["draws"], b["draws"])
+        alone.close()
+        beside.close()
