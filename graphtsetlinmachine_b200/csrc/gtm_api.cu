@@ -803,10 +803,11 @@ static bool scores_by_stream(gtm_model *m, gtm_dataset *ds, int n_types)
 }
 
 // The option that forces the tile kernel stands for tiles of several graphs and one pass of the votes, and is an error beyond.
+// So are tiles that a set got for its first transform: the option is to be set before the set is made.
 static bool scores_by_tile(gtm_model *m, gtm_dataset *ds, int n_types)
 {
     if (!tile_supported(ds->td, n_types)) return false;
-    return m->opt_score_kernel == 0 || (m->opt_score_kernel == 3 && !ds->td.span && m->dm.K <= 16);
+    return m->opt_score_kernel == 0 || (m->opt_score_kernel == 3 && !ds->td.span && m->dm.K <= 16 && !ds->tiles_tried);
 }
 
 // One launch of a tiled kernel; clause_out_dev: the tile kernel only.  Its scratch belongs to the launch alone: kept with the

@@ -4,6 +4,8 @@
 import numpy as np
 import pytest
 
+from graphtsetlinmachine_b200 import _lib
+
 from oracle.oracle import OracleTM
 from util import EngineTM, encode_labels, random_graphs
 
@@ -59,3 +61,24 @@ def test_class_counts(engine_lib, classes, max_nodes):
 @pytest.mark.parametrize("classes", [2, 19])
 def test_transform_of_models_without_message_layers(engine_lib, fixed, classes):
     compare(150, 7 + classes, clauses=101, classes=classes, hv=33, depth=1, ms=32, max_nodes=fixed or 9, node_types=1, fixed=fixed)
+
+
+def test_tiles_of_a_transform_do_not_serve_the_forced_kernel(engine_lib):
+    """A set of a model without message layers that came without tiles gets them on its first transform; forcing the tile kernel
+    afterwards stays an error, as it is without the transform."""
+    rng = np.random.default_rng(8)
+    np.random.seed(8)
+    graphs = random_graphs(30, rng, hv_size=20, max_nodes=4)
+    gpu = EngineTM(clauses=40, classes=3, literals=40, threshold=50, s=3.0, max_nodes=4)
+    gpu.set_graphs(graphs)
+    gpu.prepare()
+    want = gpu.score()
+    for transformed in (False, True):
+        if transformed:
+            assert np.array_equal(gpu.transform()[1], want)
+        _lib.check(engine_lib.gtm_set_option(gpu.model, b"score_kernel", 3))
+        with pytest.raises(_lib.GtmError):
+            gpu.score()
+        _lib.check(engine_lib.gtm_set_option(gpu.model, b"score_kernel", 0))
+        assert np.array_equal(gpu.score(), want)
+    gpu.close()
