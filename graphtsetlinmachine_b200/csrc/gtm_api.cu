@@ -66,6 +66,16 @@ static u32 *layer_planes(const gtm_model *m, int layer)
     return layer == 0 ? d.ta0 : d.tam + (size_t)(layer - 1) * d.C * d.SB * d.M;
 }
 
+// The host reads and writes callers' arrays itself where the driver once copied all of them: device memory is refused here, as
+// the driver refused it.
+static int check_on_host(const void *p, const char *what)
+{
+    cudaPointerAttributes at;
+    if (!p) return GTM_OK;
+    if (cudaPointerGetAttributes(&at, p) != cudaSuccess) { cudaGetLastError(); return GTM_OK; }
+    return at.type == cudaMemoryTypeDevice ? fail(GTM_ERR_ARG, "%s is in device memory, not in host memory", what) : GTM_OK;
+}
+
 // --------------------------------------------------------------------------------------------- library
 extern "C" const char *gtm_version(void) { return "gtm_b200 0.1 (sm_100a)"; }
 extern "C" const char *gtm_last_error(void) { return gtm_error_text().c_str(); }
@@ -270,6 +280,7 @@ extern "C" int gtm_get_ta_state(gtm_model *m, int layer, uint32_t *out)
     GTM_TRY(bind(m));
     GTM_TRY(check_layer(m, layer));
     if (!out) return fail(GTM_ERR_ARG, "ta_state_out is null");
+    GTM_TRY(check_on_host(out, "ta_state_out"));
     const DevModel &d = m->dm;
     const int W = layer_words(m, layer);
     const size_t total = (size_t)d.C * d.SB * W;
@@ -441,6 +452,17 @@ static int validate_graphs(const gtm_graphs_view *v, int64_t g_lo, int64_t g_hi,
     if (all.bad_edges) return fail(GTM_ERR_ARG, "edge_index is not the running sum of number_of_graph_node_edges (or exceeds total_edges)");
     if (all_out) *all_out = all;
     return GTM_OK;
+}
+
+static int check_view_on_host(const gtm_graphs_view *v)
+{
+    GTM_TRY(check_on_host(v->X, "X"));
+    GTM_TRY(check_on_host(v->node_type, "node_type"));
+    GTM_TRY(check_on_host(v->number_of_graph_node_edges, "number_of_graph_node_edges"));
+    GTM_TRY(check_on_host(v->edge_index, "edge_index"));
+    GTM_TRY(check_on_host(v->edge, "edge"));
+    GTM_TRY(check_on_host(v->node_index, "node_index"));
+    return check_on_host(v->number_of_graph_nodes, "number_of_graph_nodes");
 }
 
 static int check_view(const gtm_graphs_view *v)
@@ -675,6 +697,7 @@ extern "C" int gtm_dataset_create(gtm_model *m, const gtm_graphs_view *v, gtm_da
     if (!v || !out) return fail(GTM_ERR_ARG, "null argument");
     *out = nullptr;
     GTM_TRY(check_view(v));
+    GTM_TRY(check_view_on_host(v));
     LaneGuard guard;
     GTM_TRY(lane_acquire(m->cfg.device, &guard.lane));
     GTM_TRY(dataset_create(m, v, out, SetCopy::whole, guard.lane));
@@ -975,6 +998,7 @@ extern "C" int gtm_score(gtm_model *m, gtm_dataset *ds, int n_types, int64_t fir
     GTM_TRY(check_range(m, ds, n_types, first, count));
     if (count == 0) return GTM_OK;
     if (!out) return fail(GTM_ERR_ARG, "class_sums_out is null");
+    GTM_TRY(check_on_host(out, "class_sums_out"));
     LaneGuard guard;
     GTM_TRY(lane_acquire(m->cfg.device, &guard.lane));
     return score_to_host(m, ds, n_types, first, count, out, guard.lane);
@@ -992,6 +1016,8 @@ extern "C" int gtm_dataset_create_scored(gtm_model *m, const gtm_graphs_view *v,
     if (!m->has_state) return fail(GTM_ERR_STATE, "model has no state: call gtm_init_state or gtm_set_ta_state first");
     if (n_types < 1) return fail(GTM_ERR_ARG, "number_of_node_types must be positive");
     GTM_TRY(check_view(v));
+    GTM_TRY(check_view_on_host(v));
+    GTM_TRY(check_on_host(out, "class_sums_out"));
     LaneGuard guard;
     GTM_TRY(lane_acquire(m->cfg.device, &guard.lane));
     // what a tiled kernel may cover; stream_supported / tile_supported decide once the tiles are made
@@ -1046,6 +1072,9 @@ static int transform_common(gtm_model *m, gtm_dataset *ds, int n_types, int64_t 
     GTM_TRY(bind(m));
     GTM_TRY(check_range(m, ds, n_types, first, count));
     if (count == 0) return GTM_OK;
+    GTM_TRY(check_on_host(clause_out, "clause_outputs_out"));
+    GTM_TRY(check_on_host(node_out, "node_outputs_out"));
+    GTM_TRY(check_on_host(sums_out, "class_sums_out"));
     int *sums_dev = nullptr, *co_dev = nullptr, *no_dev = nullptr;
     const size_t n_sums = (size_t)count * m->dm.K, n_co = (size_t)count * m->dm.C, n_no = n_co * (size_t)node_stride;
     LaneGuard guard;

@@ -184,3 +184,37 @@ def test_locked_memory_goes_with_the_last_model(engine_lib):
         assert hostmem._locked == 0 and not any(hostmem._free.values())
     a = hostmem.empty(shape, np.int32)                           # and the module serves on
     a[...] = 1
+
+
+@pytest.mark.parametrize("n", [40, 30000])                        # packed in one copy / in chunks
+def test_device_memory_is_refused_where_host_memory_is_meant(engine_lib, n):
+    import torch
+
+    rng = np.random.default_rng(n)
+    np.random.seed(1)
+    graphs = random_graphs(40, rng, hv_size=20, max_nodes=3)[np.arange(n) % 40]
+    gpu = EngineTM(clauses=30, classes=3, literals=40, threshold=50, s=3.0, max_nodes=3)
+    gpu.set_graphs(graphs)
+    gpu.prepare()
+    want = gpu.score()
+    dev = torch.zeros(max(n * 30, 30 * 2 * 8), dtype=torch.int32, device="cuda")
+    p = C.c_void_p(dev.data_ptr())
+    refused = lambda status: status == 1 and b"device memory" in engine_lib.gtm_last_error()
+    assert refused(engine_lib.gtm_score(gpu.model, gpu.ds, 1, 0, n, p))
+    assert refused(engine_lib.gtm_transform(gpu.model, gpu.ds, 1, 0, n, p, None))
+    assert refused(engine_lib.gtm_get_ta_state(gpu.model, 0, p))
+    arrays = [np.ascontiguousarray(a, dtype=np.uint32) for a in (graphs.X, graphs.node_type, graphs.number_of_graph_node_edges, graphs.edge_index,
+                                                                 graphs.edge, graphs.node_index, graphs.number_of_graph_nodes)]
+    copies = [torch.from_numpy(a.view(np.int32)).cuda() for a in arrays]
+    names = ("X", "node_type", "number_of_graph_node_edges", "edge_index", "edge", "node_index", "number_of_graph_nodes")
+    out, ds = np.zeros((n, 3), dtype=np.int32), C.c_void_p()
+    for name, copy in zip(names, copies):
+        v = _lib.GraphsView()
+        for field, a in zip(names, arrays):
+            setattr(v, field, a.ctypes.data)
+        setattr(v, name, copy.data_ptr())
+        v.number_of_graphs, v.total_nodes, v.total_edges, v.max_number_of_graph_nodes = n, len(arrays[0]), len(arrays[4]), 3
+        assert refused(engine_lib.gtm_dataset_create(gpu.model, C.byref(v), C.byref(ds))) and not ds.value
+        assert refused(engine_lib.gtm_dataset_create_scored(gpu.model, C.byref(v), 1, out.ctypes.data, C.byref(ds))) and not ds.value
+    assert np.array_equal(gpu.score(), want)
+    gpu.close()
