@@ -1270,6 +1270,14 @@ extern "C" int gtm_debug_fit_phase_cycles(gtm_model *m, uint64_t *cycles_out)
     return GTM_OK;
 }
 
+extern "C" int gtm_debug_last_fit_kernel(gtm_model *m, int32_t *info_out)
+{
+    GTM_TRY(bind(m));
+    if (!info_out) return fail(GTM_ERR_ARG, "info_out is null");
+    memcpy(info_out, m->last_fit, sizeof m->last_fit);
+    return GTM_OK;
+}
+
 extern "C" int gtm_debug_last_feedback(gtm_model *m, int32_t *clause_node_out, int32_t *update_out)
 {
     GTM_TRY(bind(m));

@@ -224,6 +224,8 @@ int launch_fit_chain(gtm_model *m, gtm_dataset *ds, int n_types, const int *Y_de
     void *args[] = {&dm, &g, &a};
     GTM_CU(cudaLaunchCooperativeKernel(fn, dim3(plan.grid), dim3(plan.threads), args, plan.smem, m->stream));
     *done = 1;
+    const int info[6] = {2, plan.grid, plan.rw, plan.hybrid, plan.a.narrow != 0, a.solo != 0};
+    memcpy(m->last_fit, info, sizeof info);
     int err = 0;
     GTM_CU(cudaMemcpyAsync(&err, a.error, sizeof(int), cudaMemcpyDeviceToHost, m->stream));
     GTM_CU(cudaStreamSynchronize(m->stream));

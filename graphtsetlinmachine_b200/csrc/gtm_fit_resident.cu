@@ -734,6 +734,10 @@ int launch_fit(gtm_model *m, gtm_dataset *ds, int n_types, const int *Y_dev, int
         void *args[] = {&dm, &g, &sc, &a, &eval_only};
         GTM_CU(cudaLaunchCooperativeKernel(fn, dim3(grid), dim3(block), args, smem, m->stream));
     }
+    if (!eval_only) {
+        const int info[6] = {resident, grid, 0, 0, 0, a.solo};
+        memcpy(m->last_fit, info, sizeof info);
+    }
     if (sharded) {   // what the counters and tags look like after this launch (the same on every rank)
         const unsigned long long steps = (unsigned long long)epochs * (unsigned long long)count;
         const unsigned long long barriers = (d.D > 1 ? 1ull : 0ull) + steps * (unsigned long long)(d.D - 1);

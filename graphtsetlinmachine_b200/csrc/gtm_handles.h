@@ -38,6 +38,7 @@ struct gtm_model {
     bool hv_lists_valid = false;
     int *hv_off = nullptr, *hv_clause = nullptr;
     unsigned long long *phase_cycles = nullptr;
+    int last_fit[6] = {-1, 0, 0, 0, 0, 0};    // gtm_debug_last_fit_kernel
     // node-stream scoring: derived include lists (rebuilt when the automata changed)
     StreamModel sm;
     bool lists_dirty = true;

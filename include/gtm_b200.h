@@ -238,10 +238,15 @@ int gtm_transform_nodewise(gtm_model *model, gtm_dataset *dataset, int number_of
  *   each layer; messages_out: uint32[depth-1][n][ceil(2*MESSAGE_SIZE/32)] packed messages (clause_X);
  *   n_inc_out: int32[CLAUSES]; class_sum_out: int32[CLASSES].  Any output may be NULL.
  *  gtm_debug_last_feedback: after gtm_fit, the selected node per clause int32[CLAUSES] (clause_node) and the
- *   feedback type int32[CLASSES][CLAUSES] (class_clause_update) of the last graph processed. */
+ *   feedback type int32[CLASSES][CLAUSES] (class_clause_update) of the last graph processed.
+ *  gtm_debug_last_fit_kernel: what the last gtm_fit launched, int32[6] = {kernel: 0 global-state, 1 state-resident, 2 chain
+ *   (one GPU), -1 none yet; thread blocks; and for the chain kernel: node words of its transposed rows (1, 4, 16, 32), 1 when
+ *   only the include planes are in shared memory, 1 when a warp updates all layers of its clause, 1 when one thread block
+ *   learns the model alone}. */
 int gtm_debug_evaluate(gtm_model *model, gtm_dataset *dataset, int number_of_node_types, int64_t graph, int path,
                        uint32_t *cno_out, uint32_t *messages_out, int32_t *n_inc_out, int32_t *class_sum_out);
 int gtm_debug_last_feedback(gtm_model *model, int32_t *clause_node_out, int32_t *class_clause_update_out);
+int gtm_debug_last_fit_kernel(gtm_model *model, int32_t *info_out);
 
 /* Profiling tap (no counterpart in the reference): SM clock cycles that the first warp of CTA 0 of the last gtm_fit launch
  * spent in its phases, uint64[8] = {clause evaluation, waiting at grid barriers, vote exchange (with the work done in

@@ -185,6 +185,11 @@ class EngineTM:
         y = np.ascontiguousarray(encoded_Y, dtype=np.int32)
         _lib.check(self.lib.gtm_fit(self.model, self.ds, self.n_types, _ptr(y), int(first), int(count), int(epochs)))
 
+    def last_fit_kernel(self):
+        info = np.zeros(6, dtype=np.int32)
+        _lib.check(self.lib.gtm_debug_last_fit_kernel(self.model, _ptr(info)))
+        return dict(zip(("kernel", "ctas", "node_words", "hybrid", "narrow", "one_cta"), info.tolist()))
+
     def last_feedback(self):
         node = np.zeros(self.C, dtype=np.int32)
         upd = np.zeros((self.K, self.C), dtype=np.int32)
