@@ -8,10 +8,8 @@
 #include <cstdio>
 #include <cmath>
 #include <cstring>
-#include <exception>
 #include <new>
 #include <string>
-#include <thread>
 #include <vector>
 
 #include "gtm_handles.h"
@@ -429,21 +427,18 @@ static void check_graph_span(const gtm_graphs_view *v, int64_t g_lo, int64_t g_h
 static int validate_graphs(const gtm_graphs_view *v, int64_t g_lo, int64_t g_hi, GraphChecks *all_out = nullptr)
 {
     if (g_lo == 0 && (v->node_index[0] != 0 || v->edge_index[0] != 0)) return fail(GTM_ERR_ARG, "node_index[0] and edge_index[0] must be 0");
-    // large sets are checked by a few threads side by side (the arrays are only read); what finds no thread is checked here
-    const int64_t span = g_hi - g_lo;
-    const int pieces = (int)std::max<int64_t>(1, std::min<int64_t>(8, span / (1 << 18)));
-    GraphChecks parts[8];
-    std::thread threads[8];
-    auto check = [&](int i) { check_graph_span(v, g_lo + span * i / pieces, g_lo + span * (i + 1) / pieces, &parts[i]); };
-    for (int i = 1; i < pieces; ++i) {
-        try { threads[i] = std::thread(check, i); }
-        catch (const std::exception &) { check(i); }
-    }
-    check(0);
+    // large sets are checked by the copy threads side by side (the arrays are only read); a thread takes about 2^15 nodes
+    const int64_t span = g_hi - g_lo, nodes = span * (v->total_nodes / v->number_of_graphs + 1);
+    const int pieces = (int)std::max<int64_t>(1, std::min<int64_t>(std::min<int64_t>(16, span), nodes >> 15));
+    struct Job { const gtm_graphs_view *v; int64_t lo, span; int pieces; GraphChecks parts[16]; } job;
+    job.v = v; job.lo = g_lo; job.span = span; job.pieces = pieces;
+    host_parallel(pieces, [](void *c, int i) {
+        Job *j = (Job *)c;
+        check_graph_span(j->v, j->lo + j->span * i / j->pieces, j->lo + j->span * (i + 1) / j->pieces, &j->parts[i]);
+    }, &job);
     GraphChecks all;
     for (int i = 0; i < pieces; ++i) {
-        if (threads[i].joinable()) threads[i].join();
-        const GraphChecks &c = parts[i];
+        const GraphChecks &c = job.parts[i];
         all.bad_count |= c.bad_count; all.bad_index |= c.bad_index; all.bad_edges |= c.bad_edges; all.types |= c.types;
         all.n_min = std::min(all.n_min, c.n_min); all.n_max = std::max(all.n_max, c.n_max);
     }
@@ -482,6 +477,7 @@ static int check_view(const gtm_graphs_view *v)
 extern "C" int gtm_validate_graphs(const gtm_graphs_view *v)
 {
     GTM_TRY(check_view(v));
+    struct Keep { Keep() { stage_retain(-1); } ~Keep() { stage_drop(); } } keep;      // the copy threads stay while they check
     return validate_graphs(v, 0, v->number_of_graphs);
 }
 
@@ -521,7 +517,8 @@ __global__ void __launch_bounds__(256) fill_range_kernel(RangeFill f)
 }
 
 // Graphs [g0, g1) of the set: copies queued on stream `in`, and the rest of their arrays described for fill_range_kernel.
-static int upload_range(gtm_dataset *ds, const gtm_graphs_view *v, int64_t g0, int64_t g1, const GraphChecks &facts, cudaStream_t in, RangeFill *fill)
+static int upload_range(gtm_dataset *ds, const gtm_graphs_view *v, StageLane *lane, int64_t g0, int64_t g1, const GraphChecks &facts, cudaStream_t in,
+                        RangeFill *fill)
 {
     const DevGraphs &dg = ds->dg;
     const int64_t N = v->number_of_graphs;
@@ -540,21 +537,21 @@ static int upload_range(gtm_dataset *ds, const gtm_graphs_view *v, int64_t g0, i
     f.node_index = const_cast<u32 *>(dg.node_index); f.n_nodes = const_cast<u32 *>(dg.n_nodes);
     f.graph_edge0 = const_cast<u32 *>(dg.graph_edge0); f.graph_edges = const_cast<u32 *>(dg.graph_edges);
     *fill = f;
-    auto up = [&](const u32 *dst, const u32 *src, size_t first, size_t count) -> int {
-        if (count) GTM_CU(cudaMemcpyAsync(const_cast<u32 *>(dst) + first, src + first, count * sizeof(u32), cudaMemcpyHostToDevice, in));
-        return GTM_OK;
+    const bool pinned = host_is_pinned(v->X);
+    auto up = [&](const u32 *dst, const u32 *src, size_t first, size_t count, bool pin) {
+        return stage_up(lane, const_cast<u32 *>(dst) + first, src + first, count * sizeof(u32), pin, in);
     };
     const size_t v0 = (size_t)f.v0, nodes = (size_t)(f.v1 - f.v0), graphs = (size_t)(g1 - g0);
-    GTM_TRY(up(dg.X, v->X, v0 * L0, nodes * L0));
-    if (!f.no_types) GTM_TRY(up(dg.node_type, v->node_type, v0, nodes));
+    GTM_TRY(up(dg.X, v->X, v0 * L0, nodes * L0, pinned));
+    if (!f.no_types) GTM_TRY(up(dg.node_type, v->node_type, v0, nodes, host_is_pinned(v->node_type)));
     if (!f.no_edges) {
-        GTM_TRY(up(dg.degree, v->number_of_graph_node_edges, v0, nodes));
-        GTM_TRY(up(dg.edge_index, v->edge_index, v0, nodes));
-        GTM_TRY(up(dg.edge, v->edge, 2 * (size_t)f.e0, 2 * (size_t)(e1 - f.e0)));
+        GTM_TRY(up(dg.degree, v->number_of_graph_node_edges, v0, nodes, host_is_pinned(v->number_of_graph_node_edges)));
+        GTM_TRY(up(dg.edge_index, v->edge_index, v0, nodes, host_is_pinned(v->edge_index)));
+        GTM_TRY(up(dg.edge, v->edge, 2 * (size_t)f.e0, 2 * (size_t)(e1 - f.e0), host_is_pinned(v->edge)));
     }
     if (f.uniform_n == 0) {
-        GTM_TRY(up(dg.node_index, v->node_index, (size_t)g0, graphs + (g1 < N ? 1 : 0)));
-        GTM_TRY(up(dg.n_nodes, v->number_of_graph_nodes, (size_t)g0, graphs));
+        GTM_TRY(up(dg.node_index, v->node_index, (size_t)g0, graphs + (g1 < N ? 1 : 0), host_is_pinned(v->node_index)));
+        GTM_TRY(up(dg.n_nodes, v->number_of_graph_nodes, (size_t)g0, graphs, host_is_pinned(v->number_of_graph_nodes)));
     }
     return GTM_OK;
 }
@@ -616,7 +613,7 @@ static int dataset_build(gtm_model *m, const gtm_graphs_view *v, gtm_dataset *ds
             GTM_TRY(upload_small(ds, v, lane, l, dev, s));
         } else {
             RangeFill f;
-            GTM_TRY(upload_range(ds, v, 0, v->number_of_graphs, facts, s, &f));
+            GTM_TRY(upload_range(ds, v, lane, 0, v->number_of_graphs, facts, s, &f));
             GTM_TRY(fill_range(f, s));
         }
     } else if (ds->max_nodes > 1) {                      // not validated yet: the tilings take these only as hints
@@ -936,7 +933,7 @@ static int score_in_chunks(gtm_model *m, gtm_dataset *ds, const gtm_graphs_view 
                 GraphChecks facts;
                 RangeFill f;
                 GTM_TRY(validate_graphs(v, g0, g1, &facts));      // overlaps the copies of the chunks before
-                GTM_TRY(upload_range(ds, v, g0, g1, facts, lane->in, &f));
+                GTM_TRY(upload_range(ds, v, lane, g0, g1, facts, lane->in, &f));
                 GTM_CU(cudaEventRecord(lane->event[1], lane->in));
                 GTM_CU(cudaStreamWaitEvent(cs, lane->event[1], 0));
                 GTM_TRY(fill_range(f, cs));

@@ -98,7 +98,7 @@ def test_shifted_ranges_of_large_sets_are_refused():
     """Spans of a large set are checked side by side.  Ranges that are shifted from some graph on are consistent within the
     spans behind it, whose nodes must not be looked up where they say."""
     lib = _lib.load()
-    graphs, per = 800000, 1                                       # three spans
+    graphs, per = 1200, 500                                       # 600,000 nodes: sixteen spans
     nodes = graphs * per
 
     def arrays():
