@@ -844,19 +844,25 @@ static size_t tiled_scratch_bytes(const gtm_model *m, const gtm_dataset *ds, boo
     return by_stream ? stream_scratch_bytes(ds->sd, m->dm, first, count) : tile_scratch_bytes(ds->td, m->dm, first, count);
 }
 
-// The same on the model's stream, with lists and scratch.
+// The same on the model's stream, with lists and scratch: the lane's for a call that waits for its kernels, and else, without a
+// lane, a block from the memory pool in stream order.
 static int score_tiled(gtm_model *m, gtm_dataset *ds, bool by_stream, int n_types, int64_t first, int64_t count, int *sums_dev,
-                       int *clause_out_dev = nullptr)
+                       int *clause_out_dev, StageLane *lane)
 {
     GTM_TRY(by_stream ? refresh_lists(m) : refresh_tile_lists(m));
+    const size_t need = tiled_scratch_bytes(m, ds, by_stream, first, count);
+    if (lane) {
+        GTM_TRY(lane_scratch(lane, 0, need));
+        return launch_score_tiled(m, ds, by_stream, n_types, first, count, sums_dev, clause_out_dev, lane->scratch[0], m->stream);
+    }
     char *scratch;
-    GTM_TRY(pool_alloc(&scratch, tiled_scratch_bytes(m, ds, by_stream, first, count), m->stream));
+    GTM_TRY(pool_alloc(&scratch, need, m->stream));
     const int st = launch_score_tiled(m, ds, by_stream, n_types, first, count, sums_dev, clause_out_dev, scratch, m->stream);
     cudaFreeAsync(scratch, m->stream);
     return st;
 }
 
-static int score_device(gtm_model *m, gtm_dataset *ds, int n_types, int64_t first, int64_t count, int32_t *sums_dev)
+static int score_device(gtm_model *m, gtm_dataset *ds, int n_types, int64_t first, int64_t count, int32_t *sums_dev, StageLane *lane)
 {
     GTM_TRY(bind(m));
     GTM_TRY(check_range(m, ds, n_types, first, count));
@@ -867,14 +873,14 @@ static int score_device(gtm_model *m, gtm_dataset *ds, int n_types, int64_t firs
     if (m->opt_score_kernel == 3 && !scores_by_tile(m, ds, n_types))
         return fail(GTM_ERR_ARG, "the tile scoring kernel does not cover this model / graph set");
     const bool by_stream = scores_by_stream(m, ds, n_types);
-    if (by_stream || scores_by_tile(m, ds, n_types)) return score_tiled(m, ds, by_stream, n_types, first, count, sums_dev);
+    if (by_stream || scores_by_tile(m, ds, n_types)) return score_tiled(m, ds, by_stream, n_types, first, count, sums_dev, nullptr, lane);
     return launch_score_general(m, ds, n_types, first, count, sums_dev, nullptr);
 }
 
 extern "C" int gtm_score_device(gtm_model *m, gtm_dataset *ds, int n_types, int64_t first, int64_t count,
                                 int32_t *sums_dev)
 {
-    GTM_TRY(score_device(m, ds, n_types, first, count, sums_dev));
+    GTM_TRY(score_device(m, ds, n_types, first, count, sums_dev, nullptr));
     return note_queued(m);
 }
 
@@ -912,13 +918,12 @@ static int score_in_chunks(gtm_model *m, gtm_dataset *ds, const gtm_graphs_view 
     auto chunk_lo = [&](int t0) { return std::max(first, tile_first(t0)); };
     auto chunk_hi = [&](int t0) { return std::min(first + count, tile_first(t0 + chunk_tiles)); };
     int *dev = nullptr;
-    char *scratch[2] = {nullptr, nullptr};              // of the launches on either stream
     auto body = [&]() -> int {
         GTM_TRY(by_stream ? refresh_lists(m) : refresh_tile_lists(m));
         size_t need = 0;
         for (int t0 = t_lo; t0 < t_hi; t0 += chunk_tiles)
             if (chunk_hi(t0) > chunk_lo(t0)) need = std::max(need, tiled_scratch_bytes(m, ds, by_stream, chunk_lo(t0), chunk_hi(t0) - chunk_lo(t0)));
-        for (int i = 0; i < (chunk_tiles < tiles ? 2 : 1); ++i) GTM_TRY(pool_alloc(&scratch[i], need, m->stream));
+        for (int i = 0; i < (chunk_tiles < tiles ? 2 : 1); ++i) GTM_TRY(lane_scratch(lane, i, need));
         GTM_TRY(pool_alloc(&dev, (size_t)count * d.K, m->stream));
         GTM_CU(cudaEventRecord(lane->event[0], m->stream));       // allocations, tile tables and literal lists are in stream order
         GTM_CU(cudaStreamWaitEvent(lane->in, lane->event[0], 0));
@@ -938,7 +943,7 @@ static int score_in_chunks(gtm_model *m, gtm_dataset *ds, const gtm_graphs_view 
                 GTM_CU(cudaStreamWaitEvent(cs, lane->event[1], 0));
                 GTM_TRY(fill_range(f, cs));
             }
-            GTM_TRY(launch_score_tiled(m, ds, by_stream, n_types, g0, (int64_t)cnt, dev + at, nullptr, scratch[turn], cs));
+            GTM_TRY(launch_score_tiled(m, ds, by_stream, n_types, g0, (int64_t)cnt, dev + at, nullptr, lane->scratch[turn], cs));
             GTM_CU(cudaEventRecord(lane->event[2], cs));
             GTM_CU(cudaStreamWaitEvent(lane->back, lane->event[2], 0));
             GTM_TRY(stage_down(lane, out + at, dev + at, cnt * d.K * sizeof(int), pinned_out, lane->back));
@@ -956,7 +961,6 @@ static int score_in_chunks(gtm_model *m, gtm_dataset *ds, const gtm_graphs_view 
         cudaStreamSynchronize(m->stream);
     }
     if (dev) cudaFreeAsync(dev, m->stream);
-    for (char *p : scratch) if (p) cudaFreeAsync(p, m->stream);
     return st;
 }
 
@@ -967,7 +971,7 @@ static int score_to_host(gtm_model *m, gtm_dataset *ds, int n_types, int64_t fir
     // a few results: the kernel writes them to page-locked host memory itself, which takes less than starting a copy
     if (bytes <= 16 * 1024) {
         int *direct = (int *)(lane->small + kStageSmall);
-        GTM_TRY(score_device(m, ds, n_types, first, count, direct));
+        GTM_TRY(score_device(m, ds, n_types, first, count, direct, lane));
         GTM_CU(cudaStreamSynchronize(m->stream));
         GTM_TRY(score_flag_status(m));
         memcpy(out, direct, bytes);
@@ -980,7 +984,7 @@ static int score_to_host(gtm_model *m, gtm_dataset *ds, int n_types, int64_t fir
     }
     int *dev;
     GTM_TRY(pool_alloc(&dev, (size_t)count * m->dm.K, m->stream));
-    int st = score_device(m, ds, n_types, first, count, dev);
+    int st = score_device(m, ds, n_types, first, count, dev, lane);
     if (st == GTM_OK) st = stage_down(lane, out, dev, bytes, host_is_pinned(out), m->stream);
     cudaFreeAsync(dev, m->stream);
     if (st == GTM_OK) st = stage_down_finish(lane);
@@ -1083,7 +1087,7 @@ static int transform_common(gtm_model *m, gtm_dataset *ds, int n_types, int64_t 
         // clause outputs of whole graphs come out of the tile kernel too; outputs per node only out of the general one
         if (!node_out && clause_out && m->opt_score_kernel != 1) st = ensure_tiles(m, ds);
         if (st == GTM_OK && !node_out && clause_out && m->opt_score_kernel != 1 && tile_supported(ds->td, n_types)) {
-            st = score_tiled(m, ds, false, n_types, first, count, sums_dev, co_dev);
+            st = score_tiled(m, ds, false, n_types, first, count, sums_dev, co_dev, guard.lane);
         } else if (st == GTM_OK) {
             st = launch_score_general(m, ds, n_types, first, count, sums_dev, co_dev, no_dev, node_stride);
         }

@@ -128,6 +128,7 @@ void lane_destroy(StageLane *l)
     if (l->back) cudaStreamDestroy(l->back);
     if (l->aux) cudaStreamDestroy(l->aux);
     if (l->small) cudaFreeHost(l->small);
+    for (char *p : l->scratch) if (p) cudaFree(p);
     delete l;
 }
 
@@ -236,6 +237,18 @@ void lane_release(StageLane *lane)
         if (kept < kLanesKept && g_users > 0) { lane->next = g_lanes; g_lanes = lane; return; }
     }
     lane_destroy(lane);
+}
+
+int lane_scratch(StageLane *lane, int i, size_t bytes)
+{
+    if (bytes <= lane->scratch_bytes[i]) return GTM_OK;
+    char *old = lane->scratch[i];
+    lane->scratch[i] = nullptr;
+    lane->scratch_bytes[i] = 0;
+    GTM_CU(cudaFree(old));
+    GTM_TRY(dev_alloc(&lane->scratch[i], bytes));
+    lane->scratch_bytes[i] = bytes;
+    return GTM_OK;
 }
 
 void stage_retain(int device)
