@@ -125,11 +125,11 @@ NCU_DRAM_BYTES_PER_GRAPH = {1: (270.0e6 + 30.0e6) / 4194304,
 
 # what binds the scoring kernel of every configuration according to its ncu capture (profiles/)
 NCU_BINDING = {
-    1: "tile_score_kernel<2>: short barrier-separated phases per tile (barrier stall 17.7 warps per issue); shared-memory wavefronts 27 % of peak, DRAM 1.2 %",
-    2: "stream_score_kernel<10>: shared memory (wavefronts 64 % of peak, short-scoreboard stall 5.7 warps per issue); DRAM 0.5 %",
-    3: "stream_score_kernel<10>: shared memory (wavefronts 62 % of peak); DRAM 0.5 %",
-    4: "tile_score_kernel<2>, a graph per tile: shared-memory reads, 128 bytes per included literal and graph (not captured for this shape)",
-    5: "tile_score_kernel<10>: shared memory (wavefronts 76 % of peak, 4.8 % of them from bank conflicts, issue slots 53 %); DRAM 7.9 %",
+    1: "tile_score_kernel<2, true>: short barrier-separated phases per tile (barrier stall 17.7 warps per issue); shared-memory wavefronts 27 % of peak, DRAM 1.2 %",
+    2: "stream_score_kernel<1, 8>: phases between barriers and shared memory (wavefronts 45 % of peak; barrier stall 3.3, short-scoreboard 3.2 warps per issue); DRAM 0.9 %",
+    3: "stream_score_kernel<1, 8>: as on single-node graphs (not captured for this shape)",
+    4: "tile_score_kernel<2, false>, a graph per tile: shared-memory reads (wavefronts 75 % of peak, short-scoreboard stall 8.3 warps per issue); DRAM 1.4 %",
+    5: "tile_score_kernel<10, true>: shared memory (wavefronts 85 % of peak, issue slots 48 %); DRAM 4.0 % (8,192 graphs, short training)",
 }
 
 

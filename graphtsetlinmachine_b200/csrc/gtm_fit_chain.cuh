@@ -23,7 +23,7 @@
 //
 // What bounds it: instructions of few warps.  One epoch and the way back of the state on one B200, ms, here / in
 // fit_resident_kernel or fit_kernel: 10,000 Noisy-XOR graphs (one CTA) 57 / 109; 4,000 images x 2,500 clauses 22 / 44; 200
-// sequences of 1,000 nodes 8.1 / 26.7; 300 multigraphs x 20,000 clauses 51 / 160, 36 of them in the kernel, half of that for the
+// sequences of 1,000 nodes 7.6 / 26.7; 300 multigraphs x 20,000 clauses 54 / 160, 36 of them in the kernel, half of that for the
 // Philox draws and the automata of some 95 clauses per CTA and graph.
 //
 // State: automaton planes in shared memory while they fit; otherwise (kHybrid) only the include planes, which the
@@ -468,10 +468,11 @@ __device__ __forceinline__ void solo_messages(const DevModel &m, const GraphView
 }
 
 // ------------------------------------------------------------------------------------------------ the kernel
-// Shared memory, in words: [KP] vote partial | [KP] totals | [KP] targets | [KP] thresholds | [3][KP] targets of staged graphs |
-// [4][4] graph sizes | [2] work list counters .. | [3] staged graphs | message scratch | T: transposed rows, then type rows |
-// [warps] nothing | per clause: record [kChainRec], mask stream [pre_words], state [clause_words] =
-// draw position (2), include count, its pending change, weights [KP], node words [RW], planes (or include planes) of all layers
+// Dynamic shared memory, in words (plan_chain counts the same): [KP] vote partial | [KP] totals | [KP] targets | [KP] thresholds |
+// [kChainStages][KP] targets of staged graphs | [4][4] graph sizes | [kChainStages] staged graphs, stage_total each | message
+// scratch [msg_words] | T: transposed rows [t_rows][RW] | type rows [kTransposedTypes][max(RW, 4)] | per clause: record
+// [kChainRec], mask stream [pre_words], state [clause_words] = draw position (2), include count, its pending change, weights
+// [KP], node words [max(RW, 4)], planes (or include planes) of all layers
 template <int RW, bool kOneLayer, bool kHybrid, bool kNarrow>
 __global__ void __launch_bounds__(chain_threads(kHybrid, kNarrow), 1) fit_chain_kernel(DevModel m_in, DevGraphs g, ChainArgs a)
 {

@@ -88,19 +88,26 @@ int gtm_destroy(gtm_model *model);
 int gtm_set_stream(gtm_model *model, void *cuda_stream);
 
 /* Kernel selection (the reference has one code path; its only launch knobs are grid/block, tm.py:53-54).
- *   "fit_kernel":   0 = automatic, 1 = learning kernel with state in global memory, 2 = state-resident kernel
+ *   "fit_kernel":   0 = automatic: the chain kernel (one GPU; at most 1,024 nodes per graph, 32 classes and 8 node types, 8
+ *                   state bits, Philox draws, and edge types up to 24 unless one thread block learns the model), else 2, else
+ *                   1; 1 = learning kernel with state in global memory, 2 = state-resident kernel
  *   "score_kernel": 0 = automatic, 1 = general kernel, 2 = node-stream kernel (depth 1), 3 = tile kernel (any depth,
- *                   graphs of at most 128 nodes); set it before the graph set is created
+ *                   graphs of at most 128 nodes, at most 16 classes); set it before the graph set is created
  *   "fit_timers":   1 = the learning kernels time their phases for gtm_debug_fit_phase_cycles (default 0); 2 and 3 = the
- *                   state-resident kernel splits its evaluation phase instead of its feedback phase (see that function)
- *   "fit_block_clauses": clauses per thread block of the state-resident learning kernel, 0 = automatic (default)
+ *                   state-resident kernel splits its evaluation phase instead of its feedback phase (see that function; the
+ *                   chain kernel takes 1, 2 and 3 alike)
+ *   "fit_block_clauses": clauses per thread block of the chain and the state-resident kernel, 0 = automatic (default)
  *   "fit_wait_ms":  wall-time budget of ONE device-side wait of the learning kernels (grid barrier, vote exchange between
  *                   thread blocks or GPUs), 1..600000 ms, default 2000.  A wait that runs out ends the launch; gtm_fit
- *                   returns GTM_ERR_TIMEOUT, the CUDA context stays usable.  The state-resident kernel leaves the model as
- *                   it was before the call; otherwise part of the call's updates may have been applied - restore a
- *                   checkpoint (gtm_set_ta_state / gtm_set_weights / gtm_set_draw_positions) before learning on.
+ *                   returns GTM_ERR_TIMEOUT, the CUDA context stays usable.  The state-resident kernel, and the chain kernel
+ *                   when the automata fit shared memory, leave the model as it was before the call.  Otherwise part of the
+ *                   call's updates may have been applied, and with the chain kernel automata may be left that no sequence of
+ *                   updates gives (their include bits belong to the state before the call, their other bits do not) -
+ *                   restore a checkpoint (gtm_set_ta_state / gtm_set_weights / gtm_set_draw_positions) before learning on.
+ *                   gtm_debug_last_fit_kernel tells which kernel a call ran.
  *   "fit_missing_cta": test hook, 1 = every wait of later gtm_fit calls expects one arrival more than there are thread
- *                   blocks, i.e. a participant that never shows up: the waits run out (default 0)
+ *                   blocks, i.e. a participant that never shows up: the waits run out (default 0).  A model that one thread
+ *                   block learns alone waits for nobody and learns as without it.
  * Forcing a kernel that cannot serve the model makes the next fit / score call fail with GTM_ERR_ARG. */
 int gtm_set_option(gtm_model *model, const char *name, int value);
 
@@ -249,8 +256,11 @@ int gtm_debug_last_feedback(gtm_model *model, int32_t *clause_node_out, int32_t 
 int gtm_debug_last_fit_kernel(gtm_model *model, int32_t *info_out);
 
 /* Profiling tap (no counterpart in the reference): SM clock cycles that the first warp of CTA 0 of the last gtm_fit launch
- * spent in its phases, uint64[8] = {clause evaluation, waiting at grid barriers, vote exchange (with the work done in
- * its shadow), end of step, and then
+ * spent in its phases.  Chain kernel: uint64[8] = {clause evaluation of message layers, waiting at grid barriers, waiting for
+ * the votes, updates and the next graph's first layer (narrow layers: decisions too), message bits pulled, message rows
+ * copied (one thread block: made and transposed), work in the shadow of the vote exchange, decisions of wide layers}, none
+ * part of another.  The other kernels: uint64[8] = {clause evaluation, waiting at grid barriers, vote exchange (with the work
+ * done in its shadow), end of step, and then
  *   state-resident kernel, "fit_timers" 1: decisions, work-item table, remaining mask generation, automaton updates;
  *   state-resident kernel, "fit_timers" 2: next-graph copies issued, own clauses, waiting for the other warps, sending marks;
  *   state-resident kernel, "fit_timers" 3: next-graph copies issued, message rows built, transposition, own clauses
